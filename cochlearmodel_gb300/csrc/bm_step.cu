@@ -46,6 +46,7 @@
 #include <cmath>
 #include <cstdio>
 
+#include "bm_common.cuh"
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
 #include "warmstart.cuh"
@@ -53,39 +54,6 @@
 namespace cgb {
 
 constexpr int kSPL = 8;  // sections per lane
-
-struct BMArgs {
-  const float* secp;   // [8][256]: 1/M, 1/m, R, S, Q, S_ohc, S_tm, R_tm
-  const float* gamma;  // [P][256]
-  const cgb_unit* units;
-  int n_units;
-  const float* in;
-  float* out;
-  // host mirror of out (pinned, mapped): its byte offset from out, or 0 for
-  // none; a row's host address is its device address plus the offset
-  long long host_delta;
-  int32_t* failed;
-  float* conv;  // [rows][3] mean dt, substeps, mean outer iterations per sample
-  cgb_unit_stats* stats;
-  int32_t* work;
-  float ratio, nas, al, e1, e2, nw, ar, dx2, dxa0, na1, na2, gme, sow;
-  float dt0, dtmin, dtmax;
-  // the reference's float constants 1/Ts, 1/sigma_ow (each formed in double
-  // and rounded, src/cochlea.cu:1099,1105) and time_step_out
-  float fs_f, rsow, tout_f;
-  // sigma_ow is a power of two (its reciprocal rsow is exact), so x / sigma_ow
-  // is x * rsow bit for bit
-  int ow_pow2;
-  int jfast, jslow, max_outer, max_sub;
-  // tolerance mode (jacobi_mode 2)
-  float jtol;
-  int jcap, guess, learn_every;
-  const unsigned char* ws_blob;  // packed network weights (guess 2)
-  float* log;                    // training records [6][256] (optional)
-  long long log_cap;
-  int log_every;
-  int* log_count;
-};
 
 __device__ __forceinline__ void load8(const float* p, float (&r)[kSPL]) {
   const float4 a = reinterpret_cast<const float4*>(p)[0];
@@ -226,12 +194,6 @@ struct SideVec {
     }
   }
 };
-
-// CUDA's tanhf and __fdividef on a pair (ARITH 1).
-__device__ __forceinline__ float2 tanhf2(float2 x) { return f2(tanhf(x.x), tanhf(x.y)); }
-__device__ __forceinline__ float2 fdividef2(float2 a, float2 b) {
-  return f2(__fdividef(a.x, b.x), __fdividef(a.y, b.y));
-}
 
 // Sum over the 256 sections in BMOHC_NEW_kernel's order (ARITH 1): its
 // shared-memory tree adds element i + t into element i for t = 128, 64, ...,
@@ -945,6 +907,13 @@ const LaunchShape kCountShape = CGB_SHAPE(4, 1, false, 0, 1, 0);
 const LaunchShape kRefArithShape = CGB_SHAPE(4, 1, false, 0, 1, 1);
 int g_shape = 0;
 
+// Tables of up to this many units per SM run on four warps per unit
+// (bm_quad.cu), two CTAs to an SM: at 2 x 152 units 13.4 ms against 16.5 with a
+// warp per unit (5 ms blocks).  Past that a second wave of its CTAs begins (at
+// least 10.4 ms more), while a warp per unit takes 16.5 ms up to four units an
+// SM (608) and 22.6 at eight.
+constexpr int kQuadUnitsPerSM = 2;
+
 }  // namespace cgb
 
 extern "C" int cgb_bm_set_launch_shape(int shape) {
@@ -1080,6 +1049,11 @@ extern "C" int cgb_bm_run_ex_dev(const float* d_secp, const float* d_gamma, int 
   CGB_TRY_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
   CGB_TRY_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev),
                "cudaDeviceGetAttribute");
+  // Few units: four warps each.  The launch shapes other than the default (the
+  // autotuner's) keep to their kernels.
+  if (!tol && g_shape == 0 && n_units <= kQuadUnitsPerSM * n_sm &&
+      sc->jacobi_slow <= kQuadMaxSweeps && sc->jacobi_fast <= kQuadMaxSweeps)
+    return bm_quad_launch(A, sc->controller, sc->arith, st);
   const LaunchShape& shape = learned               ? kLearnedShape
                              : tol                 ? kTolShape
                              : ref_arith           ? kRefArithShape
