@@ -29,6 +29,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -37,88 +38,20 @@
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
+#include "ihc_common.cuh"
+#include "ihc_tensor.h"
 
 namespace cgb {
 namespace {
 
-constexpr int kSecTile = 32;   // sections per CTA (one per lane)
 constexpr int kBoxRows = 64;   // rows per TMA box
-constexpr int kIhcWarps = 16;
 constexpr int kRB = 8;         // output rows per register block
-// bound on one staging wait, in nanoseconds of the GPU's global timer
-constexpr unsigned long long kWaitNs = 1000000000ull;
 constexpr int kTilesPerRun = 8;  // consecutive tiles per CTA (short runs)
-
-struct IHCArgs {
-  const cgb_ihc_frame* frames;
-  const int32_t* tile_prefix;  // [n_frames + 1] runs of tiles before each frame
-  int n_frames;
-  const float* taps;           // [n_ac] AC taps (x scale) then [n_dc] DC taps
-  int n_ac, n_dc;
-  float scale, eta_ac, eta_dc, sat;
-  float spont0, spont1, spont2;
-  const float* dmg;            // [P][256] 10^ihc
-  const float* aihc;           // [3][256]
-  float* lam;                  // [3][lam_plane_rows][256]
-  float* lam_host;             // host mirror of lam (pinned, mapped), or null
-  int64_t lam_plane_rows;
-  float* ihc;                  // [lam rows][256] or null
-  int TR, xrows;               // output rows per tile, staged rows (multiple of 64)
-  int32_t* status;
-  int dc_uniform;              // all DC taps equal: running window sum
-  int ac_sym;                  // AC taps symmetric: FIR over tap pairs
-  int run;                     // tiles per CTA (consecutive, one frame)
-  const float* ac_ext;         // AC by velocity row (the IIR path), or null: the FIR
-  int skip_first_copy;         // test-only: arm the first staging wait but issue no copy
-  // RunIHCKernel's debug stage: 9 AC, 10 DC, 11 dS (0 none), stored by lambda
-  // row into stage_out [lam rows][256]
-  int stage;
-  float* stage_out;
-};
 
 // Test-only fault injection (cgb_ihc_set_fault_injection): the next launches
 // arm the first staging mbarrier without issuing its copies, so the bounded
 // wait runs out with nothing in flight and the kernel reports status bit 1.
 int g_fault_skip_copy = 0;
-
-__device__ __forceinline__ int taps_used(int k, const cgb_ihc_frame& f, int taps) {
-  const int sg = k < f.frdp - 1 ? f.seg : f.total;
-  const int lim = (k + 1) % sg;
-  return lim < taps ? lim : taps;
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// Compensated tap accumulation (Ogita-Rump-Oishi Dot2): the product error
-// comes from one FMA, the sum error from TwoSum, and both are carried in c.
-// The result equals the dot product evaluated in about twice the working
-// precision and rounded once -- what the reference's double accumulators
-// give after their float store -- at FP32 instruction rates.
-struct Dot2 {
-  float s, c;
-  __device__ __forceinline__ void init() { s = c = 0.0f; }
-  __device__ __forceinline__ void add(float b, float x) {
-    const float p = __fmul_rn(b, x);
-    const float q = __fmaf_rn(b, x, -p);
-    const float t = __fadd_rn(s, p);
-    const float z = __fsub_rn(t, s);
-    const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z));
-    s = t;
-    c = __fadd_rn(c, __fadd_rn(e, q));
-  }
-  // b (x1 + x2) for a symmetric tap pair: the pair sum by TwoSum, Dot2 on
-  // its rounded value, b times its rounding error into c by one fma
-  __device__ __forceinline__ void add_pair(float b, float x1, float x2) {
-    const float sg = __fadd_rn(x1, x2);
-    const float zz = __fsub_rn(sg, x1);
-    const float ep = __fadd_rn(__fsub_rn(x1, __fsub_rn(sg, zz)), __fsub_rn(x2, zz));
-    add(b, sg);
-    c = __fmaf_rn(b, ep, c);
-  }
-  __device__ __forceinline__ float result() const { return __fadd_rn(s, c); }
-};
 
 // Dot2 on two independent sums at once (two-wide FP32); each element
 // performs exactly the scalar Dot2 sequence.
@@ -237,18 +170,6 @@ __device__ __forceinline__ float fir_row_sym(const float* __restrict__ src,
   return acc.result();
 }
 
-// s + c += x exactly (Knuth's TwoSum; the rounding error goes to c).
-__device__ __forceinline__ void two_sum_add(float& s, float& c, float x) {
-  const float t = __fadd_rn(s, x);
-  const float z = __fsub_rn(t, s);
-  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z));
-  s = t;
-  c = __fadd_rn(c, e);
-}
-
-constexpr int kDcAnchor = 32;  // DC window re-summed at frame rows k % 32 == 0
-constexpr int kEmitRows = 4;   // rows per warp in one IHC / lambda batch
-
 __device__ __forceinline__ float fir_row(const float* __restrict__ src,
                                          const float* __restrict__ b, int tu) {
   Dot2 acc;
@@ -277,29 +198,6 @@ __device__ __forceinline__ void stage_rows(const CUtensorMap* vmap, float* X, ui
         "l"(vmap), "r"(s0), "r"(y), "r"(smem_u32(mbar))
         : "memory");
   }
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Wait on phase `parity` of mbar by every thread, for at most kWaitNs of the
-// global timer (each try_wait returns within a short system-defined time),
-// then a block-wide vote so that all threads take the same branch.
-__device__ __forceinline__ bool wait_stage(uint64_t* mbar, uint32_t parity) {
-  uint32_t done = 0;
-  const unsigned long long t_start = global_ns();
-  while (!done) {
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(smem_u32(mbar)), "r"(parity)
-        : "memory");
-    if (!done && global_ns() - t_start > kWaitNs) break;
-  }
-  return __syncthreads_and(done) != 0;
 }
 
 // One CTA = 32 sections x a run of up to A.run consecutive tiles of TR rows
@@ -591,20 +489,77 @@ int ac_symmetric(const float* ac_taps, int n_ac, float scale) {
 // Tiles per run forced by cgb_ihc_set_run_length (the autotuner), 0: the rule below.
 int g_forced_run = 0;
 
-// The run length each scratch buffer's tables were uploaded with: the tile
-// prefix on the device depends on it, so a launch of uploaded tables must use
-// the same run length whatever the setting is by then.
+// How each scratch buffer's tables were uploaded: the tile prefix on the device
+// depends on the kernel and the run length, so a launch of uploaded tables must
+// use the same ones whatever the settings are by then.
+struct Uploaded {
+  int run;
+  bool tensor;
+  int exp_b;    // of the uploaded taps, for the tensor kernel
+  float slack;
+};
 std::mutex g_upload_run_mu;
-std::unordered_map<const void*, int> g_upload_run;
+std::unordered_map<const void*, Uploaded> g_upload_run;
+
+int sm_count() {
+  int dev = 0, n_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return n_sm;
+}
+
+// The tensor kernel's run: each CTA (one per SM) takes the time of its tiles and
+// of the two before the first that the DC filter looks back on, and the CTAs
+// go in waves over the SMs; the length with the least waves x tiles.
+int pick_tensor_run(const cgb_ihc_frame* frames, int n_frames, int n_dc) {
+  if (g_forced_run > 0) return g_forced_run;
+  const int n_sm = std::max(1, sm_count());
+  const long long back = (n_dc - 1 + kTensorTileRows - 1) / kTensorTileRows;
+  int best = 1;
+  long long best_cost = 0;
+  for (int r : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64}) {
+    long long runs = 0;
+    for (int i = 0; i < n_frames; ++i) {
+      const long long tiles = ((long long)frames[i].lam_rows + kTensorTileRows - 1) /
+                              kTensorTileRows;
+      runs += (tiles + r - 1) / r;
+    }
+    const long long ctas = runs * (256 / kTensorSections);
+    const long long cost = (ctas + n_sm - 1) / n_sm * (r + back);
+    if (r == 1 || cost < best_cost) {
+      best = r;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// What the tensor kernel needs to know of the AC taps (scaled, as the kernels
+// use them): the exponent of the largest, and the slack of its rounding test in
+// the units of its accumulators (2^16 of the product of the two scales), from
+// the sum of their magnitudes.  False: no usable exponent.
+bool tensor_taps(const float* ac_taps, int n_ac, float scale, int* exp_b, float* slack) {
+  float top = 0.0f;
+  double sum = 0.0;
+  for (int i = 0; i < n_ac; ++i) {
+    const float b = ac_taps[i] * scale;
+    if (!std::isfinite(b)) return false;
+    top = std::max(top, std::fabs(b));
+    sum += std::fabs((double)b);
+  }
+  if (!(top > 0.0f)) return false;
+  std::frexp(top, exp_b);
+  if (*exp_b < -16 || *exp_b > 16) return false;
+  *slack = (float)std::ldexp(std::ldexp(sum, -43 - *exp_b) + std::ldexp(1.0, -39), 16);
+  return true;
+}
 
 int pick_run(const cgb_ihc_frame* frames, int n_frames, int TR, int n_dc) {
   if (TR < n_dc) return 1;
   if (g_forced_run > 0) return g_forced_run;
-  int dev = 0, n_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      n_sm < 1)
-    n_sm = 1 << 20;  // unknown: keep the short runs
+  int n_sm = sm_count();
+  if (n_sm < 1) n_sm = 1 << 20;  // unknown: keep the short runs
   for (int r : {32, 16}) {
     long long runs = 0;
     for (int i = 0; i < n_frames; ++i) {
@@ -678,16 +633,31 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   int TR = 0, xrows = 0;
   pick_tile(n_ac, n_dc, &TR, &xrows);
   if (TR < 32) return fail(CGB_ERR_RANGE, "cgb_ihc_lambda_dev: filters too long for one tile");
-  int run = pick_run(frames, n_frames, TR, n_dc);
+  int dc_uniform = 1;
+  for (int i = 1; i < n_dc; ++i) dc_uniform &= dc_taps[i] == dc_taps[0];
+  // The AC filter goes to the tensor cores where the kernel is built for it: a
+  // uniform DC filter, no debug stage, no AC given, lengths that fit.
+  int exp_b = 0;
+  float slack = 0.0f;
+  bool tensor = !ac_ext && stage == 0 && dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
+                tensor_taps(ac_taps, n_ac, prm->scale, &exp_b, &slack);
+  int run = tensor ? pick_tensor_run(frames, n_frames, n_dc)
+                   : pick_run(frames, n_frames, TR, n_dc);
   {
     std::lock_guard<std::mutex> lock(g_upload_run_mu);
     if (mode & kUpload) {
-      g_upload_run[d_scratch] = run;
+      g_upload_run[d_scratch] = {run, tensor, exp_b, slack};
     } else {
       const auto it = g_upload_run.find(d_scratch);
-      if (it != g_upload_run.end()) run = it->second;
+      if (it != g_upload_run.end()) {
+        run = it->second.run;
+        tensor = it->second.tensor;
+        exp_b = it->second.exp_b;
+        slack = it->second.slack;
+      }
     }
   }
+  if (tensor) TR = kTensorTileRows;
   for (int i = 0; i < n_frames; ++i) {
     const cgb_ihc_frame& fr = frames[i];
     const bool ok = fr.v_row0 >= 0 && fr.lam_rows >= 0 && fr.lam_rows <= fr.rows &&
@@ -728,20 +698,6 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   }
   if (!(mode & kLaunch)) return CGB_OK;
 
-  auto encode = get_encode();
-  if (!encode) return fail(CGB_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-  CUtensorMap map;
-  cuuint64_t dims[2] = {256, (cuuint64_t)v_rows};
-  cuuint64_t strides[1] = {256 * 4};
-  cuuint32_t box[2] = {(cuuint32_t)kSecTile, (cuuint32_t)kBoxRows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(d_v), dims,
-                       strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (cr != CUDA_SUCCESS)
-    return fail(CGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)cr) + ")");
-
   IHCArgs A{};
   A.frames = reinterpret_cast<const cgb_ihc_frame*>(sc);
   A.tile_prefix = reinterpret_cast<const int32_t*>(sc + fbytes);
@@ -770,9 +726,24 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   A.stage = stage == 12 ? 11 : stage;  // the reference's 12 ("Shigh") is dS too
   A.stage_out = d_stage;
   A.run = run;
-  A.dc_uniform = 1;
-  for (int i = 1; i < n_dc; ++i) A.dc_uniform &= dc_taps[i] == dc_taps[0];
+  A.dc_uniform = dc_uniform;
   A.ac_sym = ac_symmetric(ac_taps, n_ac, prm->scale);
+  if (tensor) return ihc_tensor_launch(A, d_v, n_tiles, exp_b, slack, st);
+
+  CUtensorMap map;
+  auto encode = get_encode();
+  if (!encode) return fail(CGB_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+  cuuint64_t dims[2] = {256, (cuuint64_t)v_rows};
+  cuuint64_t strides[1] = {256 * 4};
+  cuuint32_t box[2] = {(cuuint32_t)kSecTile, (cuuint32_t)kBoxRows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(d_v), dims,
+                       strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (cr != CUDA_SUCCESS)
+    return fail(CGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)cr) + ")");
+
   const size_t smem = smem_bytes(TR, xrows, n_ac, n_dc);
   CGB_TRY_CUDA(cudaFuncSetAttribute(ihc_lambda_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),

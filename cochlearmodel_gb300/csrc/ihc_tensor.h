@@ -1,0 +1,23 @@
+// Host side of the IHC / lambda kernel with the AC filter on the tensor cores.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "ihc_common.cuh"
+
+namespace cgb {
+
+// Shorter filters stay on the FP32 pipe: a tile's products cost the same for
+// any length.
+constexpr int kTensorMinTaps = 64;
+constexpr int kTensorTileRows = 128;
+constexpr int kTensorSections = 64;
+
+// Whether the filters' lengths fit the kernel (taps of one tile, shared memory).
+bool ihc_tensor_fits(int n_ac, int n_dc);
+// exp_b: the exponent of the largest |tap| (2^(exp_b-1) <= it < 2^exp_b);
+// slack: see ihc_tensor.cu.
+int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b, float slack,
+                      cudaStream_t st);
+
+}  // namespace cgb
