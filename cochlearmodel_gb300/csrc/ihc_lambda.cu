@@ -495,8 +495,7 @@ int g_forced_run = 0;
 struct Uploaded {
   int run;
   bool tensor;
-  int exp_b;    // of the uploaded taps, for the tensor kernel
-  float slack;
+  int exp_b;  // of the uploaded taps, for the tensor kernel
 };
 std::mutex g_upload_run_mu;
 std::unordered_map<const void*, Uploaded> g_upload_run;
@@ -535,24 +534,18 @@ int pick_tensor_run(const cgb_ihc_frame* frames, int n_frames, int n_dc) {
   return best;
 }
 
-// What the tensor kernel needs to know of the AC taps (scaled, as the kernels
-// use them): the exponent of the largest, and the slack of its rounding test in
-// the units of its accumulators (2^16 of the product of the two scales), from
-// the sum of their magnitudes.  False: no usable exponent.
-bool tensor_taps(const float* ac_taps, int n_ac, float scale, int* exp_b, float* slack) {
+// The exponent of the largest AC tap (scaled, as the kernels use them), for the
+// tensor kernel.  False: none that it can use.
+bool tensor_taps(const float* ac_taps, int n_ac, float scale, int* exp_b) {
   float top = 0.0f;
-  double sum = 0.0;
   for (int i = 0; i < n_ac; ++i) {
     const float b = ac_taps[i] * scale;
     if (!std::isfinite(b)) return false;
     top = std::max(top, std::fabs(b));
-    sum += std::fabs((double)b);
   }
   if (!(top > 0.0f)) return false;
   std::frexp(top, exp_b);
-  if (*exp_b < -16 || *exp_b > 16) return false;
-  *slack = (float)std::ldexp(std::ldexp(sum, -43 - *exp_b) + std::ldexp(1.0, -39), 16);
-  return true;
+  return *exp_b >= -16 && *exp_b <= 16;
 }
 
 int pick_run(const cgb_ihc_frame* frames, int n_frames, int TR, int n_dc) {
@@ -638,22 +631,20 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   // The AC filter goes to the tensor cores where the kernel is built for it: a
   // uniform DC filter, no debug stage, no AC given, lengths that fit.
   int exp_b = 0;
-  float slack = 0.0f;
   bool tensor = !ac_ext && stage == 0 && dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
-                tensor_taps(ac_taps, n_ac, prm->scale, &exp_b, &slack);
+                tensor_taps(ac_taps, n_ac, prm->scale, &exp_b);
   int run = tensor ? pick_tensor_run(frames, n_frames, n_dc)
                    : pick_run(frames, n_frames, TR, n_dc);
   {
     std::lock_guard<std::mutex> lock(g_upload_run_mu);
     if (mode & kUpload) {
-      g_upload_run[d_scratch] = {run, tensor, exp_b, slack};
+      g_upload_run[d_scratch] = {run, tensor, exp_b};
     } else {
       const auto it = g_upload_run.find(d_scratch);
       if (it != g_upload_run.end()) {
         run = it->second.run;
         tensor = it->second.tensor;
         exp_b = it->second.exp_b;
-        slack = it->second.slack;
       }
     }
   }
@@ -728,7 +719,7 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   A.run = run;
   A.dc_uniform = dc_uniform;
   A.ac_sym = ac_symmetric(ac_taps, n_ac, prm->scale);
-  if (tensor) return ihc_tensor_launch(A, d_v, n_tiles, exp_b, slack, st);
+  if (tensor) return ihc_tensor_launch(A, d_v, n_tiles, exp_b, st);
 
   CUtensorMap map;
   auto encode = get_encode();

@@ -4,30 +4,40 @@
 // What bounded the stage: 127 tap pairs of compensated FP32 arithmetic per
 // point, ~2,170 lane operations (43 ms of the FP32 pipe on 2.9 million rows).
 // Here the filter is a product of digit matrices (tensor_fir.cuh) that is exact
-// to about 2^-41 of the scales, 17.6k cycles of the tensor pipe for a tile of
-// 128 rows x 64 sections; 15 exact integers per point leave TMEM as five sums.
+// to about 2^-50 of the scales, 22k cycles of the tensor pipe for a tile of
+// 128 rows x 64 sections; six exact integers per point leave TMEM.
 //
 // The same bits as the compensated FIR (Dot2).  Both are the sum rounded once,
-// up to errors far below an ulp: Dot2's stay under 2^-37.9 of (largest |x| of
-// the window x largest |b|) over 2.8 million points of solved velocity (tones of
-// 20-100 dB, noise of 0-40 dB), the digits' about 2^-41.  So the two can only
-// differ where the exact sum lies that close to a rounding boundary.  The
-// epilogue rounds sum +- slack; where that makes a difference (1-2% of the points
-// of noisy signals, next to none of others), and in rows whose look-back is
-// shorter than the tile's, the point is evaluated by Dot2 itself.
+// up to errors far below an ulp: the digits', and Dot2's, over 400,000 points of
+// solved velocity (tones of 20-100 dB, noise of 0-40 dB) at most 59 x 2^-48 of
+// the largest partial sum among four rows of a tile.  So the two can only differ
+// where the exact sum lies that close to a rounding boundary.  The tile bounds its
+// first and last row's partial sums from above (sums from either end of the
+// filter over runs of 24 rows, from registers); the epilogue rounds the sum +-
+// 40 x 2^-48 of that bound, about twice the partial sum itself; where it makes a
+// difference, and in rows whose look-back is shorter than the tile's, the point
+// is evaluated by Dot2.  On the JND sweep 39% of the tiles have no such point,
+// 48% one to eight of 8,192.
 //
 // One CTA: 64 sections x a run of tiles of one frame.  Sixteen warps hold the
 // tile's 384 rows of velocity in registers (48 values a thread) and write one
 // digit after another into two shared-memory halves; a seventeenth issues the
-// products as soon as a half is there.  The first digit's products take a third
-// of the tile's time, which the DC sums, IHC and lambda of the tile before pass
-// under.
+// products as soon as a half is there.  Between the digits the same warps finish
+// the tile before: its Dot2 points, the DC sums, IHC and lambda.
+//
+// What bounds it now: the workers' chain, ~57k cycles a tile (Dot2 points 12k, DC
+// sums 11k, IHC / lambda 7k, loads 7k, digits 10k, epilogue 4k) at 41% of the
+// issue slots, not the tensor pipe.  Finishing a tile at once instead of between
+// the next one's digits takes 22.0 ms against 18.9 (JND sweep); without the products
+// (accumulators left as they are) the chain takes the same time.
 //
 // Measured (GB300), against the FP32 pipe: JND sweep (2.9 million rows) 53.7 ->
-// 25.9 ms, 176,000 rows in 33 intervals 4.46 -> 2.05 ms, one signal of 5,330 rows
-// 0.80 -> 0.38 ms.
+// 18.3 ms, 176,000 rows in 33 intervals 4.46 -> 1.52 ms, one signal of 5,330 rows
+// 0.80 -> 0.28 ms.
 
 #include <cuda_runtime.h>
+
+#include <cstddef>
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
@@ -48,17 +58,32 @@ static_assert(kWorkers * kWorkerRegs + 128 * kIssueRegs <= kThreads * 96, "regis
 constexpr int kCols = tfir::kCols;
 constexpr int kPitch = kCols + 1;          // a row of dS / AC: lanes along rows too
 constexpr int kGroups = kCols / 32;        // section halves
+constexpr int kList = 1024;                // points for Dot2 listed by tile
+constexpr int kFewPoints = 48;             // up to here a warp to a point
+constexpr int kRuns = 16;                  // runs of 24 rows of a tile's x
 
 struct TensorShared {
   uint64_t mbar[2];          // products of half h are done
   uint32_t tmem;
-  int abort;
-  int listed;                // points for Dot2
-  int listed_pad;
+  int abort;                 // a wait ran out
+  int stop;                  // the workers have ended the run early
+  int listed;                // points for Dot2 (more than kList: all of the tile)
+  int dot2_rows[2];          // rows for Dot2, by tile parity
+  int kmin[2];               // first row of x of the tile, by tile parity
   uint32_t top[2][kCols];    // largest |x| bits of the tile, by tile parity
-  float slack[kCols];        // in units of the accumulators; +inf: no usable scale
-  float unit[kCols];         // 2^(e+eb-16)
+  alignas(16) float2 scale[kCols];       // slack in units of the accumulators (+inf: no usable
+                             // scale), and the unit 2^(e+eb-16)
+  uint32_t partial[kCols];   // bits of the largest partial sum of the sampled rows
+  // of the first and last row's sum over each run of 24 rows of x: the sum and
+  // its largest partial sum
+  float2 sample[2][kRuns][kCols];
+  uint16_t list[kList];
+  unsigned char row[tfir::kRows];  // how the tile's row gets its AC: kRow...
 };
+static_assert(offsetof(TensorShared, mbar) % 8 == 0 && offsetof(TensorShared, scale) % 16 == 0 &&
+                  offsetof(TensorShared, sample) % 8 == 0 && sizeof(TensorShared) % 16 == 0,
+              "vector accesses");
+constexpr int kRowZero = 0, kRowSum = 1, kRowDot2 = 2;
 
 __device__ __forceinline__ void sync_workers() {
   asm volatile("bar.sync 3, %0;" ::"n"(kWorkers) : "memory");
@@ -70,44 +95,199 @@ __device__ __forceinline__ void half_wait(int h) {  // the issuing warp
   asm volatile("bar.sync %0, %1;" ::"r"(1 + h), "n"(kBarrier) : "memory");
 }
 
-// TwoSum
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-  const float t = __fadd_rn(a, b);
-  const float z = __fsub_rn(t, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
+// TwoSum, two at once
+__device__ __forceinline__ float2 two_sum2(float2 a, float2 b, float2& err) {
+  const float2 t = add2(a, b);
+  const float2 z = sub2(t, a);
+  err = add2(sub2(a, sub2(t, z)), sub2(b, z));
   return t;
+}
+
+// own_log10f on a pair: the same operation sequence per element.
+__device__ __forceinline__ float2 own_log10f2(float2 x) {
+  const int ix = __float_as_int(x.x), iy = __float_as_int(x.y);
+  float mx = __int_as_float((ix & 0x7fffff) | 0x3f800000);
+  float my = __int_as_float((iy & 0x7fffff) | 0x3f800000);
+  const bool hx = mx > 1.41421356f, hy = my > 1.41421356f;
+  mx = hx ? __fmul_rn(mx, 0.5f) : mx;
+  my = hy ? __fmul_rn(my, 0.5f) : my;
+  const float2 ef = f2((float)(((ix >> 23) & 0xff) - 127 + (hx ? 1 : 0)),
+                       (float)(((iy >> 23) & 0xff) - 127 + (hy ? 1 : 0)));
+  const float2 f = add2(f2(mx, my), f2b(-1.0f));
+  const float2 s = mul2(f, own_rcpf2(add2(f2b(2.0f), f)));
+  const float2 s2 = mul2(s, s);
+  float2 p = f2b(1.0f / 11.0f);
+  p = fma2(p, s2, f2b(1.0f / 9.0f));
+  p = fma2(p, s2, f2b(1.0f / 7.0f));
+  p = fma2(p, s2, f2b(1.0f / 5.0f));
+  p = fma2(p, s2, f2b(1.0f / 3.0f));
+  const float2 two_s = mul2(f2b(2.0f), s);
+  const float2 lnm = fma2(mul2(two_s, s2), p, two_s);
+  const float l2hi = 0.30102999566398120f;
+  const float l2lo = (float)(0.30102999566398120 - (double)0.30102999566398120f);
+  return fma2(ef, f2b(l2hi), fma2(ef, f2b(l2lo), mul2(lnm, f2b(0.43429448190325182f))));
+}
+
+// Dot2::add and Dot2::add_pair of N taps at once, in order: what does not depend
+// on the sums first, then their chain, the errors, and the chain of those.  (One
+// after another the ~12 dependent operations of a tap cost 90 cycles.)
+template <int N>
+__device__ __forceinline__ void dot2_taps(Dot2& acc, const float (&b)[N], const float (&x)[N]) {
+  float p[N], t[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = __fmul_rn(b[i], x[i]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) t[i] = __fadd_rn(i ? t[i - 1] : acc.s, p[i]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float a = i ? t[i - 1] : acc.s;
+    const float q = __fmaf_rn(b[i], x[i], -p[i]);
+    const float z = __fsub_rn(t[i], a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t[i], z)), __fsub_rn(p[i], z));
+    acc.c = __fadd_rn(acc.c, __fadd_rn(e, q));
+  }
+  acc.s = t[N - 1];
+}
+template <int N>
+__device__ __forceinline__ void dot2_pairs(Dot2& acc, const float (&b)[N], const float (&x1)[N],
+                                           const float (&x2)[N]) {
+  float sg[N], p[N], t[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    sg[i] = __fadd_rn(x1[i], x2[i]);
+    p[i] = __fmul_rn(b[i], sg[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) t[i] = __fadd_rn(i ? t[i - 1] : acc.s, p[i]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float zz = __fsub_rn(sg[i], x1[i]);
+    const float ep = __fadd_rn(__fsub_rn(x1[i], __fsub_rn(sg[i], zz)), __fsub_rn(x2[i], zz));
+    const float a = i ? t[i - 1] : acc.s;
+    const float q = __fmaf_rn(b[i], sg[i], -p[i]);
+    const float z = __fsub_rn(t[i], a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t[i], z)), __fsub_rn(p[i], z));
+    acc.c = __fadd_rn(acc.c, __fadd_rn(e, q));
+    acc.c = __fmaf_rn(b[i], ep, acc.c);
+  }
+  acc.s = t[N - 1];
 }
 
 // Dot2 of one output in the orders of ihc_lambda.cu (fir_row, fir_row_sym),
 // rows of 256 sections in global memory; src points at the output's row.
-__device__ float dot2_row(const float* __restrict__ src, const float* __restrict__ b, int taps,
-                          int n, bool sym) {
+__device__ __forceinline__ float dot2_row(const float* __restrict__ src,
+                                          const float* __restrict__ taps_b, int taps, int n,
+                                          bool sym) {
+  constexpr int kBatch = 8;
   Dot2 acc;
   acc.init();
   if (sym && taps == n) {
-#pragma unroll 4
-    for (int k = 0; k < n / 2; ++k)
-      acc.add_pair(b[k], src[-(int64_t)k * 256], src[-(int64_t)(n - 1 - k) * 256]);
-    if (n & 1) acc.add(b[n / 2], src[-(int64_t)(n / 2) * 256]);
+    const float* far = src - (int64_t)(n - 1) * 256;
+    const int half = n / 2, whole = half / kBatch * kBatch;
+    for (int k0 = 0; k0 < whole; k0 += kBatch) {
+      float b[kBatch], u[kBatch], w[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        u[i] = __ldg(src - (k0 + i) * 256);
+        w[i] = __ldg(far + (k0 + i) * 256);
+        b[i] = taps_b[k0 + i];
+      }
+      dot2_pairs(acc, b, u, w);
+    }
+    for (int k = whole; k < half; ++k)
+      acc.add_pair(taps_b[k], __ldg(src - k * 256), __ldg(far + k * 256));
+    if (n & 1) acc.add(taps_b[half], __ldg(src - half * 256));
   } else {
-#pragma unroll 4
-    for (int i = 0; i < taps; ++i) acc.add(b[i], src[-(int64_t)i * 256]);
+    const int whole = taps / kBatch * kBatch;
+    for (int i0 = 0; i0 < whole; i0 += kBatch) {
+      float b[kBatch], u[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        u[i] = __ldg(src - (i0 + i) * 256);
+        b[i] = taps_b[i0 + i];
+      }
+      dot2_taps(acc, b, u);
+    }
+    for (int i = whole; i < taps; ++i) acc.add(taps_b[i], __ldg(src - i * 256));
   }
   return acc.result();
 }
 
+// Adds N values to s + c by TwoSum, in order: the chain of rounded sums first,
+// then their errors, which do not depend on each other, then the chain of those.
+template <int N>
+__device__ __forceinline__ void two_sum_chain(float& s, float& c, const float (&x)[N]) {
+  float t[N];
+  t[0] = __fadd_rn(s, x[0]);
+#pragma unroll
+  for (int q = 1; q < N; ++q) t[q] = __fadd_rn(t[q - 1], x[q]);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const float a = q ? t[q - 1] : s;
+    const float z = __fsub_rn(t[q], a);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(a, __fsub_rn(t[q], z)), __fsub_rn(x[q], z)));
+  }
+  s = t[N - 1];
+}
+
+// Eight rows of a full window: row q adds x[2q] and x[2q + 1] to s + c, whose
+// values after it are rs[q], rc[q].
+__device__ __forceinline__ void two_sum_rows(float& s, float& c, const float (&x)[16],
+                                             float (&rs)[8], float (&rc)[8]) {
+  float t[16];
+  t[0] = __fadd_rn(s, x[0]);
+#pragma unroll
+  for (int q = 1; q < 16; ++q) t[q] = __fadd_rn(t[q - 1], x[q]);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const float a = q ? t[q - 1] : s;
+    const float z = __fsub_rn(t[q], a);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(a, __fsub_rn(t[q], z)), __fsub_rn(x[q], z)));
+    if (q & 1) {
+      rs[q >> 1] = t[q];
+      rc[q >> 1] = c;
+    }
+  }
+  s = t[15];
+}
+
+// The DC window of `taps` rows that ends at ring row i, newest first, by TwoSum;
+// the loads of sixteen rows ahead of their sums.  col: the section's column of
+// the ring.
+__device__ __forceinline__ void window_sum(const float* col, int i, int taps, int ring,
+                                           float& ws, float& wc) {
+  float s = 0.0f, c = 0.0f;
+  while (taps > 0) {
+    const int len = min(taps, i + 1);
+    const float* p = col + i * kPitch;
+    int j = 0;
+    for (; j + 16 <= len; j += 16, p -= 16 * kPitch) {
+      float u[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) u[q] = p[-q * kPitch];
+      two_sum_chain(s, c, u);
+    }
+    for (; j < len; ++j, p -= kPitch) two_sum_add(s, c, *p);
+    taps -= len;
+    i = ring - 1;
+  }
+  ws = s;
+  wc = c;
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
-    ihc_tensor_kernel(const IHCArgs A, const float* __restrict__ v, int exp_b, float slack) {
+    ihc_tensor_kernel(const IHCArgs A, const float* __restrict__ v, int exp_b) {
   extern __shared__ __align__(128) unsigned char smem[];
-  // layout: digits of x, two halves | band of the taps | dS [n_dc + 128] | AC
-  // [128] | taps | TensorShared
+  // layout: digits of x, two halves | band of the taps | dS, a ring of n_dc + 128
+  // rows | AC [128] | taps with 128 zeros before and zeros up to 384 | TensorShared
   unsigned char* XD = smem;
   unsigned char* AD = XD + 2 * tfir::kHalfBytes;
+  const int ring = A.n_dc + tfir::kRows;
   float* DS = reinterpret_cast<float*>(AD + tfir::kTapBytes);
-  float* AC = DS + (size_t)(A.n_dc + tfir::kRows) * kPitch;
-  float* TP = AC + (size_t)tfir::kRows * kPitch;
+  float* AC = DS + (size_t)ring * kPitch;
+  float* TP = AC + (size_t)tfir::kRows * kPitch + tfir::kRows;  // zeros before and after
   TensorShared& S = *reinterpret_cast<TensorShared*>(
-      (reinterpret_cast<uintptr_t>(TP + A.n_ac) + 15) & ~uintptr_t(15));
+      (reinterpret_cast<uintptr_t>(TP + tfir::kDepth) + 15) & ~uintptr_t(15));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_ac = A.n_ac, n_dc = A.n_dc;
 
@@ -132,16 +312,19 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int h = 0; h < 2; ++h)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.mbar[h])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    S.abort = 0;
+    S.abort = S.stop = 0;
     S.listed = 0;
+    S.dot2_rows[0] = S.dot2_rows[1] = 0;
   }
   if (threadIdx.x < 2 * kCols) (&S.top[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x < kCols) S.partial[threadIdx.x] = 0;
   if (warp == kIhcWarps) tfir::tmem_alloc(&S.tmem);
   // taps, and the band of their digits (the digits of a tap pass through AC)
   uint16_t* td = reinterpret_cast<uint16_t*>(AC);
-  for (int i = threadIdx.x; i < n_ac; i += kThreads) {
-    const float b = A.taps[i];
+  for (int i = (int)threadIdx.x - tfir::kRows; i < tfir::kDepth; i += kThreads) {
+    const float b = i >= 0 && i < n_ac ? A.taps[i] : 0.0f;
     TP[i] = b;
+    if (i < 0 || i >= n_ac) continue;
     float r = b;
     float up = __int_as_float((127 + 8 - exp_b) << 23);
     for (int j = 0; j < tfir::kDigits; ++j) {
@@ -167,15 +350,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kIhcWarps) {
     // the issuing warp
     const uint32_t issue = tfir::elected();
-    bool run = true;
-    for (int t = first; t < t1 && run; ++t) {
-      for (int i = 0; i < tfir::kDigits && run; ++i) {
+    for (int t = first; t < t1; ++t) {
+      for (int i = 0; i < tfir::kDigits; ++i) {
         for (int h = 0; h < 2; ++h) {
           half_wait(h);
-          if (*(volatile int*)&S.abort) {
-            run = false;
-            break;
-          }
+          if (i == 0 && h == 0 && *(volatile int*)&S.stop) goto done;
           tfir::fence_after();
           // (test-only: the first half's products are left out, so that the
           // wait for them runs out)
@@ -186,42 +365,90 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+  done:;
   } else if (warp < kIhcWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
-    const int sg = warp & 1, gw = warp >> 1;  // section half; row groups gw, gw + 8, ...
+    const int sg = warp & 1, gw = warp >> 1;  // section half; rows of x 24 gw .. of each half
     const int sec = 32 * sg + lane;           // this lane's section of the tile
-    const float dmg = A.dmg[(size_t)f.ihc_profile * 256 + s0 + sec];
-    const float a0 = A.aihc[0 * 256 + s0 + sec], a1 = A.aihc[1 * 256 + s0 + sec],
-                a2 = A.aihc[2 * 256 + s0 + sec];
-    const bool sec0 = s0 + sec == 0;
     const float* vf = v + (int64_t)f.v_row0 * 256 + s0;
 
-    // Rows of the tile at kb whose sums the products can give: x is taken from
-    // row kmin on (the first row of the segment, or of the first output's full
+    // Rows of the tile whose sums the products can give: x is taken from row
+    // kmin on (the first row of the segment, or of the first output's full
     // look-back), so a row qualifies if its own window starts there or has all
-    // taps.  Others, in the tile where a segment ends, go to Dot2.
+    // taps.  Others, in the tile where a segment ends, go to Dot2.  Called by
+    // 128 threads and one (kmin).
     auto window_start = [&](int kb) {
       int k = kb;
       int tu = taps_used(k, f, n_ac);
       if (tu == 0) tu = taps_used(++k, f, n_ac);
       return k - tu + 1;
     };
+    auto classify = [&](int t, int r) {
+      const int k = t * tfir::kRows + r;
+      const int tu = k < f.lam_rows ? taps_used(k, f, n_ac) : 0;
+      const int kmin = window_start(t * tfir::kRows);
+      const bool fits = (tu == n_ac && k - n_ac + 1 >= kmin) || k - tu + 1 == kmin;
+      S.row[r] = tu == 0 ? kRowZero : (fits ? kRowSum : kRowDot2);
+      if (tu > 0 && !fits) S.dot2_rows[t & 1] = 1;
+    };
 
     float x[2][3][8];  // the tile's rows: half, row group, row (from the newest)
     auto load_tile = [&](int t) {
-      const int kb = t * tfir::kRows, kmin = window_start(kb),
+      const int kb = t * tfir::kRows, kmin = S.kmin[t & 1],
                 kmax = min(kb + tfir::kRows, f.lam_rows);
+      // the newest row of the thread's first group, and the groups down from it
+      const float* src = vf + (int64_t)(kb + tfir::kRows - 1 - 24 * gw) * 256 + sec;
+      const bool whole = kmax == kb + tfir::kRows && kmin <= kb - 192;
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int g = 0; g < 3; ++g) {
-          const int top = kb + tfir::kRows - 1 - 8 * (24 * h + gw + 8 * g);
+          const int group = 24 * h + 3 * gw + g;
+          const int top = kb + tfir::kRows - 1 - 8 * group;
+          const float* row = src - (192 * h + 8 * g) * 256;
+          if (whole && group < 40) {  // rows kb - 192 and up
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const int k = top - c;
-            x[h][g][c] = k >= kmin && k < kmax ? __ldg(vf + (int64_t)k * 256 + sec) : 0.0f;
+            for (int c = 0; c < 8; ++c) x[h][g][c] = __ldg(row - c * 256);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              x[h][g][c] = top - c >= kmin && top - c < kmax ? __ldg(row - c * 256) : 0.0f;
           }
         }
+    };
+    // The sums of the tile's last and first row over this thread's two runs of
+    // 24 rows, in tap order, with their largest partial sums.
+    auto sample_runs = [&]() {
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          // the tap of the last row's first product; of the first row's, 127 less
+          const int i0 = 192 * h + 24 * gw - (r ? tfir::kRows - 1 : 0);
+          float sum = 0.0f, most = 0.0f;
+#pragma unroll
+          for (int q = 0; q < 24; ++q) {
+            sum = __fmaf_rn(TP[i0 + q], x[h][q / 8][q % 8], sum);
+            most = fmaxf(most, fabsf(sum));
+          }
+          S.sample[r][8 * h + gw][sec] = make_float2(sum, most);
+        }
+    };
+    // The largest partial sum of a sampled row, from above: of the sums from
+    // either end (a symmetric filter adds tap pairs from both).
+    auto sampled_partial = [&](int r, int c) {
+      float total = 0.0f, most = 0.0f, back = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kRuns; ++i) total = __fadd_rn(total, S.sample[r][i][c].x);
+      float at = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kRuns; ++i) {
+        const float2 q = S.sample[r][i][c];
+        most = fmaxf(most, __fadd_rn(fabsf(at), q.y));
+        back = fmaxf(back, __fadd_rn(fabsf(__fsub_rn(total, at)), q.y));
+        at = __fadd_rn(at, q.x);
+      }
+      atomicMax(&S.partial[c], __float_as_uint(__fadd_rn(most, back)));
     };
     // one digit of one half: three 16-byte stores per thread
     auto put_digit = [&](int h, float up) {
@@ -230,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         float d[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) d[c] = tfir::digit(x[h][g][c], up);
-        *reinterpret_cast<uint4*>(XD + h * tfir::kHalfBytes + (gw + 8 * g) * tfir::kBlockBytes +
+        *reinterpret_cast<uint4*>(XD + h * tfir::kHalfBytes + (3 * gw + g) * tfir::kBlockBytes +
                                   sec * 16) =
             make_uint4(tfir::pack2(d[0], d[1]), tfir::pack2(d[2], d[3]), tfir::pack2(d[4], d[5]),
                        tfir::pack2(d[6], d[7]));
@@ -238,136 +465,301 @@ __global__ void __launch_bounds__(kThreads, 1)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       half_ready(h);
     };
-    // phase `n` of mbar[h], bounded; false: every worker gives up
+    // Phase `n` of mbar[h].  Bounded; after a wait that ran out none waits, the
+    // tile goes on with what is there and the run ends with it.
     auto wait_half = [&](int h, int n) {
       uint32_t done = 0;
-      const unsigned long long start = global_ns();
+      unsigned long long start = 0;
       while (!done) {
         asm volatile(
             "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
             : "=r"(done)
             : "r"(smem_u32(&S.mbar[h])), "r"((uint32_t)(n & 1))
             : "memory");
-        if (!done && global_ns() - start > kWaitNs) break;
+        if (done) break;
+        if (*(volatile int*)&S.abort) break;
+        if (start == 0) start = global_ns();
+        if (global_ns() - start > kWaitNs) {
+          *(volatile int*)&S.abort = 1;
+          break;
+        }
       }
-      if (!done) *(volatile int*)&S.abort = 1;
-      sync_workers();
-      return *(volatile int*)&S.abort == 0;
+    };
+    auto next_digit = [&](int n) {
+      wait_half(0, n);
+      put_digit(0, 512.0f);
+      wait_half(1, n);
+      put_digit(1, 512.0f);
     };
 
-    // DC sums, IHC and lambda of tile t (dS and AC in shared memory): phase 2
-    // of ihc_lambda.cu's kernel.
-    auto finish_tile = [&](int t) {
-      const int row0 = t * tfir::kRows, k_hi = min(row0 + tfir::kRows, f.lam_rows);
-      const int dsbase = row0 - n_dc;
-      const float d = A.taps[n_ac];  // uniform DC taps
-      if (warp < 4 * kGroups) {
-        const int kb = row0 + (warp >> 1) * kDcAnchor;
-        const int ke = min(kb + kDcAnchor, k_hi);
-        const float* col = DS + sec;
-        float ws = 0.0f, wc = 0.0f;
-        int tu_prev = -1;
-        int sgm = kb < f.frdp - 1 ? f.seg : f.total;
-        int lim = (kb + 1) % sgm;
-#pragma unroll 4
-        for (int k = kb; k < ke; ++k) {
-          const int tu = lim < n_dc ? lim : n_dc;
-          const float x_new = col[(k - dsbase) * kPitch];
-          const float x_old = col[(k - tu - dsbase) * kPitch];
-          if (k == kb || (tu != tu_prev && tu != tu_prev + 1)) {
-            ws = wc = 0.0f;
-            for (int j = 0; j < tu; ++j) two_sum_add(ws, wc, col[(k - j - dsbase) * kPitch]);
+    // The steps that finish a tile, each between two barriers of the workers.
+    // at: ring row of the tile's first dS row.
+    auto dot2_points = [&](int t, int at) {
+      const int listed = S.listed, kb = t * tfir::kRows;
+      const bool all = listed > kList;
+      if (listed <= kFewPoints) {
+        // Few points: a warp to each.  Its lanes fetch the point's rows and the
+        // taps at once (one trip to L2 where a lane's own sequence of batches
+        // takes sixteen) and hand them round by shuffles, which do not wait for
+        // the shared memory that the products are reading.
+        for (int p = warp; p < listed; p += kIhcWarps) {
+          const int r = S.list[p] / kCols, c = S.list[p] % kCols;
+          const float* src = vf + (int64_t)(kb + r) * 256 + c;
+          const int taps = taps_used(kb + r, f, n_ac);
+          const bool sym = A.ac_sym && taps == n_ac;
+          const int half = n_ac / 2;
+          // lane + 32 i: the row of that tap, and of its mirror tap
+          float u[9], w[4], b[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) {
+            const int k = lane + 32 * i;
+            u[i] = k < taps ? __ldg(src - k * 256) : 0.0f;
+            b[i] = k < n_ac ? TP[k] : 0.0f;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int k = lane + 32 * i;
+            w[i] = sym && k < half ? __ldg(src - (n_ac - 1 - k) * 256) : 0.0f;
+          }
+          Dot2 acc;
+          acc.init();
+          // the value of lane q of the i-th register of v (i, q uniform)
+          auto from = [&](const float (&v)[9], int k) {
+            float r = v[0];
+#pragma unroll
+            for (int i = 1; i < 9; ++i) r = k >> 5 == i ? v[i] : r;
+            return __shfl_sync(kFull, r, k & 31);
+          };
+          if (sym) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll 1
+              for (int q = 0; q < 32 && 32 * i + q + 8 <= half; q += 8) {
+                float gb[8], gu[8], gw8[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  gb[e] = __shfl_sync(kFull, b[i], q + e);
+                  gu[e] = __shfl_sync(kFull, u[i], q + e);
+                  gw8[e] = __shfl_sync(kFull, w[i], q + e);
+                }
+                dot2_pairs(acc, gb, gu, gw8);
+              }
+            for (int k = half & ~7; k < half; ++k) acc.add_pair(from(b, k), from(u, k), from(u, n_ac - 1 - k));
+            if (n_ac & 1) acc.add(from(b, half), from(u, half));
           } else {
-            two_sum_add(ws, wc, x_new);
-            if (tu == tu_prev) two_sum_add(ws, wc, -x_old);
+#pragma unroll
+            for (int i = 0; i < 9; ++i)
+#pragma unroll 1
+              for (int q = 0; q < 32 && 32 * i + q + 8 <= taps; q += 8) {
+                float gb[8], gu[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  gb[e] = __shfl_sync(kFull, b[i], q + e);
+                  gu[e] = __shfl_sync(kFull, u[i], q + e);
+                }
+                dot2_taps(acc, gb, gu);
+              }
+            for (int k = taps & ~7; k < taps; ++k) acc.add(from(b, k), from(u, k));
           }
-          tu_prev = tu;
-          if (k + 1 == f.frdp - 1) {
-            sgm = f.total;
-            lim = (k + 2) % sgm;
-          } else if (++lim == sgm) {
-            lim = 0;
+          const float ac = acc.result();
+          const float ms = __fmaf_rn(u[0], A.scale, -ac);  // (lane 0's is the point's own)
+          int slot = at + r;
+          slot -= slot >= ring ? ring : 0;
+          if (lane == 0) {
+            AC[r * kPitch + c] = ac;
+            DS[slot * kPitch + c] = __fmul_rn(ms, ms);
           }
-          const float p = __fmul_rn(d, ws);
-          const float q = __fmaf_rn(d, ws, -p);
-          const float dc = __fadd_rn(p, __fmaf_rn(d, wc, q));
-          float& slot = AC[(k - row0) * kPitch + sec];
-          slot = __fmaf_rn(slot, A.eta_ac, __fmul_rn(dc, A.eta_dc));
         }
       }
-      sync_workers();
-      for (int kb = row0 + gw * kEmitRows; kb < k_hi; kb += 8 * kEmitRows) {
+      // first the rows that the products cannot give, a warp to 32 sections;
+      // then single points, as few warps as hold them (what a warp's sequence
+      // costs does not depend on its lanes), from the highest warp down
+      int row = all || S.dot2_rows[t & 1] ? gw : tfir::kRows;
+      int p = (kIhcWarps - 1 - warp) * 32 + lane;
+      while (true) {
+        int r, c;
+        if (row < tfir::kRows) {
+          const int kind = S.row[row];
+          r = row;
+          c = sec;
+          row += 8;
+          if (!(kind == kRowDot2 || (all && kind == kRowSum))) continue;
+        } else {
+          if (all || listed <= kFewPoints || p >= listed) break;
+          r = S.list[p] / kCols;
+          c = S.list[p] % kCols;
+          p += kWorkers;
+        }
+        const float* src = vf + (int64_t)(kb + r) * 256 + c;
+        const float ac =
+            dot2_row(src, TP, taps_used(kb + r, f, n_ac), n_ac, A.ac_sym != 0);
+        const float ms = __fmaf_rn(__ldg(src), A.scale, -ac);
+        int slot = at + r;
+        slot -= slot >= ring ? ring : 0;
+        AC[r * kPitch + c] = ac;
+        DS[slot * kPitch + c] = __fmul_rn(ms, ms);
+      }
+    };
+    // DC sums of ihc_lambda.cu's kernel: a warp per 32 rows and section half
+    auto dc_sums = [&](int t, int at) {
+      if (warp >= 4 * kGroups) return;
+      const float d = A.taps[n_ac];  // uniform DC taps
+      const int row0 = t * tfir::kRows, k_hi = min(row0 + tfir::kRows, f.lam_rows);
+      const int kb = row0 + gw * kDcAnchor, ke = min(kb + kDcAnchor, k_hi);
+      const float* col = DS + sec;
+      auto pre = [&](float ws, float wc, float ac) {
+        const float p = __fmul_rn(d, ws);
+        const float q = __fmaf_rn(d, ws, -p);
+        const float dc = __fadd_rn(p, __fmaf_rn(d, wc, q));
+        return __fmaf_rn(ac, A.eta_ac, __fmul_rn(dc, A.eta_dc));
+      };
+      if (kb >= ke) return;
+      int now = at + (kb - row0);  // ring row of k
+      now -= now >= ring ? ring : 0;
+      int sgm = kb < f.frdp - 1 ? f.seg : f.total;
+      int lim = (kb + 1) % sgm;
+      float* slot = AC + (kb - row0) * kPitch + sec;
+      float ws, wc;
+      if (ke - kb == kDcAnchor && lim >= n_dc && lim + kDcAnchor - 1 < sgm &&
+          (ke <= f.frdp - 1 || kb >= f.frdp - 1)) {
+        // every row of the block has the full window
+        window_sum(col, now, n_dc, ring, ws, wc);
+        slot[0] = pre(ws, wc, slot[0]);
+        int old = now >= n_dc ? now - n_dc : now - n_dc + ring;
+        // eight rows at a time (the first of them done)
+#pragma unroll 1
+        for (int r0 = 0; r0 < kDcAnchor; r0 += 8) {
+          float un[8], uo[8], ac[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            un[q] = col[now * kPitch];
+            uo[q] = col[old * kPitch];
+            ac[q] = slot[q * kPitch];
+            now = now + 1 == ring ? 0 : now + 1;
+            old = old + 1 == ring ? 0 : old + 1;
+          }
+          // the block's first row is done: adding and removing nothing keeps it
+          if (r0 == 0) un[0] = uo[0] = 0.0f;
+          float y[16], tw[8], tc[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            y[2 * q] = un[q];
+            y[2 * q + 1] = -uo[q];
+          }
+          two_sum_rows(ws, wc, y, tw, tc);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (r0 + q > 0) slot[q * kPitch] = pre(tw[q], tc[q], ac[q]);
+          slot += 8 * kPitch;
+        }
+        return;
+      }
+      ws = wc = 0.0f;
+      int tu_prev = -1;
+      for (int k = kb; k < ke; ++k) {
+        const int tu = lim < n_dc ? lim : n_dc;
+        if (k == kb || (tu != tu_prev && tu != tu_prev + 1)) {
+          ws = wc = 0.0f;
+          int i = now;
+          for (int j = 0; j < tu; ++j) {
+            two_sum_add(ws, wc, col[i * kPitch]);
+            i = i == 0 ? ring - 1 : i - 1;
+          }
+        } else {
+          two_sum_add(ws, wc, col[now * kPitch]);
+          const int old = now >= tu ? now - tu : now - tu + ring;
+          if (tu == tu_prev) two_sum_add(ws, wc, -col[old * kPitch]);
+        }
+        tu_prev = tu;
+        if (k + 1 == f.frdp - 1) {
+          sgm = f.total;
+          lim = (k + 2) % sgm;
+        } else if (++lim == sgm) {
+          lim = 0;
+        }
+        *slot = pre(ws, wc, *slot);
+        slot += kPitch;
+        now = now + 1 == ring ? 0 : now + 1;
+      }
+    };
+    auto emit = [&](int t, int from, int to) {
+      const int row0 = t * tfir::kRows, k_hi = min(row0 + to, f.lam_rows);
+      const float dmg = __ldg(A.dmg + (size_t)f.ihc_profile * 256 + s0 + sec);
+      const float a0 = __ldg(A.aihc + s0 + sec), a1 = __ldg(A.aihc + 256 + s0 + sec),
+                  a2 = __ldg(A.aihc + 512 + s0 + sec);
+      const bool sec0 = s0 + sec == 0;
+      for (int kb = row0 + from + gw * kEmitRows; kb < k_hi; kb += 8 * kEmitRows) {
         float lg[kEmitRows], l0[kEmitRows], l1[kEmitRows], l2[kEmitRows];
 #pragma unroll
-        for (int r = 0; r < kEmitRows; ++r) {
-          const int k = min(kb + r, k_hi - 1);
-          const float y = __fmul_rn(dmg, AC[(k - row0) * kPitch + sec]);
-          lg[r] = own_log10f(__fadd_rn(fmaxf(y, 0.0f), 1e-20f));
-          l0[r] = sec0 ? A.spont0 : fminf(A.sat, fmaxf(__fmul_rn(a0, lg[r]), A.spont0));
-          l1[r] = sec0 ? A.spont1 : fminf(A.sat, fmaxf(__fmul_rn(a1, lg[r]), A.spont1));
-          l2[r] = sec0 ? A.spont2 : fminf(A.sat, fmaxf(__fmul_rn(a2, lg[r]), A.spont2));
+        for (int r = 0; r < kEmitRows; r += 2) {
+          // (rows past the frame: what is there, not stored)
+          const float* pre = AC + (kb + r - row0) * kPitch + sec;
+          const float2 y = mul2(f2b(dmg), f2(pre[0], pre[kPitch]));
+          const float2 g2 =
+              own_log10f2(add2(f2(fmaxf(y.x, 0.0f), fmaxf(y.y, 0.0f)), f2b(1e-20f)));
+          const float2 m0 = mul2(f2b(a0), g2), m1 = mul2(f2b(a1), g2), m2 = mul2(f2b(a2), g2);
+          lg[r] = g2.x;
+          lg[r + 1] = g2.y;
+          l0[r] = sec0 ? A.spont0 : fminf(A.sat, fmaxf(m0.x, A.spont0));
+          l1[r] = sec0 ? A.spont1 : fminf(A.sat, fmaxf(m1.x, A.spont1));
+          l2[r] = sec0 ? A.spont2 : fminf(A.sat, fmaxf(m2.x, A.spont2));
+          l0[r + 1] = sec0 ? A.spont0 : fminf(A.sat, fmaxf(m0.y, A.spont0));
+          l1[r + 1] = sec0 ? A.spont1 : fminf(A.sat, fmaxf(m1.y, A.spont1));
+          l2[r + 1] = sec0 ? A.spont2 : fminf(A.sat, fmaxf(m2.y, A.spont2));
         }
+        const int64_t at = (f.lam_row0 + kb) * 256 + s0 + sec;
+        const int64_t plane = A.lam_plane_rows * 256;
+        float* out = A.lam + at;
 #pragma unroll
         for (int r = 0; r < kEmitRows; ++r) {
           if (kb + r < k_hi) {
-            const int64_t at = (f.lam_row0 + kb + r) * 256 + s0 + sec;
-            const int64_t plane = A.lam_plane_rows * 256;
-            A.lam[at] = l0[r];
-            A.lam[plane + at] = l1[r];
-            A.lam[2 * plane + at] = l2[r];
-            if (A.ihc) A.ihc[at] = lg[r];
+            out[r * 256] = l0[r];
+            out[plane + r * 256] = l1[r];
+            out[2 * plane + r * 256] = l2[r];
+            if (A.ihc) A.ihc[at + r * 256] = lg[r];
             if (A.lam_host) {
-              A.lam_host[at] = l0[r];
-              A.lam_host[plane + at] = l1[r];
-              A.lam_host[2 * plane + at] = l2[r];
+              A.lam_host[at + r * 256] = l0[r];
+              A.lam_host[plane + at + r * 256] = l1[r];
+              A.lam_host[2 * plane + at + r * 256] = l2[r];
             }
           }
         }
       }
-      sync_workers();
-    };
-    // dS of the next tile's look-back: n_dc rows down by a tile, in steps that
-    // do not overlap
-    auto shift_ds = [&]() {
-      for (int i0 = 0; i0 < n_dc; i0 += tfir::kRows) {
-        const int i1 = min(i0 + tfir::kRows, n_dc);
-        for (int i = i0 + gw; i < i1; i += 8)
-          DS[i * kPitch + sec] = DS[(i + tfir::kRows) * kPitch + sec];
-        sync_workers();
-      }
     };
 
+    if (threadIdx.x == 0) S.kmin[first & 1] = window_start(first * tfir::kRows);
+    sync_workers();
     load_tile(first);
-    bool ok = true;
-    int n = 0;  // completed phases of each half's barrier
+    int n = 0;       // completed phases of each half's barrier
+    int at = 0;      // ring row of the tile's first dS row
+    int at_prev = 0; // and of the tile before
     for (int t = first; t < t1; ++t, n += tfir::kDigits) {
       const int kb = t * tfir::kRows, k_hi = min(kb + tfir::kRows, f.lam_rows);
-      // scales: the exponent of the section's largest |x|
+      // scales: the exponent of the section's largest |x| (a NaN is not seen
+      // here: it makes every sum of its section a NaN, which Dot2 then replaces)
       uint32_t* top = S.top[t & 1];
       {
-        uint32_t m = 0;
+        float m = 0.0f;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int g = 0; g < 3; ++g)
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-              m = max(m, __float_as_uint(x[h][g][c]) & 0x7fffffffu);
-        atomicMax(&top[sec], m);
+            for (int c = 0; c < 8; ++c) m = fmaxf(m, fabsf(x[h][g][c]));
+        atomicMax(&top[sec], __float_as_uint(m));
       }
+      sample_runs();
       sync_workers();
       const uint32_t m = top[sec];
       const int e = (int)(m >> 23) - 126;  // 2^(e-1) <= largest |x| < 2^e
       // magnitudes whose digits and result are far from the ends of the FP32
-      // range; infinities and NaN have e = 129
+      // range; an infinity has e = 129
       const bool usable = e >= -80 && e <= 100;
-      if (threadIdx.x < kCols) {
-        const uint32_t mm = top[threadIdx.x];
-        const int ee = (int)(mm >> 23) - 126;
-        const bool uu = ee >= -80 && ee <= 100;
-        S.slack[threadIdx.x] = mm == 0 ? 0.0f : (uu ? slack : __int_as_float(0x7f800000));
-        S.unit[threadIdx.x] = uu ? __int_as_float((127 + ee + exp_b - 16) << 23) : 1.0f;
-        S.top[(t + 1) & 1][threadIdx.x] = 0;
+      if (warp < kGroups && gw == 0) {
+        S.scale[sec] =
+            make_float2(m == 0 ? 0.0f : (usable ? 0x1p-31f : __int_as_float(0x7f800000)),
+                        usable ? __int_as_float((127 + e + exp_b - 16) << 23) : 1.0f);
+        S.top[(t + 1) & 1][sec] = 0;
       }
       const float up = usable ? __int_as_float((127 + 8 - e) << 23) : 0.0f;
       if (!usable) {  // (0 times an infinity is no digit)
@@ -380,102 +772,135 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       put_digit(0, up);
       put_digit(1, up);
-      if (t > first) {
-        if (t > t0) finish_tile(t - 1);
-        shift_ds();
+      if (warp >= 8 && warp < 12) sampled_partial((warp >> 1) & 1, 32 * (warp & 1) + lane);
+      sync_workers();
+      // the tile before, between the digits of this one
+      const bool prev = t > first, prev_out = t > t0;
+      if (prev) dot2_points(t - 1, at_prev);
+      next_digit(n);
+      sync_workers();
+      if (threadIdx.x == 0) {
+        S.listed = 0;
+        S.dot2_rows[(t + 1) & 1] = 0;
+        S.kmin[(t + 1) & 1] = window_start((t + 1) * tfir::kRows);
       }
-      for (int i = 1; i < tfir::kDigits && ok; ++i) {
+      if (prev_out) dc_sums(t - 1, at_prev);
+      if (warp >= 12) classify(t, (int)threadIdx.x - 384);
+      next_digit(n + 1);
+      sync_workers();
+      // slack of the rounding test (head of the file)
+      if (warp < kGroups && gw == 0) {
+        S.scale[sec].x += __fdiv_rn(__uint_as_float(S.partial[sec]) * 0x1.4p-43f, S.scale[sec].y);
+        S.partial[sec] = 0;
+      }
+      if (prev_out) emit(t - 1, 0, tfir::kRows / 2);
+      next_digit(n + 2);
+      if (prev_out) emit(t - 1, tfir::kRows / 2, tfir::kRows);
+      next_digit(n + 3);
+      // the row's velocity, for dS
+      const int row = (warp & 3) * 32 + lane, cols = (warp >> 2) * 16;
+      float4 own[4];
+      {
+        const float4* src =
+            reinterpret_cast<const float4*>(vf + (int64_t)(kb + row) * 256 + cols);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (ok && !(ok = wait_half(h, n + i - 1))) half_ready(h);  // wakes the issuing warp
-          if (ok) put_digit(h, 512.0f);
-        }
+        for (int i = 0; i < 4; ++i)
+          own[i] = kb + row < k_hi ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
-      if (!ok) break;
-      if (t + 1 < t1) load_tile(t + 1);
-      ok = wait_half(0, n + tfir::kDigits - 1);
-      if (ok) ok = wait_half(1, n + tfir::kDigits - 1);
-      if (!ok) {
-        if (t + 1 < t1) half_ready(0);
-        break;
-      }
+      wait_half(0, n + 4);
+      wait_half(1, n + 4);
+      sync_workers();
       tfir::fence_after();
 
       // Epilogue: lane = row, sixteen sections per thread.  The digits' sum as
       // an unevaluated FP32 pair h + c, rounded once.
-      uint16_t* list = reinterpret_cast<uint16_t*>(XD);  // free until the next digit
       {
-        const int r = (warp & 3) * 32 + lane, k = kb + r;
-        const int tu = k < k_hi ? taps_used(k, f, n_ac) : 0;
-        const int kmin = window_start(kb);
-        const bool fits = (tu == n_ac && k - n_ac + 1 >= kmin) || k - tu + 1 == kmin;
+        const int kind = S.row[row];
+        int slot = at + row;
+        slot -= slot >= ring ? ring : 0;
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
-          const int c0 = (warp >> 2) * 16 + part * 8;
-          const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0;
-          float G[tfir::kDigits][8];
+          const int c0 = cols + part * 8;
+          const uint32_t from = tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0;
+          float G[tfir::kSums][8];
 #pragma unroll
-          for (int m2 = 0; m2 < tfir::kDigits; ++m2) tfir::tmem_load8(at + kCols * m2, G[m2]);
+          for (int i = 0; i < tfir::kSums; ++i) tfir::tmem_load8(from + kCols * i, G[i]);
           tfir::tmem_wait_loads();
           uint32_t bad = 0;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float q = 1.0f / 512.0f;
-            float e2, e1, e0;
-            const float g3 = __fmaf_rn(G[4][c], q, G[3][c]);
-            const float h2 = two_sum(G[2][c], __fmul_rn(g3, q), e2);
-            const float h1 = two_sum(G[1][c], __fmul_rn(h2, q), e1);
-            const float h0 = two_sum(G[0][c], __fmul_rn(h1, q), e0);
-            const float lo = __fmaf_rn(__fmaf_rn(e2, q, e1), q, e0);
-            const float res = __fadd_rn(h0, lo);
-            const float rest = __fsub_rn(lo, __fsub_rn(res, h0));
-            const float sl = S.slack[c0 + c];
-            const float ac = __fmul_rn(res, S.unit[c0 + c]);
-            const bool sure = __fadd_rn(res, __fadd_rn(rest, sl)) == res &&
-                              __fadd_rn(res, __fsub_rn(rest, sl)) == res &&
-                              (sl == 0.0f || fabsf(ac) > 1e-30f);
-            AC[r * kPitch + c0 + c] = tu == 0 ? 0.0f : ac;
-            if (tu > 0 && !(fits && sure)) bad |= 1u << c;
+          for (int c = 0; c < 8; c += 2) {
+            const float2 q = f2b(1.0f / 512.0f);
+            float2 g[tfir::kSums];
+#pragma unroll
+            for (int i = 0; i < tfir::kSums; ++i) g[i] = f2(G[i][c], G[i][c + 1]);
+            float2 e2, e1, e0;
+            const float2 g3 = fma2(fma2(g[5], q, g[4]), q, g[3]);
+            const float2 h2 = two_sum2(g[2], mul2(g3, q), e2);
+            const float2 h1 = two_sum2(g[1], mul2(h2, q), e1);
+            const float2 h0 = two_sum2(g[0], mul2(h1, q), e0);
+            const float2 lo = fma2(fma2(e2, q, e1), q, e0);
+            const float2 res = add2(h0, lo);
+            const float2 rest = sub2(lo, sub2(res, h0));
+            const float4 sc = *reinterpret_cast<const float4*>(&S.scale[c0 + c]);
+            const float2 slack = f2(sc.x, sc.z);
+            float2 ac = mul2(res, f2(sc.y, sc.w));
+            const float2 up = add2(res, add2(rest, slack)), down = add2(res, sub2(rest, slack));
+            const float least = 1e-30f;  // (far from where the unit's product would round)
+            if (!(up.x == res.x && down.x == res.x && (sc.x == 0.0f || fabsf(ac.x) > least)))
+              bad |= 1u << c;
+            if (!(up.y == res.y && down.y == res.y && (sc.z == 0.0f || fabsf(ac.y) > least)))
+              bad |= 2u << c;
+            if (kind == kRowZero) ac = f2b(0.0f);
+            const float4 o = own[2 * part + c / 4];
+            const float2 ms = fma2(c & 2 ? f2(o.z, o.w) : f2(o.x, o.y), f2b(A.scale), neg2(ac));
+            const float2 ds = mul2(ms, ms);
+            AC[row * kPitch + c0 + c] = ac.x;
+            AC[row * kPitch + c0 + c + 1] = ac.y;
+            DS[slot * kPitch + c0 + c] = ds.x;
+            DS[slot * kPitch + c0 + c + 1] = ds.y;
           }
-          if (bad) {
+          if (kind == kRowSum && bad) {
             int p = atomicAdd(&S.listed, __popc(bad));
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-              if (bad >> c & 1) list[p++] = (uint16_t)(r * kCols + c0 + c);
+              if (bad >> c & 1) {
+                if (p < kList) S.list[p] = (uint16_t)(row * kCols + c0 + c);
+                ++p;
+              }
           }
         }
       }
+      if (t + 1 < t1) load_tile(t + 1);
       tfir::fence_before();
       sync_workers();
-      const int listed = S.listed;
-      for (int p = threadIdx.x; p < listed; p += kWorkers) {
-        const int q = list[p], r = q / kCols, c = q - r * kCols;
-        AC[r * kPitch + c] = dot2_row(vf + (int64_t)(kb + r) * 256 + c, TP,
-                                      taps_used(kb + r, f, n_ac), n_ac, A.ac_sym != 0);
+      at_prev = at;
+      at += tfir::kRows;
+      at -= at >= ring ? ring : 0;
+      if (*(volatile int*)&S.abort) {
+        if (threadIdx.x == 0) {
+          S.stop = 1;
+          atomicOr(A.status, 1);
+        }
+        sync_workers();
+        if (t + 1 < t1) half_ready(0);
+        break;
       }
-      sync_workers();
-      if (threadIdx.x == 0) S.listed = 0;
-      // dS of the tile's rows
-#pragma unroll 4
-      for (int r = gw; r < k_hi - kb; r += 8) {
-        const float xv = __ldg(vf + (int64_t)(kb + r) * 256 + sec);
-        const float ms = __fmaf_rn(xv, A.scale, -AC[r * kPitch + sec]);
-        DS[(n_dc + r) * kPitch + sec] = __fmul_rn(ms, ms);
-      }
-      sync_workers();
     }
-    if (ok)
-      finish_tile(t1 - 1);
-    else if (threadIdx.x == 0)
-      atomicOr(A.status, 1);
+    if (!*(volatile int*)&S.abort) {
+      dot2_points(t1 - 1, at_prev);
+      sync_workers();
+      dc_sums(t1 - 1, at_prev);
+      sync_workers();
+      emit(t1 - 1, 0, tfir::kRows);
+    }
   }
   __syncthreads();
   if (warp == kIhcWarps) tfir::tmem_free(tmem);
 }
 
-size_t tensor_smem(int n_ac, int n_dc) {
+size_t tensor_smem(int n_dc) {
   return 2 * (size_t)tfir::kHalfBytes + tfir::kTapBytes +
-         ((size_t)n_dc + 2 * tfir::kRows) * kPitch * 4 + (size_t)n_ac * 4 + 16 +
+         ((size_t)n_dc + 2 * tfir::kRows) * kPitch * 4 + (size_t)(tfir::kRows + tfir::kDepth) * 4 + 16 +
          sizeof(TensorShared);
 }
 
@@ -483,17 +908,16 @@ size_t tensor_smem(int n_ac, int n_dc) {
 
 bool ihc_tensor_fits(int n_ac, int n_dc) {
   return n_ac >= kTensorMinTaps && n_ac <= tfir::kMaxTaps &&
-         tensor_smem(n_ac, n_dc) <= 227 * 1024;
+         tensor_smem(n_dc) <= 227 * 1024;
 }
 
-int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b, float slack,
+int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b,
                       cudaStream_t st) {
-  const size_t smem = tensor_smem(A.n_ac, A.n_dc);
+  const size_t smem = tensor_smem(A.n_dc);
   CGB_TRY_CUDA(cudaFuncSetAttribute(ihc_tensor_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(ihc tensor smem)");
-  ihc_tensor_kernel<<<dim3((unsigned)n_runs, 256 / kCols), kThreads, smem, st>>>(A, d_v, exp_b,
-                                                                                 slack);
+  ihc_tensor_kernel<<<dim3((unsigned)n_runs, 256 / kCols), kThreads, smem, st>>>(A, d_v, exp_b);
   CGB_TRY_CUDA(cudaGetLastError(), "ihc_tensor_kernel launch");
   note_launch();
   return CGB_OK;

@@ -15,9 +15,8 @@ constexpr int kTensorSections = 64;
 
 // Whether the filters' lengths fit the kernel (taps of one tile, shared memory).
 bool ihc_tensor_fits(int n_ac, int n_dc);
-// exp_b: the exponent of the largest |tap| (2^(exp_b-1) <= it < 2^exp_b);
-// slack: see ihc_tensor.cu.
-int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b, float slack,
+// exp_b: the exponent of the largest |tap| (2^(exp_b-1) <= it < 2^exp_b).
+int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b,
                       cudaStream_t st);
 
 }  // namespace cgb

@@ -8,10 +8,10 @@
 // |X_i|, |B_j| <= 256 (rounded to nearest, so signed), e and eb the exponents
 // of the largest magnitude of a section's 384 rows and of the taps.  Integers
 // up to 256 are exact in BF16, and the products of two digits summed over the
-// taps stay below 2^24, so the FP32 accumulators hold exact integers.  The 15
-// digit pairs with i + j <= 4 go to five accumulators G_m, m = i + j:
-//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  an error of about 2^-41 of the
-// product of the two scales.
+// taps stay below 2^24, so the FP32 accumulators hold exact integers.  The 19
+// digit pairs with i + j <= 5 go to six accumulators G_m, m = i + j:
+//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  an error of about 2^-50 of the
+// product of the two scales (2^-41 with the 15 pairs up to i + j = 4).
 //
 // T has one value per diagonal.  With the rows of x stored in reverse order its
 // band is a Hankel matrix (element (r, k') depends on r + k'), and a Hankel
@@ -40,13 +40,14 @@ constexpr int kCols = 64;            // sections of a tile (N)
 constexpr int kDepth = 384;          // rows of x of a tile (K)
 constexpr int kHalf = kDepth / 2;    // rows in one of the two buffers of a digit
 constexpr int kDigits = 5;
+constexpr int kSums = 6;             // accumulators
 constexpr int kMaxTaps = kDepth - kRows + 1;
 constexpr int kCores = (kRows + kDepth) / 8 - 1;  // block diagonals of the band
 constexpr int kTapDigit = kCores * 128;           // bytes of a digit of the band
 constexpr int kTapBytes = kDigits * kTapDigit;
 constexpr int kBlockBytes = kCols * 16;           // eight rows of a digit of x
 constexpr int kHalfBytes = kHalf / 8 * kBlockBytes;
-constexpr uint32_t kTmemCols = 512;               // five accumulators of 64 columns
+constexpr uint32_t kTmemCols = 512;               // six accumulators of 64 columns
 
 __device__ __forceinline__ uint32_t saddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -98,15 +99,15 @@ __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t
 }
 
 // The products of one digit i of x, half h of its rows, with the tap digits j
-// up to 4 - i; called by a converged warp.  Accumulator m at column 64 m of
-// tmem; the first products of a tile (digit 0, half 0) start the accumulators.
+// up to 5 - i; called by a converged warp.  Accumulator m at column 64 m of
+// tmem, started by its first product of the tile.
 __device__ __forceinline__ void products(uint32_t taps, uint32_t rows, uint32_t tmem, int i,
                                          int h, uint32_t issue) {
   const uint64_t b0 = operand(rows, kBlockBytes, 128);
   const uint64_t a0 = operand(taps + h * (kHalf / 8) * 128, 128, 128);
-  const uint32_t add = (i | h) ? 1u : 0u;
 #pragma unroll 1
-  for (int j = 0; j + i < kDigits; ++j) {
+  for (int j = 0; j < kDigits && j + i < kSums; ++j) {
+    const uint32_t add = h > 0 || (i > 0 && i + j < kDigits) || i > 1 ? 1u : 0u;
     const uint64_t a = a0 + (uint64_t)((j * kTapDigit) >> 4);
     const uint32_t d = tmem + kCols * (i + j);
 #pragma unroll
