@@ -3,9 +3,11 @@
 // (CudaCalculateJND = GlobalCalculateMeanRate + GlobalCalculateJND,
 // src/cochlea.cu:3741-3944, 3946-4065; final dB src/AudioGramCreator.cpp:454-508).
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "cgb_device.cuh"
@@ -71,10 +73,13 @@ __global__ void hearing_aid_iir_kernel(const float* __restrict__ aux, float* __r
   out[base + n] = acc;
 }
 
-constexpr int kJndSections = 256;
-constexpr int kJndGroups = 4;   // row groups per CTA (threads = 4 x 256)
+constexpr int kJndSections = 32;   // sections per CTA (one per lane)
+constexpr int kJndCluster = 8;     // CTAs per interval and plane: all 256 sections
+constexpr int kJndGroups = 4;      // row groups per CTA (a warp each)
 constexpr int kJndThreads = kJndSections * kJndGroups;
-constexpr int kJndRows = 8;     // rows per block of the walk
+constexpr int kJndRows = 8;        // rows per block of the walk
+constexpr int kJndStages = 4;      // blocks in flight per warp, through shared memory
+constexpr int kJndAhead = 2;       // blocks in flight per warp, in registers
 
 // A compensated FP32 sum (Kahan summation): s - c carries the sum of the
 // added terms with an error of about 2 ulp of the total plus n eps^2 times
@@ -91,16 +96,34 @@ struct KahanF {
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
-// The Fisher sums of one (interval, lambda plane): thread (g, s) walks the
-// 8-row blocks b = g, g + 4, ... of the window of section s and of the same
-// rows of the reference window, summing lambda and lambda_ref (the two mean
-// rates) and (lambda - lambda_ref)^2 / lambda_ref (the AI term).  Each term
-// is formed in FP32 and added to a compensated FP32 sum (KahanF), so the
-// walk needs no FP64 operation (GB300's FP64 rate would bound it).  Rows past
-// the last full block are added by the group that owns the next block.  The
-// four groups' sums are then combined in FP64 in group order and the 256
-// section terms reduced in FP64, so the result does not depend on
-// scheduling.
+// Asynchronous copy of BYTES (4 or 16, both sides aligned to them) into shared
+// memory.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(float* to, const float* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(to)),
+               "l"(from), "n"(BYTES)
+               : "memory");
+}
+
+// The Fisher sums of one (interval, lambda plane), by a cluster of eight CTAs of
+// 32 sections: thread (g, s) walks the 8-row blocks b = g, g + 4, ... of the
+// window of section s and of the same rows of the reference window, summing
+// lambda and lambda_ref (the two mean rates) and (lambda - lambda_ref)^2 /
+// lambda_ref (the AI term).  Each term is formed in FP32 and added to a
+// compensated FP32 sum (KahanF), so the walk needs no FP64 operation (GB300's
+// FP64 rate would bound it).  Rows past the last full block are added by the
+// group that owns the next block.  The four groups' sums are then combined in
+// FP64 in group order, a warp reduces its 32 section terms, and the cluster's
+// first CTA adds the eight CTAs' terms in order, so the result does not depend
+// on scheduling.
+//
+// What bounded it: the trip of a block's loads to memory (1,400 cycles for 8 rows
+// of both windows) on few SMs: one CTA of 1,024 threads per interval and plane
+// kept 33 of 152 SMs busy for 11 intervals.  As clusters they are 264 CTAs, and
+// more blocks are in flight per warp.  Measured (GB300): 11 intervals of 8,465
+// rows 339 -> 125 us, 3 of 18,400 677 -> 139, the JND sweep's 264 1,997 -> 1,572.
+template <bool ASYNC, bool WIDE>
 __device__ __forceinline__ void jnd_interval(const float* __restrict__ lam, int64_t plane_rows,
                                              int j, int64_t row, int64_t ref_row, int len,
                                              double da, int out, int n_out,
@@ -108,27 +131,93 @@ __device__ __forceinline__ void jnd_interval(const float* __restrict__ lam, int6
                                              double Fs, double T, double* __restrict__ F_RA,
                                              double* __restrict__ F_AI,
                                              double* __restrict__ MR) {
-  const int s = threadIdx.x & (kJndSections - 1), g = threadIdx.x / kJndSections;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  auto started = cluster.barrier_arrive();  // (the first CTA is there before it is written to)
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int rank = (int)cluster.block_rank(), s = rank * kJndSections + lane;
   const float* c = lam + ((int64_t)j * plane_rows + row) * 256 + s;
   const float* rf = lam + ((int64_t)j * plane_rows + ref_row) * 256 + s;
   KahanF kc, kr, ka;
   const int nb = len / kJndRows;
-  // two blocks per pass keep twice the loads in flight (same order of sums)
-#pragma unroll 2
-  for (int b = g; b < nb; b += kJndGroups) {
-    const int t = b * kJndRows;
-    float lc[kJndRows], lr[kJndRows];
-#pragma unroll
-    for (int k = 0; k < kJndRows; ++k) {
-      lc[k] = c[(int64_t)(t + k) * 256];
-      lr[k] = rf[(int64_t)(t + k) * 256];
-    }
+  auto sum = [&](const float (&lc)[kJndRows], const float (&lr)[kJndRows]) {
 #pragma unroll
     for (int k = 0; k < kJndRows; ++k) {
       const float d = __fsub_rn(lc[k], lr[k]);
       kc.add(lc[k]);
       kr.add(lr[k]);
       ka.add(__fmul_rn(__fmul_rn(d, d), own_rcpf(lr[k])));
+    }
+  };
+  if (ASYNC) {
+    // The warp's blocks come through a ring of stages in shared memory, copied
+    // asynchronously: kJndStages blocks of both windows (2 KB each) are in flight
+    // while one is summed.  Registers do not do: a warp's loads share a few
+    // scoreboards, so that waiting for the oldest waits for later ones too.
+    __shared__ __align__(16) float stage[kJndGroups][ASYNC ? kJndStages : 1][2][kJndRows]
+                                       [kJndSections];
+    const int mine = nb > g ? (nb - g + kJndGroups - 1) / kJndGroups : 0;  // the group's blocks
+    auto fetch = [&](int i) {
+      if (i < mine) {
+        const int64_t t = (int64_t)(g + i * kJndGroups) * kJndRows;
+        float(*to)[kJndRows][kJndSections] = stage[g][i % kJndStages];
+        if (WIDE) {  // 16 bytes a lane: eight lanes to a row's 32 sections
+          const int r = lane >> 3, q = 4 * (lane & 7);
+#pragma unroll
+          for (int k = 0; k < kJndRows; k += 4) {
+            copy_async<16>(&to[0][k + r][q], c - lane + (t + k + r) * 256 + q);
+            copy_async<16>(&to[1][k + r][q], rf - lane + (t + k + r) * 256 + q);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < kJndRows; ++k) {
+            copy_async<4>(&to[0][k][lane], c + (t + k) * 256);
+            copy_async<4>(&to[1][k][lane], rf + (t + k) * 256);
+          }
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll 1
+    for (int i = 0; i < kJndStages; ++i) fetch(i);
+#pragma unroll 1
+    for (int i = 0; i < mine; ++i) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kJndStages - 1) : "memory");
+      __syncwarp();
+      const float(*from)[kJndRows][kJndSections] = stage[g][i % kJndStages];
+      float lc[kJndRows], lr[kJndRows];
+#pragma unroll
+      for (int k = 0; k < kJndRows; ++k) {
+        lc[k] = from[0][k][lane];
+        lr[k] = from[1][k][lane];
+      }
+      __syncwarp();
+      fetch(i + kJndStages);
+      sum(lc, lr);
+    }
+  } else {
+    // the next blocks' loads are in flight while a block is summed
+    auto block = [&](int b, float (&lc)[kJndRows], float (&lr)[kJndRows]) {
+      const int64_t t = (int64_t)b * kJndRows;
+#pragma unroll
+      for (int k = 0; k < kJndRows; ++k) {
+        lc[k] = c[(t + k) * 256];
+        lr[k] = rf[(t + k) * 256];
+      }
+    };
+    float lc[kJndAhead][kJndRows], lr[kJndAhead][kJndRows];
+#pragma unroll
+    for (int a = 0; a < kJndAhead; ++a)
+      if (g + a * kJndGroups < nb) block(g + a * kJndGroups, lc[a], lr[a]);
+    for (int b = g; b < nb; b += kJndAhead * kJndGroups) {
+#pragma unroll
+      for (int a = 0; a < kJndAhead; ++a) {
+        const int now = b + a * kJndGroups, next = now + kJndAhead * kJndGroups;
+        if (now < nb) {
+          sum(lc[a], lr[a]);
+          if (next < nb) block(next, lc[a], lr[a]);
+        }
+      }
     }
   }
   if (g == nb % kJndGroups) {
@@ -143,16 +232,17 @@ __device__ __forceinline__ void jnd_interval(const float* __restrict__ lam, int6
   }
   double sum_c = kc.value(), sum_r = kr.value(), sum_ai = ka.value();
   __shared__ double sh[3][kJndGroups][kJndSections];
-  __shared__ double red[2][kJndSections / 32];
-  sh[0][g][s] = sum_c;
-  sh[1][g][s] = sum_r;
-  sh[2][g][s] = sum_ai;
+  __shared__ double red[2][kJndCluster];  // the first CTA's: the terms of all eight
+  sh[0][g][lane] = sum_c;
+  sh[1][g][lane] = sum_r;
+  sh[2][g][lane] = sum_ai;
+  cluster.barrier_wait(std::move(started));
   __syncthreads();
   if (g == 0) {
     for (int k = 1; k < kJndGroups; ++k) {
-      sum_c += sh[0][k][s];
-      sum_r += sh[1][k][s];
-      sum_ai += sh[2][k][s];
+      sum_c += sh[0][k][lane];
+      sum_r += sh[1][k][lane];
+      sum_ai += sh[2][k][lane];
     }
     const double mr = sum_c / len, mrr = sum_r / len;
     if (MR) MR[((int64_t)j * n_out + out) * 256 + s] = mr;
@@ -168,15 +258,16 @@ __device__ __forceinline__ void jnd_interval(const float* __restrict__ lam, int6
       rate += __shfl_xor_sync(kFull, rate, o);
       ai += __shfl_xor_sync(kFull, ai, o);
     }
-    if ((s & 31) == 0) {
-      red[0][s >> 5] = rate;
-      red[1][s >> 5] = ai;
+    if (lane == 0) {
+      double* first = cluster.map_shared_rank(&red[0][0], 0);
+      first[rank] = rate;
+      first[kJndCluster + rank] = ai;
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  cluster.sync();  // (the first CTA's shared memory stays until it has all terms)
+  if (rank == 0 && threadIdx.x == 0) {
     double tr = 0.0, ta = 0.0;
-    for (int k = 0; k < kJndSections / 32; ++k) {
+    for (int k = 0; k < kJndCluster; ++k) {
       tr += red[0][k];
       ta += red[1][k];
     }
@@ -187,31 +278,50 @@ __device__ __forceinline__ void jnd_interval(const float* __restrict__ lam, int6
 
 // Intervals of one run: interval i's window starts at row i * interval_nodes
 // + head, its reference's at ref_of[i] * interval_nodes + head.
-__global__ void __launch_bounds__(kJndThreads)
+template <bool ASYNC, bool WIDE>
+__global__ void __cluster_dims__(kJndCluster, 1, 1) __launch_bounds__(kJndThreads)
     jnd_kernel(const float* __restrict__ lam, int64_t plane_rows, int interval_nodes, int head,
                int len, const double* __restrict__ dA, const int32_t* __restrict__ ref_of,
                const double* __restrict__ nihc, double w0, double w1, double w2, double Fs,
                double T, double* __restrict__ F_RA, double* __restrict__ F_AI,
                double* __restrict__ MR, int n_int) {
-  const int i = blockIdx.x, j = blockIdx.y;
-  jnd_interval(lam, plane_rows, j, (int64_t)i * interval_nodes + head,
+  const int i = blockIdx.x / kJndCluster, j = blockIdx.y;
+  jnd_interval<ASYNC, WIDE>(lam, plane_rows, j, (int64_t)i * interval_nodes + head,
                (int64_t)ref_of[i] * interval_nodes + head, len, dA[i], i, n_int, nihc,
                j == 0 ? w0 : (j == 1 ? w1 : w2), Fs, T, F_RA, F_AI, MR);
 }
 
 // Intervals of any number of runs (groups of signals of different lengths)
 // in one launch, from a descriptor table.
-__global__ void __launch_bounds__(kJndThreads)
+template <bool ASYNC, bool WIDE>
+__global__ void __cluster_dims__(kJndCluster, 1, 1) __launch_bounds__(kJndThreads)
     jnd_batch_kernel(const float* __restrict__ lam, int64_t plane_rows,
                      const cgb_jnd_interval* __restrict__ iv, int n_out,
                      const double* __restrict__ nihc, double w0, double w1, double w2, double Fs,
                      double T, double* __restrict__ F_RA, double* __restrict__ F_AI,
                      double* __restrict__ MR) {
-  // CTA b: descriptor b / 3, plane b % 3 (table order, planes together)
-  const int b = (int)blockIdx.x, i = b / 3, j = b - 3 * i;
+  // cluster b: descriptor b / 3, plane b % 3 (table order, planes together)
+  const int b = (int)blockIdx.x / kJndCluster, i = b / 3, j = b - 3 * i;
   const cgb_jnd_interval d = iv[i];
-  jnd_interval(lam, plane_rows, j, d.row, d.ref_row, d.len, d.dA, d.out, n_out, nihc,
+  jnd_interval<ASYNC, WIDE>(lam, plane_rows, j, d.row, d.ref_row, d.len, d.dA, d.out, n_out, nihc,
                j == 0 ? w0 : (j == 1 ? w1 : w2), Fs, T, F_RA, F_AI, MR);
+}
+
+// Which copies of the windows the kernel makes.  Few clusters: asynchronous ones
+// through shared memory, which keep more in flight per warp (5 intervals of 8,465
+// rows 78 us against 201, 11 of 8,465 125 / 204, 16 of 3,400 77 / 97, 21 of 3,400
+// 95 / 100); from 3.5 CTAs per SM on the loads to registers of many warps take
+// their place, at a quarter of the cost per row once the SMs are full (26 of 3,400
+// 113 / 104, 41 of 8,465 367 / 273, the JND sweep 2,356 / 1,572).  Rows start on 1
+// KB multiples from the planes' base, so the base decides whether a lane can copy
+// 16 bytes at a time.
+int jnd_copies(const float* lam, long long ctas) {
+  int dev = 0, n_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    n_sm = 0;
+  if (2 * ctas > 7LL * n_sm) return 0;
+  return (reinterpret_cast<uintptr_t>(lam) & 15) == 0 ? 2 : 1;
 }
 
 }  // namespace
@@ -253,11 +363,15 @@ extern "C" int cgb_jnd_dev(const float* d_lam, int64_t plane_rows, int n_int, in
     return fail(CGB_ERR_ARG, "cgb_jnd_dev: bad arguments");
   if ((int64_t)n_int * interval_nodes > plane_rows || head + len > interval_nodes)
     return fail(CGB_ERR_RANGE, "cgb_jnd_dev: intervals reach outside the lambda planes");
-  if (n_int > 2147483647 / 2) return fail(CGB_ERR_RANGE, "cgb_jnd_dev: too many intervals");
+  if (n_int > 2147483647 / kJndCluster) return fail(CGB_ERR_RANGE, "cgb_jnd_dev: too many intervals");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const double T = delta_alpha_len_factor / Fs;
-  dim3 grid((unsigned)n_int, 3);
-  jnd_kernel<<<grid, kJndThreads, 0, st>>>(d_lam, plane_rows, interval_nodes, head, len, d_dA,
+  dim3 grid((unsigned)n_int * kJndCluster, 3);
+  const int copies = jnd_copies(d_lam, 3LL * n_int * kJndCluster);
+  auto kernel = copies == 0   ? jnd_kernel<false, false>
+                : copies == 1 ? jnd_kernel<true, false>
+                              : jnd_kernel<true, true>;
+  kernel<<<grid, kJndThreads, 0, st>>>(d_lam, plane_rows, interval_nodes, head, len, d_dA,
                                            d_ref_of, d_nihc, (double)W[0], (double)W[1],
                                            (double)W[2], Fs, T, d_F_RA, d_F_AI, d_MR, n_int);
   CGB_TRY_CUDA(cudaGetLastError(), "jnd_kernel launch");
@@ -301,11 +415,15 @@ extern "C" int cgb_jnd_batch_dev(const float* d_lam, int64_t plane_rows,
   if (!d_lam || !d_iv || !d_nihc || !W || !d_F_RA || !d_F_AI || n_iv < 0 || n_out <= 0 ||
       plane_rows <= 0)
     return fail(CGB_ERR_ARG, "cgb_jnd_batch_dev: bad arguments");
-  if (n_iv > 2147483647 / 3) return fail(CGB_ERR_RANGE, "cgb_jnd_batch_dev: too many intervals");
+  if (n_iv > 2147483647 / (3 * kJndCluster)) return fail(CGB_ERR_RANGE, "cgb_jnd_batch_dev: too many intervals");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const double T = delta_alpha_len_factor / Fs;
-  dim3 grid((unsigned)(3 * n_iv));
-  jnd_batch_kernel<<<grid, kJndThreads, 0, st>>>(d_lam, plane_rows, d_iv, n_out, d_nihc,
+  dim3 grid((unsigned)(3 * n_iv) * kJndCluster);
+  const int copies = jnd_copies(d_lam, 3LL * n_iv * kJndCluster);
+  auto kernel = copies == 0   ? jnd_batch_kernel<false, false>
+                : copies == 1 ? jnd_batch_kernel<true, false>
+                              : jnd_batch_kernel<true, true>;
+  kernel<<<grid, kJndThreads, 0, st>>>(d_lam, plane_rows, d_iv, n_out, d_nihc,
                                                  (double)W[0], (double)W[1], (double)W[2], Fs, T,
                                                  d_F_RA, d_F_AI, d_MR);
   CGB_TRY_CUDA(cudaGetLastError(), "jnd_batch_kernel launch");
