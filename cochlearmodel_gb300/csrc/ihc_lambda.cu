@@ -921,10 +921,18 @@ extern "C" int cgb_ihc_lambda_noalloc_dev(const float* d_v, int64_t v_rows,
 // with ob the FIR look-back bound.  The reference keeps Y in float (lambdaFloat)
 // and adds each double-tap term in double before rounding back to float; the
 // kernel performs those FP64 operations in the same order (products and sums
-// rounded separately).  The recursion is sequential in time, so one CTA walks
-// one segment of a frame -- rows between two points where the look-back rule
-// gives zero taps, which start the recursion afresh -- with one thread per
-// section.
+// rounded separately).  The recursion is sequential in time, so a CTA walks one
+// segment of a frame -- rows between two points where the look-back rule gives
+// zero taps, which start the recursion afresh -- for 32 sections.  A row's b
+// terms come first and need no earlier output: three warps form them for the
+// next rows while the fourth runs the a terms, its last outputs in registers.
+//
+// What bounds it: the chain of a row's a terms, each a widening, an FP64 addition
+// and a rounding that wait for one another (192 cycles).  With a CTA of 256
+// threads per segment it was the SM's FP64 unit under eight warps (413 cycles a
+// term), and the outputs were read back from memory.  Measured (GB300), the whole
+// stage from and to host arrays: four segments of 2,500 rows, order 2, 6.4 -> 2.7
+// ms; order 4, 10.5 -> 2.3; one of 5,000, order 2, 9.5 -> 2.1.
 // ---------------------------------------------------------------------------
 namespace cgb {
 namespace {
@@ -936,24 +944,85 @@ struct IIRSeg {
   int32_t pad;
 };
 
-__global__ void __launch_bounds__(256)
+constexpr int kIirWarps = 4;   // three for the b terms, one for the a terms
+constexpr int kIirChunk = 24;  // rows of b terms formed ahead
+
+// N: the filter's length where its N - 1 last outputs fit in registers, else 0
+// (they are read back).
+template <int N>
+__global__ void __launch_bounds__(kIirWarps * 32)
     iir_ac_kernel(const float* __restrict__ v, float* __restrict__ ac,
                   const IIRSeg* __restrict__ segs, const cgb_ihc_frame* __restrict__ frames,
                   const double* __restrict__ b, const double* __restrict__ a, int n) {
+  __shared__ float input[2][kIirChunk][32];
   const IIRSeg sg = segs[blockIdx.x];
   const cgb_ihc_frame f = frames[sg.frame];
-  const int s = threadIdx.x;
-  const float* x = v + sg.v_row0 * 256 + s;
-  float* y = ac + sg.v_row0 * 256 + s;
-  for (int k = sg.k0; k < sg.k1; ++k) {
-    const int ob = taps_used(k, f, n);
-    float yk = 0.0f;
-    for (int i = 0; i < ob; ++i)
-      yk = __double2float_rn(__dadd_rn((double)yk, __dmul_rn(b[i], (double)x[(int64_t)(k - i) * 256])));
-    for (int j = 1; j < ob; ++j)
-      yk = __double2float_rn(__dsub_rn((double)yk, __dmul_rn(a[j], (double)y[(int64_t)(k - j) * 256])));
-    y[(int64_t)k * 256] = yk;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t at = sg.v_row0 * 256 + 32 * blockIdx.y + lane;
+  const float* x = v + at;
+  float* y = ac + at;
+  auto b_terms = [&](int chunk) {
+    const int k_first = sg.k0 + chunk * kIirChunk;
+    for (int q = warp - 1; q < kIirChunk && k_first + q < sg.k1; q += kIirWarps - 1) {
+      const int k = k_first + q, ob = taps_used(k, f, n);
+      float yk = 0.0f;
+      for (int i = 0; i < ob; ++i)
+        yk = __double2float_rn(
+            __dadd_rn((double)yk, __dmul_rn(b[i], (double)x[(int64_t)(k - i) * 256])));
+      input[chunk & 1][q][lane] = yk;
+    }
+  };
+  double ra[N > 1 ? N : 1], past[N > 1 ? N : 1];  // past[j]: output k - j
+#pragma unroll
+  for (int j = 1; j < N; ++j) {
+    ra[j] = a[j];
+    past[j] = 0.0;
   }
+  // the look-back rule stepped from row to row: lim = (k + 1) mod rule(k)
+  int rule = sg.k0 < f.frdp - 1 ? f.seg : f.total;
+  int lim = (sg.k0 + 1) % rule;
+  const int chunks = (sg.k1 - sg.k0 + kIirChunk - 1) / kIirChunk;
+  if (warp > 0) b_terms(0);
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    __syncthreads();
+    if (warp > 0) {
+      if (chunk + 1 < chunks) b_terms(chunk + 1);
+      continue;
+    }
+    const int k_first = sg.k0 + chunk * kIirChunk;
+    const int rows = min(kIirChunk, sg.k1 - k_first);
+    for (int q = 0; q < rows; ++q) {
+      const int k = k_first + q, ob = lim < n ? lim : n;
+      float yk = input[chunk & 1][q][lane];
+      if (N > 0) {
+#pragma unroll
+        for (int j = 1; j < N; ++j)
+          if (j < ob) yk = __double2float_rn(__dsub_rn((double)yk, __dmul_rn(ra[j], past[j])));
+#pragma unroll
+        for (int j = N - 1; j > 1; --j) past[j] = past[j - 1];
+        if (N > 1) past[1] = (double)yk;
+      } else {
+        for (int j = 1; j < ob; ++j)
+          yk = __double2float_rn(
+              __dsub_rn((double)yk, __dmul_rn(a[j], (double)y[(int64_t)(k - j) * 256])));
+      }
+      y[(int64_t)k * 256] = yk;
+      if (k + 1 == f.frdp - 1) {
+        rule = f.total;
+        lim = (k + 2) % rule;
+      } else if (++lim == rule) {
+        lim = 0;
+      }
+    }
+  }
+}
+
+template <int N>
+void iir_launch(const float* v, float* ac, const IIRSeg* segs, int n_segs,
+                const cgb_ihc_frame* frames, const double* b, const double* a, int n,
+                cudaStream_t st) {
+  iir_ac_kernel<N><<<dim3((unsigned)n_segs, 8), kIirWarps * 32, 0, st>>>(v, ac, segs, frames, b,
+                                                                         a, n);
 }
 
 constexpr int kMaxIIR = 64;
@@ -1048,11 +1117,16 @@ int ihc_lambda_iir_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* f
     CGB_TRY_CUDA(cudaMemcpyAsync(sc + seg_bytes, taps.data(), taps.size() * 8,
                                  cudaMemcpyHostToDevice, st),
                  "upload IIR taps");
-    iir_ac_kernel<<<(unsigned)segs.size(), 256, 0, st>>>(
-        d_v, d_ac, reinterpret_cast<const IIRSeg*>(sc),
-        reinterpret_cast<const cgb_ihc_frame*>(d_scratch),
-        reinterpret_cast<const double*>(sc + seg_bytes),
-        reinterpret_cast<const double*>(sc + seg_bytes) + n_iir, n_iir);
+    const double* d_b = reinterpret_cast<const double*>(sc + seg_bytes);
+    // orders up to 8 keep their outputs in registers
+    using Launch = decltype(&iir_launch<0>);
+    static const Launch kByLength[] = {iir_launch<0>, iir_launch<1>, iir_launch<2>, iir_launch<3>,
+                                      iir_launch<4>, iir_launch<5>, iir_launch<6>, iir_launch<7>,
+                                      iir_launch<8>, iir_launch<9>};
+    kByLength[n_iir <= 9 ? n_iir : 0](d_v, d_ac, reinterpret_cast<const IIRSeg*>(sc),
+                                     (int)segs.size(),
+                                     reinterpret_cast<const cgb_ihc_frame*>(d_scratch), d_b,
+                                     d_b + n_iir, n_iir, st);
     CGB_TRY_CUDA(cudaGetLastError(), "iir_ac_kernel launch");
     note_launch();
   }
