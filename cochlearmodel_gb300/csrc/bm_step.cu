@@ -37,6 +37,17 @@
 //      --fmad=true, checked on every float input.)
 //   Both keep simulated time in a float accumulator, as the reference does.
 //
+// What bounds it: the issue of dependent FP32 work at two warps per scheduler (a
+// two-wide fma of three distinct register pairs takes 2.8 cycles).  The first
+// iteration of a step, the second and the later ones are compiled apart, without
+// the branches, copies and votes that tell them apart at run time; the halo of a
+// solve's first round and the next input sample are fetched ahead of their use.
+// Measured (GB300, JND sweep, 3,025 units): one loop body for all iterations
+// 140.3 ms, the input sample ahead 138.5, the kinds apart 130.4, the halo ahead
+// 129.8; the default kernel's semantics (3,000 units of 2 ms) 44.2 -> 37.6.
+// Tried and slower: scalar fmas in the two-step update, all (145.4) or the last of
+// a chain (140.9); both sums of the step test in one two-wide butterfly (131.6).
+//
 // Floating-point order is fixed: the file is compiled with --fmad=false and
 // every fused multiply-add is an explicit __fmaf_rn.
 
@@ -45,6 +56,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdio>
+#include <type_traits>
 
 #include "bm_common.cuh"
 #include "cgb_device.cuh"
@@ -296,7 +308,9 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
   // reference's curr_time_f (include/cochlea.cuh:13642,14230)
   float tau_f = 0.0f;
   int n = un.start;
-  float sx0 = inb[n], sx1 = inb[n + 1];
+  // input samples n, n + 1 and, loaded a sample ahead, n + 2 (the last sample
+  // that a unit uses is end + 1)
+  float sx0 = inb[n], sx1 = inb[n + 1], sx2 = inb[min(n + 2, un.end + 1)];
   int fail_flag = 0;
   long long n_sub = 0, n_it = 0, n_sw = 0;
   int n_failed = 0, n_written = 0, status = 0, sub_in_sample = 0;
@@ -308,7 +322,6 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       status = 1;
       break;
     }
-    int out_loop = 0, reset = 1, another = 1;
     if (TOL) {
       // rotate the pressure history: slot (n_sub & 1) receives p at the start
       // of this step, the other slot holds the start of the previous one
@@ -324,11 +337,14 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
     // one fma with the half step
     const float hdt = __fmul_rn(dt, 0.5f);
     const float2 dt2 = f2b(dt), hdt2 = f2b(hdt);
-    do {
-      // Predictor.  The first iteration of a step (or one after a reset) is
-      // Euler, which is the trapezoid rule with the new-derivative slots
-      // holding the previous derivatives: (d0 + d0) * 0.5 == d0 exactly, so
-      // one code path serves both.
+    // One outer iteration; true to go on.  The three kinds an iteration can be
+    // are compiled separately, each as straight-line code around its solve:
+    //   FIRST  the first of a step: the Euler predictor, which is the trapezoid
+    //          rule with the new-derivative slots holding the previous
+    //          derivatives ((d0 + d0) * 0.5 == d0 exactly); no step test
+    //   SLOW   the first two: the TM update and (fixed counts) jslow sweeps
+    auto iterate = [&](auto first_c, auto slow_c) -> bool {
+      constexpr bool FIRST = decltype(first_c)::value, SLOW = decltype(slow_c)::value;
       float2 x0[4], v0[4], a0[4], y0[4], u0[4], ps0[4], dp0[4];
       prev.load(0, qb, x0);
       prev.load(1, qb, v0);
@@ -337,49 +353,45 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       prev.load(4, qb, u0);
       prev.load(5, qb, ps0);
       prev.load(6, qb, dp0);
-      if (__all_sync(kFull, out_loop == 0 || reset)) {
-        out_loop = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          a[k] = a0[k];
-          u[k] = u0[k];
-          dp[k] = dp0[k];
-        }
-        wd = wd0;
-        wdd = wdd0;
+      // the pressure next to the lane, for the solve's first round: known since
+      // the iteration before
+      float2 pH = f2b(0.0f), pH2 = f2b(0.0f);
+      if (!TOL && !ARITH) {
+        pH = f2(__shfl_sync(kFull, p[0].y, src_l), __shfl_down_sync(kFull, p[0].x, 1));
+        pH2 = f2(__shfl_sync(kFull, p[1].y, src_l), __shfl_down_sync(kFull, p[1].x, 1));
       }
       float2 dv[4], fl[4];
       const float2 mtt2 = f2b(mtt);
       bool fault = false;  // CTL 1: some section of this lane fails the speed test
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float2 vn = fma2(add2(a0[k], a[k]), hdt2, v0[k]);
-        dv[k] = abs2(sub2(vn, v[k]));
-        const float2 thr = max2(mtt2, mul2(vn, dt2));
-        if (CTL == 0) fl[k] = sub2(dv[k], thr);
-        else fault = fault || dv[k].x > thr.x || dv[k].y > thr.y;
+        const float2 vn = fma2(add2(a0[k], FIRST ? a0[k] : a[k]), hdt2, v0[k]);
+        if (!FIRST) {
+          dv[k] = abs2(sub2(vn, v[k]));
+          const float2 thr = max2(mtt2, mul2(vn, dt2));
+          if (CTL == 0) fl[k] = sub2(dv[k], thr);
+          else fault = fault || dv[k].x > thr.x || dv[k].y > thr.y;
+        }
         v[k] = vn;
         x[k] = fma2(add2(v0[k], vn), hdt2, x0[k]);
-        y[k] = fma2(add2(u0[k], u[k]), hdt2, y0[k]);
-        ps[k] = fma2(add2(dp0[k], dp[k]), hdt2, ps0[k]);
+        y[k] = fma2(add2(u0[k], FIRST ? u0[k] : u[k]), hdt2, y0[k]);
+        ps[k] = fma2(add2(dp0[k], FIRST ? dp0[k] : dp[k]), hdt2, ps0[k]);
       }
-      w = __fmaf_rn(__fadd_rn(wd0, wd), hdt, w0);
-      wd = __fmaf_rn(__fadd_rn(wdd0, wdd), hdt, wd0);
+      w = __fmaf_rn(__fadd_rn(wd0, FIRST ? wd0 : wd), hdt, w0);
+      wd = __fmaf_rn(__fadd_rn(wdd0, FIRST ? wdd0 : wdd), hdt, wd0);
       // The velocity-error sum (ARITH 1: in the reference's tree order) and,
       // for CTL 0, the summed margin.  The whole-warp reductions are issued
       // here, where nothing waits on them, so their shuffle latency overlaps
-      // the TM update and the sweeps (the tester runs only when reset == 0,
-      // a warp-uniform condition).
+      // the TM update and the sweeps.
       float ev = 0.0f, Fsum = 0.0f;
       bool faulty = false;
-      if (__all_sync(kFull, reset == 0)) {
+      if (!FIRST) {
         ev = ARITH ? ref_tree_sum(dv) : warp_sum_xor(pair_sum8p(dv));
         if (CTL == 0) Fsum = warp_sum_xor(pair_sum8p(fl));
         else faulty = __any_sync(kFull, fault);
       }
 
       // OHC / TM coupling, G and the right-hand side Y (scaled by 1/m).
-      const bool tm_update = out_loop < 2;
       // the G/Y section tables are loaded here, so that their shared-memory
       // latency passes under the TM update (2% of the step against loading
       // them next to their use)
@@ -389,7 +401,7 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       load8q(sp + 4 * 256 + qb, Qs);
       {
         // the TM tables are loaded next to their use (short live ranges)
-        if (tm_update) {
+        if (SLOW) {
           float2 Stm[4], Rtm[4], gs[4], gm[4], Ptm[4];
           load8q(sp + 6 * 256 + qb, Stm);
           load8q(sp + 7 * 256 + qb, Rtm);
@@ -451,11 +463,11 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       // sections duplicate exactly what the neighbours compute) and the
       // second on its own sections, so one shuffle round serves two sweeps.
       // Sections 254 and 255 carry no lower coefficient; p_{-1} = p_256 = 0.
-      const int J = TOL ? A.jcap : (tm_update ? A.jslow : A.jfast);
+      const int J = TOL ? A.jcap : (SLOW ? A.jslow : A.jfast);
       const float2 Yrmh = f2(kWrap ? __shfl_sync(kFull, Yrm[0].y, src_l)
                                    : __shfl_up_sync(kFull, Yrm[0].y, 1),
                              __shfl_down_sync(kFull, Yrm[0].x, 1));
-      if (TOL && out_loop == 0 && n_sub >= 2) {
+      if (TOL && FIRST && n_sub >= 2) {
         float2 p2[4];
         load8q(hist + ((n_sub + 1) & 1) * 256 + qb, p2);
         if (A.log && n_sub % A.log_every == 0) {
@@ -501,11 +513,14 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       }
       // two sweeps with one shuffle round; q holds the first sweep's result
       float2 q[4];
-      auto sweep_pair = [&]() {
+      auto sweep_pair = [&](bool first_round) {
         float2 T[4];
         // halo pairs: (8l-1, 8l+8) and (8l-2, 8l+9)
         float2 H, H2;
-        if (kWrap) {
+        if (first_round) {
+          H = pH;
+          H2 = pH2;
+        } else if (kWrap) {
           H = f2(__shfl_sync(kFull, p[0].y, src_l), __shfl_down_sync(kFull, p[0].x, 1));
           H2 = f2(__shfl_sync(kFull, p[1].y, src_l), __shfl_down_sync(kFull, p[1].x, 1));
         } else {
@@ -568,11 +583,7 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
 #pragma unroll
         for (int k = 0; k < 4; ++k) C2[k] = fma2(neg2(T[k]), rm[k], Yrm[k]);
       };
-      auto two_step = [&]() {
-        const float2 H =
-            f2(__shfl_sync(kFull, p[0].y, src_l), __shfl_down_sync(kFull, p[0].x, 1));
-        const float2 H2 =
-            f2(__shfl_sync(kFull, p[1].y, src_l), __shfl_down_sync(kFull, p[1].x, 1));
+      auto two_step_with = [&](float2 H, float2 H2) {
         float2 r[4];
         r[0] = fma2(KL[0], H2, fma2(KH[0], p[2], fma2(KB[0], p[0], C2[0])));
         r[1] = fma2(KL[1], H, fma2(KH[1], p[3], fma2(KB[1], p[1], C2[1])));
@@ -580,6 +591,13 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
         r[3] = fma2(KL[3], p[1], fma2(KH[3], f2(p[2].y, p[2].x), fma2(KB[3], p[3], C2[3])));
 #pragma unroll
         for (int k = 0; k < 4; ++k) p[k] = r[k];
+      };
+      auto two_step = [&]() {
+        const float2 H =
+            f2(__shfl_sync(kFull, p[0].y, src_l), __shfl_down_sync(kFull, p[0].x, 1));
+        const float2 H2 =
+            f2(__shfl_sync(kFull, p[1].y, src_l), __shfl_down_sync(kFull, p[1].x, 1));
+        two_step_with(H, H2);
       };
       int it = 0;
       if (ARITH) {
@@ -602,15 +620,16 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
 #pragma unroll
           for (int k = 0; k < 4; ++k) p[k] = mul2(sub2(Yrm[k], T[k]), rm[k]);
         }
-      } else if (!TOL && J == 20) {
+      } else if (!TOL && SLOW && J == 20) {
         // the reference schedule's slow count, fully unrolled
         two_step_setup();
+        two_step_with(pH, pH2);
 #pragma unroll
-        for (int r = 0; r < 10; ++r) two_step();
+        for (int r = 1; r < 10; ++r) two_step();
         it = 20;
-      } else if (!TOL && J == 2) {
+      } else if (!TOL && !SLOW && J == 2) {
         // and its fast count, one pair without the loop
-        sweep_pair();
+        sweep_pair(true);
         it = 2;
       } else if (!TOL && J >= 4) {
         two_step_setup();
@@ -618,7 +637,7 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
       } else {
 #pragma unroll 2
         for (; it + 1 < J; it += 2) {
-          sweep_pair();
+          sweep_pair(false);
           if (TOL) {
             float dm = 0.0f, pm = 0.0f;
 #pragma unroll
@@ -684,53 +703,47 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
         wdd = A.ow_pow2 ? __fmul_rn(ws, A.rsow) : __fdiv_rn(ws, A.sow);
       }
 
-      if (reset == 0) {
-        const float2 m = max2(max2(da[0], da[1]), max2(da[2], da[3]));
-        const float eap = fmaxf(0.0f, fmaxf(m.x, m.y));
-        const float ea = warp_max_xor(eap);
-        // CTL 0: the summed margin; CTL 1: any failing section
-        if (CTL == 0) faulty = Fsum > 0.0f;
-        const float num = __fmul_rn(ea, dt);
-        // L = ea dt / ev (0 unless ev > mmspt).  ARITH 1 divides as the
-        // reference does; ARITH 0 tests L > 6 as num > 6 ev and L < 0.5 as
-        // num < 0.5 ev, with 6 ev rounded once (no division on the step's
-        // critical path).
-        const bool lcheck = ev > mmspt;
-        const float L = lcheck && ARITH ? __fdividef(num, ev) : 0.0f;
-        const bool l_big = ARITH ? L > 6.0f : lcheck && num > __fmul_rn(6.0f, ev);
-        const bool l_small = ARITH ? L < 0.5f : !lcheck || num < __fmul_rn(0.5f, ev);
-        // Step decisions are the same in every lane (they come from warp
-        // reductions and uniform counters); taking them through a vote makes
-        // that visible to the compiler, which then branches without
-        // reconvergence barriers.
-        if (__all_sync(kFull, l_big)) {
-          dt = __fmul_rn(dt, 0.5f);
-          if (dt < A.dtmin) dt = A.dtmin;
-          another = 0;
-          reset = 1;
-        } else if (__all_sync(kFull, faulty)) {
-          another = 1;
-          reset = 0;
-        } else if (__all_sync(kFull, l_small)) {
-          dt = __fmul_rn(dt, 2.0f);
-          if (dt > A.dtmax) dt = A.dtmax;
-          another = 0;
-          reset = 1;
-        } else {
-          another = 1;
-          reset = 0;
-        }
-      } else {
-        another = 1;
-        reset = 0;
-      }
+      if (FIRST) return true;
+      const float2 m = max2(max2(da[0], da[1]), max2(da[2], da[3]));
+      const float eap = fmaxf(0.0f, fmaxf(m.x, m.y));
+      const float ea = warp_max_xor(eap);
+      // CTL 0: the summed margin; CTL 1: any failing section
+      if (CTL == 0) faulty = Fsum > 0.0f;
+      const float num = __fmul_rn(ea, dt);
+      // L = ea dt / ev (0 unless ev > mmspt).  ARITH 1 divides as the
+      // reference does; ARITH 0 tests L > 6 as num > 6 ev and L < 0.5 as
+      // num < 0.5 ev, with 6 ev rounded once (no division on the step's
+      // critical path).
+      const bool lcheck = ev > mmspt;
+      const float L = lcheck && ARITH ? __fdividef(num, ev) : 0.0f;
+      const bool l_big = ARITH ? L > 6.0f : lcheck && num > __fmul_rn(6.0f, ev);
+      const bool l_small = ARITH ? L < 0.5f : !lcheck || num < __fmul_rn(0.5f, ev);
+      // The decision is the same in every lane (it comes from warp reductions);
+      // taking it through a vote makes that visible to the compiler, which then
+      // branches without reconvergence barriers.
+      const bool grow = !l_big && !faulty && l_small;
+      const float up = __fmul_rn(dt, 2.0f), down = __fmul_rn(dt, 0.5f);
+      dt = l_big ? (down < A.dtmin ? A.dtmin : down)
+                 : (grow ? (up > A.dtmax ? A.dtmax : up) : dt);
+      return __all_sync(kFull, !l_big && !grow);
+    };
+
+    using Yes = std::true_type;
+    using No = std::false_type;
+    int out_loop = 1;
+    iterate(Yes(), Yes());
+    bool another = true;
+    if (A.max_outer > 1) {
+      another = iterate(No(), Yes());
       ++out_loop;
-      if (out_loop >= A.max_outer) {
-        another = 0;
-        reset = 1;
-        fail_flag = 1;
+      while (another && out_loop < A.max_outer) {
+        another = iterate(No(), No());
+        ++out_loop;
       }
-    } while (__all_sync(kFull, another));
+    }
+    // a step that reaches max_outer iterations counts as failed, also where
+    // the last of them passes the test
+    if (out_loop >= A.max_outer) fail_flag = 1;
     ++n_sub;
     n_it += out_loop;
     smp_sub = __fadd_rn(smp_sub, 1.0f);
@@ -740,7 +753,8 @@ __device__ __forceinline__ void run_unit(const BMArgs& A, const cgb_unit& un,
     if (__all_sync(kFull, tau_f > A.tout_f)) {
       tau_f = __fsub_rn(tau_f, A.tout_f);
       sx0 = sx1;
-      sx1 = inb[n + 2];
+      sx1 = sx2;
+      sx2 = inb[min(n + 3, un.end + 1)];
       if (__all_sync(kFull, n >= un.out_first)) {
         store8p(outb + (int64_t)n * 256 + base, v);
         if (A.host_delta)
