@@ -25,11 +25,14 @@
 // products as soon as a half is there.  Between the digits the same warps finish
 // the tile before: its Dot2 points, the DC sums, IHC and lambda.
 //
-// What bounds it now: the workers' chain, ~57k cycles a tile (Dot2 points 12k, DC
+// What bounds it now: the workers' chain, ~56k cycles a tile (Dot2 points 11k, DC
 // sums 11k, IHC / lambda 7k, loads 7k, digits 10k, epilogue 4k) at 41% of the
 // issue slots, not the tensor pipe.  Finishing a tile at once instead of between
 // the next one's digits takes 22.0 ms against 18.9 (JND sweep); without the products
-// (accumulators left as they are) the chain takes the same time.
+// (accumulators left as they are) the chain takes the same time.  The taps left over
+// by a point's batches of eight in batches of four and one, not one by one with a
+// choice of register each: 18.9 -> 18.65 ms.  DC sums whose errors run a batch
+// behind, or on two blocks at once: 19.5 and 19.6.
 //
 // Measured (GB300), against the FP32 pipe: JND sweep (2.9 million rows) 53.7 ->
 // 18.3 ms, 176,000 rows in 33 intervals 4.46 -> 1.52 ms, one signal of 5,330 rows
@@ -171,6 +174,32 @@ __device__ __forceinline__ void dot2_pairs(Dot2& acc, const float (&b)[N], const
     acc.c = __fmaf_rn(b[i], ep, acc.c);
   }
   acc.s = t[N - 1];
+}
+
+// The next N taps (tap pairs) of a point whose rows and taps lie one to a lane,
+// from lane q on; N.
+template <int N>
+__device__ __forceinline__ int lane_taps(Dot2& acc, float b, float u, int q) {
+  float gb[N], gu[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    gb[e] = __shfl_sync(kFull, b, q + e);
+    gu[e] = __shfl_sync(kFull, u, q + e);
+  }
+  dot2_taps(acc, gb, gu);
+  return N;
+}
+template <int N>
+__device__ __forceinline__ int lane_pairs(Dot2& acc, float b, float u, float w, int q) {
+  float gb[N], gu[N], gw[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    gb[e] = __shfl_sync(kFull, b, q + e);
+    gu[e] = __shfl_sync(kFull, u, q + e);
+    gw[e] = __shfl_sync(kFull, w, q + e);
+  }
+  dot2_pairs(acc, gb, gu, gw);
+  return N;
 }
 
 // Dot2 of one output in the orders of ihc_lambda.cu (fir_row, fir_row_sym),
@@ -534,32 +563,29 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll 1
-              for (int q = 0; q < 32 && 32 * i + q + 8 <= half; q += 8) {
-                float gb[8], gu[8], gw8[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  gb[e] = __shfl_sync(kFull, b[i], q + e);
-                  gu[e] = __shfl_sync(kFull, u[i], q + e);
-                  gw8[e] = __shfl_sync(kFull, w[i], q + e);
-                }
-                dot2_pairs(acc, gb, gu, gw8);
+              for (int q = 0; q < 32 && 32 * i + q < half;) {
+                const int left = half - 32 * i - q;
+                if (left >= 8)
+                  q += lane_pairs<8>(acc, b[i], u[i], w[i], q);
+                else if (left >= 4)
+                  q += lane_pairs<4>(acc, b[i], u[i], w[i], q);
+                else
+                  q += lane_pairs<1>(acc, b[i], u[i], w[i], q);
               }
-            for (int k = half & ~7; k < half; ++k) acc.add_pair(from(b, k), from(u, k), from(u, n_ac - 1 - k));
             if (n_ac & 1) acc.add(from(b, half), from(u, half));
           } else {
 #pragma unroll
             for (int i = 0; i < 9; ++i)
 #pragma unroll 1
-              for (int q = 0; q < 32 && 32 * i + q + 8 <= taps; q += 8) {
-                float gb[8], gu[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  gb[e] = __shfl_sync(kFull, b[i], q + e);
-                  gu[e] = __shfl_sync(kFull, u[i], q + e);
-                }
-                dot2_taps(acc, gb, gu);
+              for (int q = 0; q < 32 && 32 * i + q < taps;) {
+                const int left = taps - 32 * i - q;
+                if (left >= 8)
+                  q += lane_taps<8>(acc, b[i], u[i], q);
+                else if (left >= 4)
+                  q += lane_taps<4>(acc, b[i], u[i], q);
+                else
+                  q += lane_taps<1>(acc, b[i], u[i], q);
               }
-            for (int k = taps & ~7; k < taps; ++k) acc.add(from(b, k), from(u, k));
           }
           const float ac = acc.result();
           const float ms = __fmaf_rn(u[0], A.scale, -ac);  // (lane 0's is the point's own)
