@@ -90,11 +90,11 @@ __device__ __forceinline__ uint32_t elected() {
 }
 
 __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate,
-                                    uint32_t issue) {
+                                    uint32_t issue, uint32_t instr = kInstr) {
   asm volatile(
       "{ .reg .pred p, q; setp.ne.b32 p, %4, 0; setp.ne.b32 q, %5, 0;\n"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(d),
-      "l"(a), "l"(b), "r"(kInstr), "r"(accumulate), "r"(issue)
+      "l"(a), "l"(b), "r"(instr), "r"(accumulate), "r"(issue)
       : "memory");
 }
 

@@ -9,9 +9,7 @@
 //   loss          : pred = s_out * o, MSE against the raw target; dL/do (BF16)
 //   backward      : one CTA per record, the transposed convolutions with the
 //                   ReLU masks -> pre-activation gradients (BF16)
-//   weight grad   : per CTA, its records' dW = sum_pos dPre (x) input,
-//                   accumulated in FP32 into the CTA's partial slot, then a
-//                   fixed-order FP64 sum over the slots (deterministic)
+//   weight grad   : warmstart_grad.cu
 //   adam          : FP32 master parameters, then re-packed to BF16.
 // All products run on the tensor cores (mma.sync m16n8k16 BF16, FP32
 // accumulate); ldmatrix (.trans for the weight gradients) feeds them.
@@ -25,12 +23,6 @@
 
 namespace cgb {
 namespace ws {
-
-// Canonical FP32 parameter offsets: W1[5][64][8], b1, W2[5][64][64], b2,
-// W3[5][64][64], b3, W4[5][64], b4[1].
-constexpr int oW1 = 0, ob1 = oW1 + 5 * 64 * 8, oW2 = ob1 + 64, ob2 = oW2 + 5 * 64 * 64,
-              oW3 = ob2 + 64, ob3 = oW3 + 5 * 64 * 64, oW4 = ob3 + 64, ob4 = oW4 + 5 * 64;
-static_assert(ob4 + 1 == kParams, "parameter layout");
 
 constexpr int kRows = 272;            // 64-channel rows per record: position + 8
 constexpr int kHBytes = kNS * 128;    // one stored hidden layer of one record
@@ -320,142 +312,6 @@ __global__ void __launch_bounds__(256) backward_kernel(const unsigned char* __re
   }
 }
 
-// ---------------------------------------------------------------------------
-// Weight gradients.  CTA c handles records c, c + grid, ...; per record the
-// inputs (features, H1..H3 at row position + 8) and the pre-activation
-// gradients (dH1..dH3, dO at row position) are staged in shared memory and
-// every (layer, tap, 16-output tile) task is one warp's 16 x Cin product over
-// the 256 positions, added into the CTA's FP32 partial slot.
-// ---------------------------------------------------------------------------
-constexpr int kWgSmem = kFeatBytes + 3 * kRows * 128 + 3 * kNS * 128 + kNS * 16 + 128;
-
-__device__ __forceinline__ void add_tile(float* __restrict__ part, int row_stride, int co0,
-                                         int n_co, const float (&acc)[8][4], int nt_count,
-                                         int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  for (int nt = 0; nt < nt_count; ++nt) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int co = co0 + g + 8 * h;
-      if (co >= n_co) continue;
-      float* pr = part + co * row_stride + nt * 8 + 2 * t;
-      pr[0] += acc[nt][2 * h];
-      pr[1] += acc[nt][2 * h + 1];
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) wgrad_kernel(const unsigned char* __restrict__ feat,
-                                                    const unsigned char* __restrict__ hid,
-                                                    const unsigned char* __restrict__ dpre,
-                                                    const unsigned char* __restrict__ dout, int n,
-                                                    float* __restrict__ partial) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  unsigned char* sF = sm;
-  unsigned char* sH = sF + kFeatBytes;              // 3 x kRows rows (position + 8)
-  unsigned char* sD = sH + 3 * kRows * 128;         // 3 x 256 rows (position)
-  unsigned char* sO = sD + 3 * kNS * 128;           // 256 rows of 16 bytes
-  unsigned char* sZ = sO + kNS * 16;                // 128 zero bytes
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = lane >> 3, r = lane & 7;
-  zero16(sH, 3 * kRows * 128, tid, 256);
-  zero16(sZ, 128, tid, 256);
-  float* part = partial + (int64_t)blockIdx.x * kParams;
-  for (int i = tid; i < kParams; i += 256) part[i] = 0.0f;
-  const int64_t lo = (int64_t)n * kHBytes;
-  for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-    __syncthreads();
-    copy16(sF, feat + (int64_t)rec * kFeatBytes, kFeatBytes, tid, 256);
-    for (int l = 0; l < 3; ++l) {
-      copy16(sH + l * kRows * 128 + 8 * 128, hid + l * lo + (int64_t)rec * kHBytes, kHBytes, tid,
-             256);
-      copy16(sD + l * kNS * 128, dpre + l * lo + (int64_t)rec * kHBytes, kHBytes, tid, 256);
-    }
-    copy16(sO, dout + (int64_t)rec * kNS * 16, kNS * 16, tid, 256);
-    __syncthreads();
-    // tasks: layer 1: 20 (tap x 4 co tiles), layers 2, 3: 20 each, layer 4: 5
-    for (int task = warp; task < 65; task += 8) {
-      float acc[8][4];
-      zero_acc(acc);
-      if (task < 20) {  // layer 1: A = dH1^T (co), B = features (8 ci)
-        const int tap = task >> 2, mt = task & 3;
-        const uint32_t uD = smem_u32(sD), uF = smem_u32(sF);
-        for (int kb = 0; kb < kNS; kb += 16) {
-          uint32_t a[4], b[2];
-          ldsm_x4_t(a, uD + swz64(kb + r + 8 * (q >> 1), 2 * mt + (q & 1)));
-          ldsm_x2_t(b, uF + (kb + r + 8 * (q & 1) + tap + 6) * 16);
-          mma_bf16(acc[0], a, b[0], b[1]);
-        }
-        __syncwarp();
-        add_tile(part + oW1 + tap * 64 * 8, 8, 16 * mt, 64, acc, 1, lane);
-      } else if (task < 60) {  // layers 2, 3: A = dH^T, B = previous hidden layer
-        const int l = (task - 20) / 20, j = (task - 20) % 20, tap = j >> 2, mt = j & 3;
-        const uint32_t uD = smem_u32(sD + (l + 1) * kNS * 128);
-        const uint32_t uH = smem_u32(sH + l * kRows * 128);
-        for (int kb = 0; kb < kNS; kb += 16) {
-          uint32_t a[4];
-          ldsm_x4_t(a, uD + swz64(kb + r + 8 * (q >> 1), 2 * mt + (q & 1)));
-          const int brow = kb + r + 8 * (q & 1) + tap + 6;
-#pragma unroll
-          for (int np = 0; np < 4; ++np) {
-            uint32_t b[4];
-            ldsm_x4_t(b, uH + swz64(brow, 2 * np + (q >> 1)));
-            mma_bf16(acc[2 * np], a, b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
-          }
-        }
-        __syncwarp();
-        add_tile(part + (l ? oW3 : oW2) + tap * 64 * 64, 64, 16 * mt, 64, acc, 8, lane);
-      } else {  // layer 4: A = dO^T (output 0; rows 8..15 of the tile read zeros)
-        const int tap = task - 60;
-        const uint32_t uO = smem_u32(sO), uZ = smem_u32(sZ);
-        const uint32_t uH = smem_u32(sH + 2 * kRows * 128);
-        for (int kb = 0; kb < kNS; kb += 16) {
-          uint32_t a[4];
-          ldsm_x4_t(a, (q & 1) ? uZ + r * 16 : uO + (kb + r + 8 * (q >> 1)) * 16);
-          const int brow = kb + r + 8 * (q & 1) + tap + 6;
-#pragma unroll
-          for (int np = 0; np < 4; ++np) {
-            uint32_t b[4];
-            ldsm_x4_t(b, uH + swz64(brow, 2 * np + (q >> 1)));
-            mma_bf16(acc[2 * np], a, b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
-          }
-        }
-        __syncwarp();
-        add_tile(part + oW4 + tap * 64, 64, 0, 1, acc, 8, lane);
-      }
-    }
-    // bias gradients: sums of the pre-activation gradients over positions
-    if (tid < 193) {
-      float sum = 0.0f;
-      if (tid < 192) {
-        const int l = tid >> 6, co = tid & 63;
-        const unsigned char* d = sD + l * kNS * 128;
-        for (int pos = 0; pos < kNS; ++pos) {
-          const uint16_t hbits =
-              *reinterpret_cast<const uint16_t*>(d + swz64(pos, co >> 3) + (co & 7) * 2);
-          sum += __uint_as_float((uint32_t)hbits << 16);
-        }
-        part[(l == 0 ? ob1 : l == 1 ? ob2 : ob3) + co] += sum;
-      } else {
-        for (int pos = 0; pos < kNS; ++pos)
-          sum += __uint_as_float((uint32_t)(*reinterpret_cast<const uint16_t*>(sO + pos * 16)) << 16);
-        part[ob4] += sum;
-      }
-    }
-  }
-}
-
-__global__ void reduce_kernel(const float* __restrict__ partial, int n_parts,
-                              float* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
-  double s = 0.0;
-  for (int c = 0; c < n_parts; ++c) s += (double)partial[(int64_t)c * kParams + i];
-  grad[i] = (float)s;
-}
-
 __global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ grad,
                             float* __restrict__ m, float* __restrict__ v, float lr, float b1,
                             float b2, float eps, float c1, float c2) {
@@ -584,25 +440,6 @@ extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, cons
       static_cast<const unsigned char*>(d_blobT), static_cast<const unsigned char*>(d_dout),
       static_cast<const unsigned char*>(d_hid), n, static_cast<unsigned char*>(d_dpre));
   CGB_TRY_CUDA(cudaGetLastError(), "backward_kernel launch");
-  note_launch();
-  return CGB_OK;
-}
-
-extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const void* d_dpre,
-                                const void* d_dout, int n, float* d_partial, int n_parts,
-                                float* d_grad, void* stream) {
-  if (n < 0 || n_parts < 1 || !d_feat || !d_hid || !d_dpre || !d_dout || !d_partial || !d_grad)
-    return fail(CGB_ERR_ARG, "cgb_ws_wgrad_dev: bad arguments");
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (set_smem(wgrad_kernel, kWgSmem, "cudaFuncSetAttribute(wgrad)")) return CGB_ERR_CUDA;
-  wgrad_kernel<<<n_parts, 256, kWgSmem, st>>>(
-      static_cast<const unsigned char*>(d_feat), static_cast<const unsigned char*>(d_hid),
-      static_cast<const unsigned char*>(d_dpre), static_cast<const unsigned char*>(d_dout), n,
-      d_partial);
-  CGB_TRY_CUDA(cudaGetLastError(), "wgrad_kernel launch");
-  note_launch();
-  reduce_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(d_partial, n_parts, d_grad);
-  CGB_TRY_CUDA(cudaGetLastError(), "reduce_kernel launch");
   note_launch();
   return CGB_OK;
 }

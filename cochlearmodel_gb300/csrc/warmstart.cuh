@@ -58,6 +58,12 @@ constexpr int kOffT2 = kOffT3 + kW64Bytes;
 constexpr int kBlobTBytes = kOffT2 + kW64Bytes;  // 88064
 constexpr int kParams = 5 * 64 * 8 + 64 + 5 * 64 * 64 + 64 + 5 * 64 * 64 + 64 + 5 * 64 + 1;
 
+// Canonical FP32 parameter offsets: W1[5][64][8], b1, W2[5][64][64], b2,
+// W3[5][64][64], b3, W4[5][64], b4[1].
+constexpr int oW1 = 0, ob1 = oW1 + 5 * 64 * 8, oW2 = ob1 + 64, ob2 = oW2 + 5 * 64 * 64,
+              oW3 = ob2 + 64, ob3 = oW3 + 5 * 64 * 64, oW4 = ob3 + 64, ob4 = oW4 + 5 * 64;
+static_assert(ob4 + 1 == kParams, "parameter layout");
+
 static_assert(kBlobBytes % 16 == 0, "blob must be a whole number of 16-byte chunks");
 
 __host__ __device__ __forceinline__ int swz64(int row, int chunk) {

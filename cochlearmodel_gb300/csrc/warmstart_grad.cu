@@ -1,0 +1,361 @@
+// Weight gradients of the warm-start network (warmstart.cuh) on the
+// 5th-generation tensor cores.
+//
+//   dW_l[tap][co][ci] = sum over records and positions of
+//                       dPre_l[pos][co] * In_l[pos + tap - 2][ci]
+// is a product whose K dimension is the position.  Both factors lie in shared
+// memory as they are in global memory, eight channels of a position in 16 bytes,
+// the rows of one chunk of eight channels following each other: eight positions
+// of a chunk are one 8 x 8 core matrix of an MN-major operand, and a shift by one
+// position (a tap) is a start address 16 bytes further on.
+//   layers 2, 3: M = 128 is dPre's 64 channels twice, the second time one position
+//                on, N = 64 input channels: one instruction gives two taps, three
+//                (at shifts -1, 1, 2 of the input) all five.
+//   layers 1, 4: the operand with 8 channels is A, and its 16 chunks of eight rows
+//                of M are the same rows from 16 positions on (a stride of 16 bytes),
+//                of which five are the taps.
+// Rows of ones beside an operand give the bias gradients in the same way.
+//
+// A third of the CTAs takes layer 2, layer 3, and layers 1 and 4 each, about equal
+// shares of the tensor pipe (2,500 cycles a record: the instructions read their
+// operands from shared memory, 49 cycles for 128 x 64 x 16).  A CTA keeps the sums of
+// its records in tensor memory, stages a record while the one before is multiplied,
+// and writes its partial slot once; the slots are added in a fixed order
+// (deterministic).
+//
+// What bounded it: with mma.sync a CTA per record staged the factors of all layers
+// (209 KB), had 65 small tasks for eight warps, and added each to its slot in global
+// memory.  256 records 160 -> 23 us, 1,024 records 390 -> 56, 32 records 52 -> 14.5
+// (both kernels; the reduction 6 us).  Setting up all of shared memory and writing
+// the slots from the accumulators' lanes (256 bytes apart) cost 12 us of 35.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "cgb_device.cuh"
+#include "cgb_internal.h"
+#include "ihc_common.cuh"
+#include "tensor_fir.cuh"
+#include "warmstart.cuh"
+
+namespace cgb {
+namespace ws {
+namespace {
+
+constexpr int kLoaders = 512;                 // threads that stage the factors
+constexpr int kGradThreads = kLoaders + 32;   // and the issuing warp
+constexpr int kGroups = 3;                    // layer 2 | layer 3 | layers 1 and 4
+
+// Layers 2, 3.  K runs over positions -1 .. 270 (17 steps); row r of A's first
+// half is position r - 1, of its second half r, of B r - 2.  The distances between
+// chunks are odd multiples of 16 bytes: the eight chunks of a position, stored by
+// eight lanes, fall into distinct banks.
+constexpr int kSteps = 17;
+constexpr int kARows = 273, kBRows = 275;
+constexpr int kAChunk = kARows * 16, kBChunk = kBRows * 16;
+constexpr int kOffB = 16 * kAChunk;           // A: 16 chunks
+constexpr int kStage23 = kOffB + 10 * kBChunk;  // B: 8 chunks and two of ones
+// Layers 1, 4.  K runs over positions 0 .. 255; row r of the features is position
+// r - 8, of dO r - 2, of dPre and H3 r.
+constexpr int kORows = 272, kHRows = 257;
+constexpr int kHChunk = kHRows * 16;
+constexpr int kFeat = kFeatRows * 16;
+constexpr int kOffO = kFeat, kOffD = kOffO + kORows * 16, kOffH = kOffD + 8 * kHChunk;
+constexpr int kStage14 = kOffH + 10 * kHChunk;  // H3: 8 chunks and two of ones
+constexpr int kStage = kStage23 > kStage14 ? kStage23 : kStage14;
+// the last row that a core matrix of the shifted operands reads
+static_assert(6 + 240 + 15 + 15 < kFeatRows && 240 + 15 + 15 < kORows, "shifts stay inside");
+static_assert(16 * kSteps <= kARows && 3 + 16 * kSteps <= kBRows && 256 <= kHRows &&
+                  16 + 16 <= kHRows, "steps stay inside");
+
+struct GradShared {
+  uint64_t mbar[2];  // the products of a stage are done
+  uint32_t tmem;
+  int failed;        // a wait ran out
+};
+constexpr int kGradSmem = 2 * kStage + (int)sizeof(GradShared);
+static_assert(kStage % 16 == 0 && kGradSmem <= 227 * 1024, "stages");
+
+// FP32 accumulators, BF16 operands, both MN-major, M = 128.
+__host__ __device__ constexpr uint32_t instr(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n / 8) << 17) |
+         (8u << 24);
+}
+// MN-major operand without swizzle: distances of the core matrices that follow
+// each other in K (always the next eight rows) and in M or N.
+__device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t mn_bytes) {
+  return tfir::operand(addr, 128, mn_bytes);
+}
+// accumulator columns
+constexpr int kD0 = 0, kD1 = 96, kD2 = 160;   // layers 2, 3: shifts -1 (and ones), 1, 2
+constexpr int kDW1 = 0, kDb1 = 64, kDW4 = 128;
+
+__global__ void __launch_bounds__(kGradThreads, 1)
+    wgrad_kernel(const unsigned char* __restrict__ feat, const unsigned char* __restrict__ hid,
+                 const unsigned char* __restrict__ dpre, const unsigned char* __restrict__ dout,
+                 int n, int parts, float* __restrict__ partial) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  GradShared& S = *reinterpret_cast<GradShared*>(sm + 2 * kStage);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = blockIdx.x % kGroups, slot = blockIdx.x / kGroups;
+  if (tid == 0) {
+    for (int h = 0; h < 2; ++h)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tfir::saddr(&S.mbar[h])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    S.failed = 0;
+  }
+  if (warp == kLoaders / 32) tfir::tmem_alloc(&S.tmem);
+  // zero rows around the positions, and the rows of ones
+  for (int st = 0; st < 2; ++st) {
+    unsigned char* s = sm + st * kStage;
+    auto fill = [&](int off, uint32_t w) {
+      *reinterpret_cast<uint4*>(s + off) = make_uint4(w, w, w, w);
+    };
+    if (group < 2) {
+      for (int i = tid; i < 16 * 16; i += kGradThreads) {
+        const int c = i >> 4, r = i & 15;
+        fill(c * kAChunk + (c < 8 && r == 0 ? 0 : 256 + r) * 16, 0);
+      }
+      constexpr int kEdge = kBRows - kNS;
+      for (int i = tid; i < 8 * kEdge; i += kGradThreads) {
+        const int c = i / kEdge, r = i - c * kEdge;
+        fill(kOffB + c * kBChunk + (r < 2 ? r : kNS + r) * 16, 0);
+      }
+      for (int i = tid; i < 2 * kBRows; i += kGradThreads)
+        fill(kOffB + 8 * kBChunk + i * 16, 0x3f803f80u);
+    } else {
+      if (tid < kORows - kNS) fill(kOffO + (tid < 2 ? tid : kNS + tid) * 16, 0);
+      for (int i = tid; i < 2 * kHRows; i += kGradThreads)
+        fill(kOffH + 8 * kHChunk + i * 16, 0x3f803f80u);
+    }
+  }
+  tfir::fence_before();
+  __syncthreads();
+  tfir::fence_after();
+  const uint32_t tmem = __shfl_sync(kFull, S.tmem, 0);
+  const int64_t layer = (int64_t)n * kNS * 128;  // bytes of a layer of hid, dpre
+  const int records = slot < n ? (n - slot + parts - 1) / parts : 0;
+
+  if (warp == kLoaders / 32) {
+    const uint32_t issue = tfir::elected();
+    for (int it = 0; it < records; ++it) {
+      const int st = it & 1;
+      const uint32_t base = tfir::saddr(sm) + st * kStage;
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + st), "n"(kGradThreads) : "memory");
+      tfir::fence_after();
+      if (group < 2) {
+        const uint64_t a = operand(base, kAChunk), b = operand(base + kOffB, kBChunk);
+#pragma unroll 1
+        for (int k = 0; k < kSteps; ++k) {
+          const uint32_t add = it > 0 || k > 0;
+          const uint64_t ak = a + 16 * k, bk = b + 16 * k;  // 16 rows of 16 bytes
+          tfir::mma(tmem + kD0, ak, bk, add, issue, instr(80));
+          tfir::mma(tmem + kD1, ak, bk + 2, add, issue, instr(64));
+          tfir::mma(tmem + kD2, ak, bk + 3, add, issue, instr(64));
+        }
+      } else {
+        const uint64_t f = operand(base + 6 * 16, 16), o = operand(base + kOffO, 16),
+                       ones = operand(base + kOffH + 8 * kHChunk, 16),
+                       d = operand(base + kOffD, kHChunk), h = operand(base + kOffH, kHChunk);
+#pragma unroll 1
+        for (int k = 0; k < kNS / 16; ++k) {
+          const uint32_t add = it > 0 || k > 0;
+          tfir::mma(tmem + kDW1, f + 16 * k, d + 16 * k, add, issue, instr(64));
+          tfir::mma(tmem + kDb1, ones, d + 16 * k, add, issue, instr(64));
+          tfir::mma(tmem + kDW4, o + 16 * k, h + 16 * k, add, issue, instr(80));
+        }
+      }
+      if (issue) tfir::commit(&S.mbar[st]);
+      __syncwarp();
+    }
+  } else {
+    // Bounded; after a wait that ran out none waits, and the slot becomes NaN.
+    auto wait_stage = [&](int st, int phase) {
+      uint32_t done = 0;
+      const unsigned long long start = global_ns();
+      while (!done && !*(volatile int*)&S.failed) {
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            : "=r"(done)
+            : "r"(tfir::saddr(&S.mbar[st])), "r"((uint32_t)(phase & 1))
+            : "memory");
+        if (!done && global_ns() - start > kWaitNs) *(volatile int*)&S.failed = 1;
+      }
+    };
+    // 16 bytes u of a record: row u / 8, and its chunk by the rows' swizzle.  The
+    // first factor (dPre) in g[0..3], the second (In) in g[4..7]; layers 1 and 4
+    // have the features and dO in g[8], g[9].
+    const unsigned char* first = dpre + (group < 2 ? (group + 1) * layer : 0);
+    const unsigned char* second = hid + (group < 2 ? group * layer : 2 * layer);
+    uint4 g[10];
+    auto load = [&](int rec) {
+      const uint4* p = reinterpret_cast<const uint4*>(first + (int64_t)rec * kNS * 128);
+      const uint4* q = reinterpret_cast<const uint4*>(second + (int64_t)rec * kNS * 128);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g[j] = __ldg(p + tid + kLoaders * j);
+        g[4 + j] = __ldg(q + tid + kLoaders * j);
+      }
+      if (group == 2) {
+        if (tid < kFeatRows)
+          g[8] = __ldg(reinterpret_cast<const uint4*>(feat + (int64_t)rec * kFeat) + tid);
+        if (tid < kNS)
+          g[9] = __ldg(reinterpret_cast<const uint4*>(dout + (int64_t)rec * kNS * 16) + tid);
+      }
+    };
+    auto store = [&](int st) {
+      unsigned char* s = sm + st * kStage;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int u = tid + kLoaders * j, row = u >> 3, c = (u & 7) ^ (row & 7);
+        if (group < 2) {
+          *reinterpret_cast<uint4*>(s + c * kAChunk + (row + 1) * 16) = g[j];
+          *reinterpret_cast<uint4*>(s + (8 + c) * kAChunk + row * 16) = g[j];
+          *reinterpret_cast<uint4*>(s + kOffB + c * kBChunk + (row + 2) * 16) = g[4 + j];
+        } else {
+          *reinterpret_cast<uint4*>(s + kOffD + c * kHChunk + row * 16) = g[j];
+          *reinterpret_cast<uint4*>(s + kOffH + c * kHChunk + row * 16) = g[4 + j];
+        }
+      }
+      if (group == 2) {
+        if (tid < kFeatRows) *reinterpret_cast<uint4*>(s + tid * 16) = g[8];
+        if (tid < kNS) *reinterpret_cast<uint4*>(s + kOffO + (tid + 2) * 16) = g[9];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("bar.arrive %0, %1;" ::"r"(1 + st), "n"(kGradThreads) : "memory");
+    };
+    if (records) load(slot);
+    for (int it = 0; it < records; ++it) {
+      if (it >= 2) wait_stage(it & 1, (it >> 1) - 1);
+      store(it & 1);
+      if (it + 1 < records) load(slot + (it + 1) * parts);
+    }
+    if (records) wait_stage((records - 1) & 1, (records - 1) >> 1);
+    tfir::fence_after();
+
+    // The group's part of the slot, put together in shared memory (the products
+    // have been read): lane = row of M, sixteen columns of an accumulator a warp.
+    const bool failed = *(volatile int*)&S.failed;
+    float* const out = reinterpret_cast<float*>(sm);
+    const int quarter = warp & 3, m = 32 * quarter + lane, c0 = (warp >> 2) * 16;
+    const uint32_t from = tmem + ((uint32_t)(32 * quarter) << 16);
+    auto read = [&](int col, float (&v)[8]) {
+      tfir::tmem_load8(from + col, v);
+      tfir::tmem_wait_loads();
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        v[i] = failed ? __int_as_float(0x7fffffff) : (records ? v[i] : 0.0f);
+    };
+    auto put = [](float* dst, const float (&v)[8]) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dst[i] = v[i];
+    };
+    float* part = partial + (int64_t)slot * kParams;
+    float v[8];
+    if (group < 2) {
+      constexpr int kPitch = 65;  // [tap][co] rows of 64 ci, then the bias gradients
+      const int half = m >> 6, co = m & 63;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int tap = (j == 0 ? 1 : j + 2) - half;
+#pragma unroll
+        for (int c = 0; c < 16; c += 8) {
+          read((j == 0 ? kD0 : j == 1 ? kD1 : kD2) + c0 + c, v);
+          if (!(j == 2 && half)) put(out + (tap * 64 + co) * kPitch + c0 + c, v);
+        }
+      }
+      if (c0 == 0) {
+        read(kD0 + 64, v);
+        if (!half) out[co * kPitch + 64] = v[0];
+      }
+      asm volatile("bar.sync 3, %0;" ::"n"(kLoaders) : "memory");
+      static_assert(ob2 == oW2 + 5 * 64 * 64 && ob3 == oW3 + 5 * 64 * 64, "bias after weights");
+      float* W = part + (group ? oW3 : oW2);
+#pragma unroll 8
+      for (int i = tid; i < 5 * 64 * 64; i += kLoaders) W[i] = out[(i >> 6) * kPitch + (i & 63)];
+      if (tid < 64) W[5 * 64 * 64 + tid] = out[tid * kPitch + 64];
+    } else {
+      constexpr int kPitch = 9;  // [tap][co] rows of 8 ci; b1; W4, b4
+      float* const out4 = out + 5 * 64 * kPitch + 64;
+#pragma unroll 1
+      for (int c = c0; c < c0 + 16; c += 8) {
+        read(kDW1 + c, v);
+        if (m < 40)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) out[((m >> 3) * 64 + c + i) * kPitch + (m & 7)] = v[i];
+        read(kDb1 + c, v);
+        if (m == 0) put(out + 5 * 64 * kPitch + c, v);
+        read(kDW4 + c, v);
+        if (m < 40 && (m & 7) == 0) put(out4 + (4 - (m >> 3)) * 64 + c, v);
+      }
+      if (c0 == 0) {
+        read(kDW4 + 64, v);
+        if (m == 16) out4[5 * 64] = v[0];
+      }
+      asm volatile("bar.sync 3, %0;" ::"n"(kLoaders) : "memory");
+      static_assert(ob1 == oW1 + 5 * 64 * 8 && ob4 == oW4 + 5 * 64, "bias after weights");
+      for (int i = tid; i < 5 * 64 * 8; i += kLoaders)
+        part[oW1 + i] = out[(i >> 3) * kPitch + (i & 7)];
+      if (tid < 64) part[ob1 + tid] = out[5 * 64 * kPitch + tid];
+      if (tid < 5 * 64 + 1) part[oW4 + tid] = out4[tid];
+    }
+    tfir::fence_before();
+  }
+  __syncthreads();
+  if (warp == kLoaders / 32) tfir::tmem_free(tmem);
+}
+
+// Sum over the slots in order, as an unevaluated FP32 pair (FP64 runs at a 64th of
+// the rate); a sum that leaves the FP32 range on the way is taken in FP64.
+__global__ void __launch_bounds__(128) reduce_kernel(const float* __restrict__ partial, int parts,
+                                                     float* __restrict__ grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kParams) return;
+  const float* p = partial + i;
+  float s = 0.0f, c = 0.0f;
+#pragma unroll 10
+  for (int k = 0; k < parts; ++k) two_sum_add(s, c, __ldg(p + (int64_t)k * kParams));
+  float total = __fadd_rn(s, c);
+  if (!(fabsf(total) < __int_as_float(0x7f800000))) {
+    double d = 0.0;
+    for (int k = 0; k < parts; ++k) d += (double)p[(int64_t)k * kParams];
+    total = (float)d;
+  }
+  grad[i] = total;
+}
+
+}  // namespace
+}  // namespace ws
+}  // namespace cgb
+
+using namespace cgb;
+using namespace cgb::ws;
+
+extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const void* d_dpre,
+                                const void* d_dout, int n, float* d_partial, int n_parts,
+                                float* d_grad, void* stream) {
+  if (n < 0 || n_parts < 1 || !d_feat || !d_hid || !d_dpre || !d_dout || !d_partial || !d_grad)
+    return fail(CGB_ERR_ARG, "cgb_ws_wgrad_dev: bad arguments");
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  int dev = 0, sms = 0;
+  CGB_TRY_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
+  CGB_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
+               "cudaDeviceGetAttribute");
+  // one CTA fits an SM: all of them at once, and no more slots than records
+  int parts = sms / kGroups < n_parts ? sms / kGroups : n_parts;
+  if (parts > n) parts = n;
+  if (parts < 1) parts = 1;
+  CGB_TRY_CUDA(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kGradSmem),
+               "cudaFuncSetAttribute(wgrad)");
+  wgrad_kernel<<<kGroups * parts, kGradThreads, kGradSmem, st>>>(
+      static_cast<const unsigned char*>(d_feat), static_cast<const unsigned char*>(d_hid),
+      static_cast<const unsigned char*>(d_dpre), static_cast<const unsigned char*>(d_dout), n,
+      parts, d_partial);
+  CGB_TRY_CUDA(cudaGetLastError(), "wgrad_kernel launch");
+  note_launch();
+  reduce_kernel<<<(kParams + 127) / 128, 128, 0, st>>>(d_partial, parts, d_grad);
+  CGB_TRY_CUDA(cudaGetLastError(), "reduce_kernel launch");
+  note_launch();
+  return CGB_OK;
+}
