@@ -4,15 +4,15 @@
 // training step is
 //   prepare (once): features + exact pressure (FP64 tridiagonal solve) of
 //                   logged step starts -> raw targets (p* - pe) / max|rt|
-//   forward       : one CTA per record, the four layers in shared memory,
-//                   hidden activations (BF16) kept for the backward pass
+//   forward       : warmstart_conv.cu, hidden activations (BF16) kept for the
+//                   backward pass
 //   loss          : pred = s_out * o, MSE against the raw target; dL/do (BF16)
-//   backward      : one CTA per record, the transposed convolutions with the
+//   backward      : warmstart_conv.cu, the transposed convolutions with the
 //                   ReLU masks -> pre-activation gradients (BF16)
 //   weight grad   : warmstart_grad.cu
 //   adam          : FP32 master parameters, then re-packed to BF16.
-// All products run on the tensor cores (mma.sync m16n8k16 BF16, FP32
-// accumulate); ldmatrix (.trans for the weight gradients) feeds them.
+// The inference runs as in the BM kernel, a warp to a record (mma.sync m16n8k16
+// BF16, FP32 accumulate); the training passes on tcgen05.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -24,8 +24,6 @@
 namespace cgb {
 namespace ws {
 
-constexpr int kRows = 272;            // 64-channel rows per record: position + 8
-constexpr int kHBytes = kNS * 128;    // one stored hidden layer of one record
 constexpr int kFeatBytes = kFeatRows * 16;
 
 __device__ __forceinline__ uint16_t bf16_half(float f) { return (uint16_t)bf16_bits(f); }
@@ -147,75 +145,10 @@ __global__ void prepare_kernel(const float* __restrict__ rec, int n, const float
   if (lane == 0) nr_out[wid] = nr;
 }
 
-// ---------------------------------------------------------------------------
-// Forward: one CTA (8 warps) per record.
-// ---------------------------------------------------------------------------
-constexpr int kFwdSmem = kBlobBytes + kFeatBytes + 2 * kRows * 128;
-
 __device__ __forceinline__ void copy16(void* dst, const void* src, int bytes, int tid, int nth) {
   const uint4* s = reinterpret_cast<const uint4*>(src);
   uint4* d = reinterpret_cast<uint4*>(dst);
   for (int i = tid; i < bytes / 16; i += nth) d[i] = s[i];
-}
-__device__ __forceinline__ void zero16(void* dst, int bytes, int tid, int nth) {
-  uint4* d = reinterpret_cast<uint4*>(dst);
-  for (int i = tid; i < bytes / 16; i += nth) d[i] = make_uint4(0, 0, 0, 0);
-}
-
-__global__ void __launch_bounds__(256) forward_kernel(const unsigned char* __restrict__ blob,
-                                                      const unsigned char* __restrict__ feat,
-                                                      int n, unsigned char* __restrict__ hid,
-                                                      float* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  unsigned char* sw = sm;
-  unsigned char* sF = sw + kBlobBytes;
-  unsigned char* sA = sF + kFeatBytes;
-  unsigned char* sB = sA + kRows * 128;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  copy16(sw, blob, kBlobBytes, tid, 256);
-  zero16(sA, 2 * kRows * 128, tid, 256);
-  const float* bias = reinterpret_cast<const float*>(sw + kOffBias);
-  const uint32_t uW1 = smem_u32(sw + kOffW1), uW2 = smem_u32(sw + kOffW2),
-                 uW3 = smem_u32(sw + kOffW3), uW4 = smem_u32(sw + kOffW4);
-  const uint32_t uF = smem_u32(sF), uA = smem_u32(sA), uB = smem_u32(sB);
-  const int g = lane >> 2, t = lane & 3;
-  for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-    __syncthreads();
-    copy16(sF, feat + (int64_t)rec * kFeatBytes, kFeatBytes, tid, 256);
-    __syncthreads();
-    unsigned char* h = hid + (int64_t)rec * kHBytes;  // layer l at h + l * n * kHBytes
-    float acc[8][4];
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv8_tile(acc, uF, 16 * mt + 6, uW1, lane);
-      store_hidden(acc, sA, 8 + 16 * mt, 16 * mt, bias, lane);
-    }
-    __syncthreads();
-    copy16(h, sA + 8 * 128, kHBytes, tid, 256);
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv64_tile<8>(acc, uA, 16 * mt + 6, uW2, lane);
-      store_hidden(acc, sB, 8 + 16 * mt, 16 * mt, bias + 64, lane);
-    }
-    __syncthreads();
-    copy16(h + (int64_t)n * kHBytes, sB + 8 * 128, kHBytes, tid, 256);
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv64_tile<8>(acc, uB, 16 * mt + 6, uW3, lane);
-      store_hidden(acc, sA, 8 + 16 * mt, 16 * mt, bias + 128, lane);
-    }
-    __syncthreads();
-    copy16(h + 2 * (int64_t)n * kHBytes, sA + 8 * 128, kHBytes, tid, 256);
-    for (int mt = warp; mt < 16; mt += 8) {
-      float o[1][4];
-      zero_acc(o);
-      conv64_tile<1>(o, uA, 16 * mt + 6, uW4, lane);
-      if (t == 0) {
-        out[(int64_t)rec * 256 + 16 * mt + g] = o[0][0] + bias[192];
-        out[(int64_t)rec * 256 + 16 * mt + g + 8] = o[0][2] + bias[192];
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -238,78 +171,6 @@ __global__ void loss_kernel(const float* __restrict__ out, const float* __restri
     __syncthreads();
   }
   if (s == 0) loss_part[rec] = red[0];
-}
-
-// ---------------------------------------------------------------------------
-// Backward (data): one CTA per record.
-//   dH3 = (W4^T * dO) . [H3 > 0], dH2 = (W3^T * dH3) . [H2 > 0],
-//   dH1 = (W2^T * dH2) . [H1 > 0], each a convolution with the transposed,
-//   tap-reversed weights.  Stored as BF16 64-channel rows (row = position).
-// ---------------------------------------------------------------------------
-constexpr int kBwdSmem = kBlobTBytes + kFeatBytes + 2 * kRows * 128;
-
-__device__ __forceinline__ void store_masked(const float (&acc)[8][4], unsigned char* sout,
-                                             int out_row0, int pos0,
-                                             const unsigned char* __restrict__ mask,
-                                             unsigned char* __restrict__ gout, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int pos = pos0 + g + 8 * h;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const int col = nt * 8 + 2 * t;
-      const int off = swz64(pos, col >> 3) + (col & 7) * 2;
-      const uint32_t m = *reinterpret_cast<const uint32_t*>(mask + off);
-      const float lo = bf16_lo(m) > 0.0f ? acc[nt][2 * h] : 0.0f;
-      const float hi = bf16_hi(m) > 0.0f ? acc[nt][2 * h + 1] : 0.0f;
-      const uint32_t w = pack_bf16(lo, hi);
-      if (sout) *reinterpret_cast<uint32_t*>(sout + swz64(out_row0 + g + 8 * h, col >> 3) +
-                                             (col & 7) * 2) = w;
-      *reinterpret_cast<uint32_t*>(gout + off) = w;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) backward_kernel(const unsigned char* __restrict__ blobT,
-                                                       const unsigned char* __restrict__ dout,
-                                                       const unsigned char* __restrict__ hid,
-                                                       int n, unsigned char* __restrict__ dpre) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  unsigned char* sw = sm;
-  unsigned char* sO = sw + kBlobTBytes;
-  unsigned char* sA = sO + kFeatBytes;
-  unsigned char* sB = sA + kRows * 128;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  copy16(sw, blobT, kBlobTBytes, tid, 256);
-  zero16(sO, kFeatBytes + 2 * kRows * 128, tid, 256);
-  const uint32_t uT4 = smem_u32(sw + kOffT4), uT3 = smem_u32(sw + kOffT3),
-                 uT2 = smem_u32(sw + kOffT2);
-  const uint32_t uO = smem_u32(sO), uA = smem_u32(sA), uB = smem_u32(sB);
-  for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-    __syncthreads();
-    copy16(sO + 8 * 16, dout + (int64_t)rec * 256 * 16, 256 * 16, tid, 256);
-    __syncthreads();
-    const int64_t ro = (int64_t)rec * kHBytes, lo = (int64_t)n * kHBytes;
-    float acc[8][4];
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv8_tile(acc, uO, 16 * mt + 6, uT4, lane);
-      store_masked(acc, sA, 8 + 16 * mt, 16 * mt, hid + 2 * lo + ro, dpre + 2 * lo + ro, lane);
-    }
-    __syncthreads();
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv64_tile<8>(acc, uA, 16 * mt + 6, uT3, lane);
-      store_masked(acc, sB, 8 + 16 * mt, 16 * mt, hid + lo + ro, dpre + lo + ro, lane);
-    }
-    __syncthreads();
-    for (int mt = warp; mt < 16; mt += 8) {
-      zero_acc(acc);
-      conv64_tile<8>(acc, uB, 16 * mt + 6, uT2, lane);
-      store_masked(acc, nullptr, 0, 16 * mt, hid + ro, dpre + ro, lane);
-    }
-  }
 }
 
 __global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ grad,
@@ -404,20 +265,6 @@ extern "C" int cgb_ws_prepare_dev(const float* d_rec, int n, const float* d_rm, 
   return CGB_OK;
 }
 
-extern "C" int cgb_ws_forward_dev(const void* d_blob, const void* d_feat, int n, void* d_hid,
-                                  float* d_out, void* stream) {
-  if (n == 0) return CGB_OK;
-  if (n < 0 || !d_blob || !d_feat || !d_hid || !d_out)
-    return fail(CGB_ERR_ARG, "cgb_ws_forward_dev: bad arguments");
-  if (set_smem(forward_kernel, kFwdSmem, "cudaFuncSetAttribute(forward)")) return CGB_ERR_CUDA;
-  forward_kernel<<<grid_for(n, 1), 256, kFwdSmem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const unsigned char*>(d_blob), static_cast<const unsigned char*>(d_feat), n,
-      static_cast<unsigned char*>(d_hid), d_out);
-  CGB_TRY_CUDA(cudaGetLastError(), "forward_kernel launch");
-  note_launch();
-  return CGB_OK;
-}
-
 extern "C" int cgb_ws_loss_dev(const float* d_out, const float* d_target, int n, float s_out,
                                void* d_dout, double* d_loss_part, void* stream) {
   if (n == 0) return CGB_OK;
@@ -426,20 +273,6 @@ extern "C" int cgb_ws_loss_dev(const float* d_out, const float* d_target, int n,
   loss_kernel<<<n, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       d_out, d_target, n, s_out, static_cast<unsigned char*>(d_dout), d_loss_part);
   CGB_TRY_CUDA(cudaGetLastError(), "loss_kernel launch");
-  note_launch();
-  return CGB_OK;
-}
-
-extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, const void* d_hid,
-                                   int n, void* d_dpre, void* stream) {
-  if (n == 0) return CGB_OK;
-  if (n < 0 || !d_blobT || !d_dout || !d_hid || !d_dpre)
-    return fail(CGB_ERR_ARG, "cgb_ws_backward_dev: bad arguments");
-  if (set_smem(backward_kernel, kBwdSmem, "cudaFuncSetAttribute(backward)")) return CGB_ERR_CUDA;
-  backward_kernel<<<grid_for(n, 1), 256, kBwdSmem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const unsigned char*>(d_blobT), static_cast<const unsigned char*>(d_dout),
-      static_cast<const unsigned char*>(d_hid), n, static_cast<unsigned char*>(d_dpre));
-  CGB_TRY_CUDA(cudaGetLastError(), "backward_kernel launch");
   note_launch();
   return CGB_OK;
 }

@@ -34,9 +34,8 @@
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
-#include "ihc_common.cuh"
-#include "tensor_fir.cuh"
 #include "warmstart.cuh"
+#include "warmstart_tensor.cuh"
 
 namespace cgb {
 namespace ws {
@@ -68,19 +67,9 @@ static_assert(6 + 240 + 15 + 15 < kFeatRows && 240 + 15 + 15 < kORows, "shifts s
 static_assert(16 * kSteps <= kARows && 3 + 16 * kSteps <= kBRows && 256 <= kHRows &&
                   16 + 16 <= kHRows, "steps stay inside");
 
-struct GradShared {
-  uint64_t mbar[2];  // the products of a stage are done
-  uint32_t tmem;
-  int failed;        // a wait ran out
-};
-constexpr int kGradSmem = 2 * kStage + (int)sizeof(GradShared);
+constexpr int kGradSmem = 2 * kStage + (int)sizeof(TensorShared);
 static_assert(kStage % 16 == 0 && kGradSmem <= 227 * 1024, "stages");
 
-// FP32 accumulators, BF16 operands, both MN-major, M = 128.
-__host__ __device__ constexpr uint32_t instr(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(n / 8) << 17) |
-         (8u << 24);
-}
 // MN-major operand without swizzle: distances of the core matrices that follow
 // each other in K (always the next eight rows) and in M or N.
 __device__ __forceinline__ uint64_t operand(uint32_t addr, uint32_t mn_bytes) {
@@ -95,15 +84,10 @@ __global__ void __launch_bounds__(kGradThreads, 1)
                  const unsigned char* __restrict__ dpre, const unsigned char* __restrict__ dout,
                  int n, int parts, float* __restrict__ partial) {
   extern __shared__ __align__(128) unsigned char sm[];
-  GradShared& S = *reinterpret_cast<GradShared*>(sm + 2 * kStage);
+  TensorShared& S = *reinterpret_cast<TensorShared*>(sm + 2 * kStage);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = blockIdx.x % kGroups, slot = blockIdx.x / kGroups;
-  if (tid == 0) {
-    for (int h = 0; h < 2; ++h)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tfir::saddr(&S.mbar[h])));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    S.failed = 0;
-  }
+  if (tid == 0) init_barriers(S);
   if (warp == kLoaders / 32) tfir::tmem_alloc(&S.tmem);
   // zero rows around the positions, and the rows of ones
   for (int st = 0; st < 2; ++st) {
@@ -149,9 +133,9 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         for (int k = 0; k < kSteps; ++k) {
           const uint32_t add = it > 0 || k > 0;
           const uint64_t ak = a + 16 * k, bk = b + 16 * k;  // 16 rows of 16 bytes
-          tfir::mma(tmem + kD0, ak, bk, add, issue, instr(80));
-          tfir::mma(tmem + kD1, ak, bk + 2, add, issue, instr(64));
-          tfir::mma(tmem + kD2, ak, bk + 3, add, issue, instr(64));
+          tfir::mma(tmem + kD0, ak, bk, add, issue, instr(80, true));
+          tfir::mma(tmem + kD1, ak, bk + 2, add, issue, instr(64, true));
+          tfir::mma(tmem + kD2, ak, bk + 3, add, issue, instr(64, true));
         }
       } else {
         const uint64_t f = operand(base + 6 * 16, 16), o = operand(base + kOffO, 16),
@@ -160,28 +144,15 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 #pragma unroll 1
         for (int k = 0; k < kNS / 16; ++k) {
           const uint32_t add = it > 0 || k > 0;
-          tfir::mma(tmem + kDW1, f + 16 * k, d + 16 * k, add, issue, instr(64));
-          tfir::mma(tmem + kDb1, ones, d + 16 * k, add, issue, instr(64));
-          tfir::mma(tmem + kDW4, o + 16 * k, h + 16 * k, add, issue, instr(80));
+          tfir::mma(tmem + kDW1, f + 16 * k, d + 16 * k, add, issue, instr(64, true));
+          tfir::mma(tmem + kDb1, ones, d + 16 * k, add, issue, instr(64, true));
+          tfir::mma(tmem + kDW4, o + 16 * k, h + 16 * k, add, issue, instr(80, true));
         }
       }
       if (issue) tfir::commit(&S.mbar[st]);
       __syncwarp();
     }
   } else {
-    // Bounded; after a wait that ran out none waits, and the slot becomes NaN.
-    auto wait_stage = [&](int st, int phase) {
-      uint32_t done = 0;
-      const unsigned long long start = global_ns();
-      while (!done && !*(volatile int*)&S.failed) {
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(done)
-            : "r"(tfir::saddr(&S.mbar[st])), "r"((uint32_t)(phase & 1))
-            : "memory");
-        if (!done && global_ns() - start > kWaitNs) *(volatile int*)&S.failed = 1;
-      }
-    };
     // 16 bytes u of a record: row u / 8, and its chunk by the rows' swizzle.  The
     // first factor (dPre) in g[0..3], the second (In) in g[4..7]; layers 1 and 4
     // have the features and dO in g[8], g[9].
@@ -226,11 +197,11 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     };
     if (records) load(slot);
     for (int it = 0; it < records; ++it) {
-      if (it >= 2) wait_stage(it & 1, (it >> 1) - 1);
+      if (it >= 2) wait_products(S, it & 1, (it >> 1) - 1);
       store(it & 1);
       if (it + 1 < records) load(slot + (it + 1) * parts);
     }
-    if (records) wait_stage((records - 1) & 1, (records - 1) >> 1);
+    if (records) wait_products(S, (records - 1) & 1, (records - 1) >> 1);  // (after one that ran out: NaN)
     tfir::fence_after();
 
     // The group's part of the slot, put together in shared memory (the products

@@ -1,12 +1,13 @@
-"""Weight gradients of the warm-start network against FP64 sums of the same
-BF16 factors."""
+"""Training kernels of the warm-start network: weight gradients and the backward
+pass against FP64 sums of the same BF16 factors, the forward pass against the
+fused inference."""
 import ctypes as C
 
 import numpy as np
 import pytest
 import torch
 
-from cochlearmodel_gb300 import native
+from cochlearmodel_gb300 import native, warmstart
 
 pytestmark = pytest.mark.gpu
 D = "cuda:0"
@@ -58,3 +59,50 @@ def test_weight_gradients_match_fp64(n, parts):
     tol = (16 + 17 * max(n, 1) + parts) * 2.0 ** -23 * size
     got = grad.double().cpu().numpy()
     assert np.all(np.abs(got - want) <= tol), np.max(np.abs(got - want) / np.maximum(tol, 1e-30))
+
+
+# fewer records than SMs, one more, and several for each
+@pytest.mark.parametrize("n", [1, 2, 153, 500])
+def test_forward_and_backward_layers(n):
+    g = torch.Generator(device=D).manual_seed(n)
+    net = warmstart.WarmStartNet(D, seed=n)
+    net.params += 0.05 * torch.randn(net.n_params, generator=g, device=D)
+    net.pack()
+    feat = torch.zeros(n, 280, 8, dtype=torch.bfloat16, device=D)
+    feat[:, 8:264] = torch.randn(n, 256, 8, generator=g, device=D).to(torch.bfloat16)
+    buf = net.buffers(n)
+    out = net.forward(feat, buf)
+    assert torch.equal(out.view(torch.int32), net.infer(feat).view(torch.int32))
+
+    w = net.params.to(torch.bfloat16).double()
+    size = [2560, 64, 20480, 64, 20480, 64, 320, 1]
+    W1, b1, W2, b2, W3, b3, W4, b4 = torch.split(w, size)
+    bias = dict(zip((1, 2, 3), torch.split(net.params.double(), size)[1:6:2]))
+    eps = 2.0 ** -8 + 2.0 ** -16  # BF16 half ulp; a sum of 320 products in FP32 on top:
+    acc = 340 * 2.0 ** -23
+
+    def close(got, want, size):
+        return bool(((got - want).abs() <= eps * want.abs() + acc * size).all())
+
+    # each hidden layer from the one before as the kernel stored it
+    h = [feat[:, 8:264].double(), *rows64(buf["hid"]).double()]
+    for layer, W, cin in ((1, W1, 8), (2, W2, 64), (3, W3, 64)):
+        W = W.reshape(5, 64, cin)
+        sums = lambda x, w: sum(  # noqa: E731
+            torch.nn.functional.pad(x, (0, 0, 2, 2))[:, t:t + 256] @ w[t].T for t in range(5))
+        assert close(h[layer], (sums(h[layer - 1], W) + bias[layer]).relu(),
+                     sums(h[layer - 1].abs(), W.abs()) + bias[layer].abs()), layer
+
+    buf["dout"][:, :, 0] = torch.randn(n, 256, generator=g, device=D).to(torch.bfloat16)
+    p = native.ptr
+    native.check(net.lib.cgb_ws_backward_dev(
+        p(net.blobT), p(buf["dout"]), p(buf["hid"]), n, p(buf["dpre"]),
+        C.c_void_p(torch.cuda.current_stream().cuda_stream)), "cgb_ws_backward_dev")
+    d = [*rows64(buf["dpre"]).double(), buf["dout"][:, :, :1].double()]
+    for layer, W, cout in ((2, W4, 1), (1, W3, 64), (0, W2, 64)):
+        W = W.reshape(5, cout, 64)
+        sums = lambda x, w: sum(  # noqa: E731
+            torch.nn.functional.pad(x, (0, 0, 2, 2))[:, 4 - t:260 - t] @ w[t] for t in range(5))
+        on = h[layer + 1] > 0
+        assert close(d[layer], sums(d[layer + 1], W) * on,
+                     sums(d[layer + 1].abs(), W.abs()) * on), layer
