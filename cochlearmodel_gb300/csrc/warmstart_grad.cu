@@ -277,14 +277,31 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 }
 
 // Sum over the slots in order, as an unevaluated FP32 pair (FP64 runs at a 64th of
-// the rate); a sum that leaves the FP32 range on the way is taken in FP64.
-__global__ void __launch_bounds__(128) reduce_kernel(const float* __restrict__ partial, int parts,
-                                                     float* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// the rate); a sum that leaves the FP32 range on the way is taken in FP64.  The last
+// CTA, if there is a loss to be given, takes the records' losses instead.
+constexpr int kSumThreads = 128;
+
+__global__ void __launch_bounds__(kSumThreads)
+    reduce_kernel(const float* __restrict__ partial, int parts, float* __restrict__ grad,
+                  const double* __restrict__ loss_part, int n, double* __restrict__ loss) {
+  if (loss && blockIdx.x == gridDim.x - 1) {
+    __shared__ double red[kSumThreads];
+    double d = 0.0;
+    for (int k = threadIdx.x; k < n; k += kSumThreads) d += loss_part[k];
+    red[threadIdx.x] = d;
+    __syncthreads();
+    for (int o = kSumThreads / 2; o >= 1; o >>= 1) {
+      if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = red[0] / ((double)n * kNS);
+    return;
+  }
+  const int i = blockIdx.x * kSumThreads + threadIdx.x;
   if (i >= kParams) return;
   const float* p = partial + i;
   float s = 0.0f, c = 0.0f;
-#pragma unroll 10
+#pragma unroll 25
   for (int k = 0; k < parts; ++k) two_sum_add(s, c, __ldg(p + (int64_t)k * kParams));
   float total = __fadd_rn(s, c);
   if (!(fabsf(total) < __int_as_float(0x7f800000))) {
@@ -302,12 +319,14 @@ __global__ void __launch_bounds__(128) reduce_kernel(const float* __restrict__ p
 using namespace cgb;
 using namespace cgb::ws;
 
-extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const void* d_dpre,
-                                const void* d_dout, int n, float* d_partial, int n_parts,
-                                float* d_grad, void* stream) {
+namespace {
+
+// loss_part, loss: null, or the records' losses and where their mean goes.
+int launch_wgrad(const void* d_feat, const void* d_hid, const void* d_dpre, const void* d_dout,
+                 int n, float* d_partial, int n_parts, float* d_grad, const double* loss_part,
+                 double* loss, cudaStream_t st) {
   if (n < 0 || n_parts < 1 || !d_feat || !d_hid || !d_dpre || !d_dout || !d_partial || !d_grad)
     return fail(CGB_ERR_ARG, "cgb_ws_wgrad_dev: bad arguments");
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int dev = 0, sms = 0;
   CGB_TRY_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
   CGB_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
@@ -325,8 +344,32 @@ extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const voi
       parts, d_partial);
   CGB_TRY_CUDA(cudaGetLastError(), "wgrad_kernel launch");
   note_launch();
-  reduce_kernel<<<(kParams + 127) / 128, 128, 0, st>>>(d_partial, parts, d_grad);
+  reduce_kernel<<<(kParams + kSumThreads - 1) / kSumThreads + (loss ? 1 : 0), kSumThreads, 0, st>>>(
+      d_partial, parts, d_grad, loss_part, n, loss);
   CGB_TRY_CUDA(cudaGetLastError(), "reduce_kernel launch");
   note_launch();
   return CGB_OK;
+}
+
+}  // namespace
+
+extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const void* d_dpre,
+                                const void* d_dout, int n, float* d_partial, int n_parts,
+                                float* d_grad, void* stream) {
+  return launch_wgrad(d_feat, d_hid, d_dpre, d_dout, n, d_partial, n_parts, d_grad, nullptr,
+                      nullptr, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, const void* d_feat,
+                                    const float* d_target, int n, float s_out, void* d_hid,
+                                    float* d_out, void* d_dout, void* d_dpre, double* d_loss_part,
+                                    float* d_partial, int n_parts, double* d_loss, float* d_grad,
+                                    void* stream) {
+  if (!d_loss) return fail(CGB_ERR_ARG, "cgb_ws_gradients_dev: bad arguments");
+  if (const int rc = cgb_ws_forward_dev(d_blob, d_feat, n, d_hid, d_out, stream)) return rc;
+  if (const int rc = cgb_ws_loss_dev(d_out, d_target, n, s_out, d_dout, d_loss_part, stream))
+    return rc;
+  if (const int rc = cgb_ws_backward_dev(d_blobT, d_dout, d_hid, n, d_dpre, stream)) return rc;
+  return launch_wgrad(d_feat, d_hid, d_dpre, d_dout, n, d_partial, n_parts, d_grad, d_loss_part,
+                      d_loss, reinterpret_cast<cudaStream_t>(stream));
 }

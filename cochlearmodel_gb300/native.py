@@ -103,6 +103,8 @@ _SIGS = {
     "cgb_ws_loss_dev": (_i, [_p, _p, _i, C.c_float, _p, _p, _p]),
     "cgb_ws_backward_dev": (_i, [_p, _p, _p, _i, _p, _p]),
     "cgb_ws_wgrad_dev": (_i, [_p, _p, _p, _p, _i, _p, _i, _p, _p]),
+    "cgb_ws_gradients_dev": (_i, [_p, _p, _p, _p, _i, C.c_float, _p, _p, _p, _p, _p, _p, _i, _p,
+                                  _p, _p]),
     "cgb_ws_adam_dev": (_i, [_p, _p, _p, _p, _i, C.c_float, C.c_float, C.c_float, C.c_float,
                              _p]),
     "cgb_ws_infer_dev": (_i, [_p, _p, _i, _p, _p]),

@@ -183,24 +183,17 @@ class WarmStartNet:
         """Forward, loss and backward; returns (mean loss tensor, grad tensor)."""
         n = int(feat.shape[0])
         buf = buf or self.buffers(n)
-        st = _stream(self.device)
-        lib = self.lib
-        self.forward(feat, buf)
-        native.check(lib.cgb_ws_loss_dev(native.ptr(buf["out"]), native.ptr(target), n,
-                                         self.s_out, native.ptr(buf["dout"]),
-                                         native.ptr(buf["loss"]), st), "cgb_ws_loss_dev")
-        native.check(lib.cgb_ws_backward_dev(native.ptr(self.blobT), native.ptr(buf["dout"]),
-                                             native.ptr(buf["hid"]), n, native.ptr(buf["dpre"]),
-                                             st), "cgb_ws_backward_dev")
         parts = n_parts or max(1, min(n, 2 * _sm_count(self.device)))
         if "partial" not in buf or buf["partial"].shape[0] < parts:
             buf["partial"] = torch.zeros((parts, self.n_params), dtype=torch.float32,
                                          device=self.device)
-        native.check(lib.cgb_ws_wgrad_dev(native.ptr(feat), native.ptr(buf["hid"]),
-                                          native.ptr(buf["dpre"]), native.ptr(buf["dout"]), n,
-                                          native.ptr(buf["partial"]), parts,
-                                          native.ptr(buf["grad"]), st), "cgb_ws_wgrad_dev")
-        return buf["loss"].sum() / (n * 256), buf["grad"]
+        loss = torch.empty((), dtype=torch.float64, device=self.device)
+        p = native.ptr
+        native.check(self.lib.cgb_ws_gradients_dev(
+            p(self.blob), p(self.blobT), p(feat), p(target), n, self.s_out, p(buf["hid"]),
+            p(buf["out"]), p(buf["dout"]), p(buf["dpre"]), p(buf["loss"]), p(buf["partial"]),
+            parts, p(loss), p(buf["grad"]), _stream(self.device)), "cgb_ws_gradients_dev")
+        return loss, buf["grad"]
 
     def adam(self, grad: torch.Tensor, lr: float) -> None:
         self.step += 1

@@ -239,6 +239,12 @@ int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, const void* d_h
 int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const void* d_dpre,
                      const void* d_dout, int n, float* d_partial, int n_parts, float* d_grad,
                      void* stream);
+/* Forward, loss, backward and weight gradients in one call; d_loss (device)
+ * receives the mean loss. */
+int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, const void* d_feat,
+                         const float* d_target, int n, float s_out, void* d_hid, float* d_out,
+                         void* d_dout, void* d_dpre, double* d_loss_part, float* d_partial,
+                         int n_parts, double* d_loss, float* d_grad, void* stream);
 int cgb_ws_adam_dev(float* d_params, const float* d_grad, float* d_m, float* d_v, int step,
                     float lr, float beta1, float beta2, float eps, void* stream);
 int cgb_ws_infer_dev(const void* d_blob, const void* d_feat, int n, float* d_out, void* stream);

@@ -106,3 +106,19 @@ def test_forward_and_backward_layers(n):
         on = h[layer + 1] > 0
         assert close(d[layer], sums(d[layer + 1], W) * on,
                      sums(d[layer + 1].abs(), W.abs()) * on), layer
+
+
+@pytest.mark.parametrize("n", [1, 129, 700])
+def test_mean_loss(n):
+    g = torch.Generator(device=D).manual_seed(n)
+    net = warmstart.WarmStartNet(D, seed=n)
+    feat = torch.zeros(n, 280, 8, dtype=torch.bfloat16, device=D)
+    feat[:, 8:264] = torch.randn(n, 256, 8, generator=g, device=D).to(torch.bfloat16)
+    target = torch.randn(n, 256, generator=g, device=D)
+    buf = net.buffers(n)
+    loss, grad = net.gradients(feat, target, buf)
+    e = net.s_out * buf["out"] - target  # FP32, as the kernel forms it
+    want = float(np.sum(np.square(e.cpu().numpy().astype(np.float64)))) / (n * 256)
+    # an FP32 product and difference (two roundings) per term, or one if contracted
+    assert abs(float(loss) - want) <= 2.0 ** -21 * want
+    assert abs(float(loss) - float(buf["loss"].sum()) / (n * 256)) <= (n + 16) * 2.0 ** -52 * want
