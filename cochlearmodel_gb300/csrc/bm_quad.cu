@@ -20,15 +20,18 @@
 // 24, and a solve has 10 rounds.
 //
 // The three kinds of outer iteration are compiled apart, and the sums' shuffle
-// rounds are spread over them; 1.4k warp instructions a substep, 3.5k cycles.
+// rounds are spread over them; 1.4k warp instructions a substep, 3.4k cycles.
 //
 // Measured (GB300, 5 ms blocks with 1 ms overlap, kernel 17 / the default
-// kernel's semantics), against a warp per unit: 1 unit 17.5 / 37.7 -> 11.2 /
-// 23.4 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 10.4 / 22.9 ms, 304 units
-// (two) 16.5 / 35.1 -> 13.4 / 26.6 ms.  Tried and slower: the next test's sums
+// kernel's semantics), against a warp per unit: 1 unit 17.5 / 37.7 -> 10.7 /
+// 22.6 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 9.9 / 22.2 ms, 304 units
+// (two) 16.5 / 35.1 -> 13.2 / 25.9 ms.  Tried and slower: the next test's sums
 // in the same exchange as the pressure (one barrier an iteration instead of
-// two, 12.2 against 11.5 ms: its arithmetic is then ahead of the barrier), and
-// two-wide fmas in the tail of the two-step update (11.5 against 11.3).
+// two, 12.2 against 11.5 ms: its arithmetic is then ahead of the barrier),
+// two-wide fmas in the two-step update (10.8 against 10.7), rounds of the sums
+// replaced by wider reads of them (10.9 to 13.2), and the next iteration's
+// predictor ahead of the step test's branch (11.9, with its right-hand side;
+// 11.7 without): the moves cost more than the vote's latency.
 //
 // The arithmetic is run_unit's (bm_step.cu) operation for operation, so the
 // results are the same bits; the sums over the sections keep its order.
@@ -286,14 +289,26 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
       // shared memory, and every warp adds the 64 of them in the order of the
       // butterfly over a whole warp of eight sections a lane.  Each round is
       // a shuffle (24 cycles) and an addition that nothing needs before the
-      // step test: the five rounds are spread over the iteration, where other
-      // work fills their latency.
+      // step test: the five rounds are spread over the iteration, one between
+      // two other shuffles or barriers each, where other work fills their
+      // latency.  (Next to each other in front of the solve they held it up:
+      // the warp issues in order.  11.2 / 23.4 -> 10.7 / 22.6 ms.)
       float2 sum = f2b(0.0f), sum_t;
       bool faulty = false;
       auto round = [&](int o) {
         sum_t = f2(__shfl_xor_sync(kFull, sum.x, o),
                    CTL == 0 ? __shfl_xor_sync(kFull, sum.y, o) : 0.0f);
         sum = add2(sum, sum_t);
+      };
+      // the places of a fast iteration in turn: between its two sweeps, after
+      // them, before and after the acceleration maximum, after the barrier
+      auto place = [&](int k) {
+        if (FIRST || SLOW) return;
+        if (k == 1) round(16);
+        if (k == (ARITH ? 1 : 2)) round(8);
+        if (k == (ARITH ? 2 : 3)) round(4);
+        if (k == (ARITH ? 3 : 4)) round(2);
+        if (k == (ARITH ? 4 : 5)) round(1);
       };
       if (!FIRST) {
         if (ARITH) {
@@ -323,24 +338,18 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
           const float4 q = *reinterpret_cast<const float4*>(&S.sum[2 * lane]);
           sum = f2(__fadd_rn(q.x, q.z), __fadd_rn(q.y, q.w));
         }
-        round(16);
-        if (SLOW) {
-          round(8);
-          round(4);
-          round(2);
-          round(1);
-        }
       }
 
       // two sweeps with one shuffle round: the first also on the two sections
       // next to the lane
-      auto sweep_pair = [&](float2 hA, float2 hB) {
+      auto sweep_pair = [&](float2 hA, float2 hB, bool only) {
         float2 T[2], q[2];
         const float2 Th = f2(__fadd_rn(hA.x, p[0].x), __fadd_rn(p[1].y, hB.y));
         const float2 qh = sweep(Th, rmh, Yrmh);
         neighbours(p, hA.y, hB.x, T);
         q[0] = sweep(T[0], rm[0], Yrm[0]);
         q[1] = sweep(T[1], rm[1], Yrm[1]);
+        if (only) place(1);
         neighbours(q, qh.x, qh.y, T);
         p[0] = sweep(T[0], rm[0], Yrm[0]);
         p[1] = sweep(T[1], rm[1], Yrm[1]);
@@ -354,9 +363,12 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
       };
       // two sweeps as one update over the second neighbours (bm_step.cu)
       auto two_step = [&](float2 hA, float2 hB) {
-        auto f2s = [](float2 a, float2 b, float2 c) { return f2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y)); };
-        const float2 r0 = f2s(K2[0], hA, fma2(K1[0], p[1], fma2(KB[0], p[0], C2[0])));
-        const float2 r1 = f2s(K2[1], p[0], f2s(K1[1], hB, fma2(KB[1], p[1], C2[1])));
+        // (scalar: an fma on three pairs of registers takes 3 cycles, two fmas 2.4)
+        auto f2s = [](float2 a, float2 b, float2 c) {
+          return f2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y));
+        };
+        const float2 r0 = f2s(K2[0], hA, f2s(K1[0], p[1], f2s(KB[0], p[0], C2[0])));
+        const float2 r1 = f2s(K2[1], p[0], f2s(K1[1], hB, f2s(KB[1], p[1], C2[1])));
         p[0] = r0;
         p[1] = r1;
       };
@@ -364,30 +376,37 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
         hA = f2(__shfl_sync(kFull, p[0].y, pa), __shfl_sync(kFull, p[0].x, pa));
         hB = f2(__shfl_xor_sync(kFull, p[1].y, 1), __shfl_xor_sync(kFull, p[1].x, 1));
       };
-      if (!FIRST && !SLOW) round(8);
+      const bool unrolled = SLOW && !ARITH && J == 20;
+      if (!FIRST && SLOW && !unrolled) {
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) round(o);
+      }
       float2 hA = pA, hB = pB;
       int it = 0;
-      if (SLOW && !ARITH && J == 20) {  // the reference schedule's slow count
+      if (unrolled) {  // the reference schedule's slow count
         two_step_setup();
         two_step(hA, hB);
 #pragma unroll
         for (int r = 1; r < 10; ++r) {
           halo(hA, hB);
+          if (!FIRST && r <= 5) round(32 >> r);
           two_step(hA, hB);
         }
         it = 20;
       } else if (!SLOW && J == 2) {  // and its fast count
-        sweep_pair(hA, hB);
+        sweep_pair(hA, hB, true);
         it = 2;
       } else if (!ARITH && J >= 4) {
+        place(1);
         two_step_setup();
         for (; it + 1 < J; it += 2) {
           two_step(hA, hB);
           halo(hA, hB);
         }
       } else {
+        place(1);
         for (; it + 1 < J; it += 2) {
-          sweep_pair(hA, hB);
+          sweep_pair(hA, hB, false);
           halo(hA, hB);
         }
       }
@@ -398,12 +417,12 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
         p[1] = sweep(T[1], rm[1], Yrm[1]);
       }
       n_sw += J;
+      place(2);
 
       // The pressure of the own sections and their acceleration maximum go to
       // shared memory together: one barrier, after which the halo takes its
       // owners' pressure.
       if (own) S.p[quad] = make_float4(p[0].x, p[0].y, p[1].x, p[1].y);
-      if (!FIRST && !SLOW) round(4);
       if (!FIRST) {
         float eap = 0.0f;
 #pragma unroll
@@ -411,15 +430,16 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
           const float2 da = abs2(sub2(a[k], mul2(add2(p[k], G[k]), invM[k])));
           eap = fmaxf(eap, fmaxf(da.x, da.y));
         }
+        place(3);
         const float eaw = warp_max_xor(own ? eap : 0.0f);
         if (lane == 0) S.ea[warp] = eaw;
       }
-      if (!FIRST && !SLOW) round(2);
+      place(4);
       __syncthreads();
       const float4 em = *reinterpret_cast<const float4*>(S.ea);
       const float p0 = S.p[8].x;  // section 0
       const float4 pq = S.p[quad];
-      if (!FIRST && !SLOW) round(1);
+      place(5);
 
       // Step test: the decision is voted on, which makes it uniform for the
       // compiler, before the rest of the iteration, which covers the vote.
