@@ -87,7 +87,9 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
   const bool inside = base >= 0 && base < 256;
   const bool own = lane >= 8 && lane < 24;
   const bool sec0 = base == 0, sec255 = base == 252;
-  const int pa = odd ? (lane + 1) & 31 : (lane + 31) & 31;  // the lane pair 0 faces
+  // the lane pair 0 faces; outside the unit the lane itself: its zeros stay zeros
+  // where the pressure at the ends is infinite
+  const int pa = !inside ? lane : odd ? (lane + 1) & 31 : (lane + 31) & 31;
   const cgb_unit un = A.units[blockIdx.x];
 
   auto load_row = [&](const float* row, float outside, float2 (&r)[2]) {

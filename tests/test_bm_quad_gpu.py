@@ -57,3 +57,26 @@ def test_both_sides_of_the_unit_rule(mv, bm_solver, controller, arith, extra):
     assert np.array_equal(ff[:whole * rows].reshape(whole, rows), np.broadcast_to(f, (whole, rows)))
     for k in ("substeps", "iterations", "sweeps", "failed_samples"):
         assert np.array_equal(ss[k], np.resize(st[k], n)), k
+
+
+@pytest.mark.parametrize("controller,arith", [(0, 0), (1, 0), (1, 1)])
+@pytest.mark.parametrize("value", [np.inf, 3e38])
+def test_infinite_pressure_at_the_ends(mv, bm_solver, controller, arith, value):
+    """An input that drives the pressure out of range: the sections outside a
+    unit stay zero in both kernels, so the iterations are the same too."""
+    import torch
+    sms = torch.cuda.get_device_properties(bm_solver.device).multi_processor_count
+    cfg, sc, gamma, units, x, rows = _case(mv, 0.5, 2, 20, 10, seed=7)
+    sc.controller, sc.arith = controller, arith
+    x = x.copy()
+    u = units[0]  # (a sample in the middle of a unit)
+    x[u["in_base"] + (u["start"] + u["end"]) // 2] = value
+    v, f, st = bm_solver.run(sc, gamma, units, x, rows)
+    assert not np.isfinite(v).all()
+    copies = -(-(2 * sms + 1) // len(units))
+    table = np.concatenate([units] * copies)
+    table["out_base"] += np.repeat(np.arange(copies), len(units)) * rows
+    vv, ff, ss = bm_solver.run(sc, gamma, table, x, rows * copies)
+    assert np.array_equal(vv[:rows], v, equal_nan=True) and np.array_equal(ff[:rows], f)
+    for k in ("substeps", "iterations", "sweeps", "failed_samples"):
+        assert np.array_equal(ss[k][:len(units)], st[k]), k
