@@ -48,6 +48,10 @@ __device__ __forceinline__ float2 fdividef2(float2 a, float2 b) {
   return f2(__fdividef(a.x, b.x), __fdividef(a.y, b.y));
 }
 
+// Sweeps of the reference schedule: of the first two iterations of a step, and of
+// the others.  Both kernels have instances that know these counts.
+constexpr int kSlowSweeps = 20, kFastSweeps = 2;
+
 // Launches the four-warps-per-unit kernel (fixed sweep counts); the status.
 int bm_quad_launch(const BMArgs& A, int controller, int arith, cudaStream_t st);
 // Most Jacobi sweeps of one solve that the four-warp kernel's halo carries.

@@ -23,9 +23,9 @@
 // rounds are spread over them; 1.4k warp instructions a substep, 3.4k cycles.
 //
 // Measured (GB300, 5 ms blocks with 1 ms overlap, kernel 17 / the default
-// kernel's semantics), against a warp per unit: 1 unit 17.5 / 37.7 -> 10.7 /
-// 22.6 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 9.9 / 22.2 ms, 304 units
-// (two) 16.5 / 35.1 -> 13.2 / 25.9 ms.  Tried and slower: the next test's sums
+// kernel's semantics), against a warp per unit: 1 unit 17.5 / 37.7 -> 10.0 /
+// 22.6 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 9.2 / 22.2 ms, 304 units
+// (two) 16.5 / 35.1 -> 12.5 / 25.9 ms.  Tried and slower: the next test's sums
 // in the same exchange as the pressure (one barrier an iteration instead of
 // two, 12.2 against 11.5 ms: its arithmetic is then ahead of the barrier),
 // two-wide fmas in the two-step update (10.8 against 10.7), rounds of the sums
@@ -78,7 +78,8 @@ struct __align__(16) QuadExchange {
   float ea[kQWarps]; // acceleration maxima of the warps' own sections
 };
 
-template <int CTL, int ARITH>
+// REF: the reference schedule's sweep counts, known to the compiler.
+template <int CTL, int ARITH, bool REF>
 __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
   __shared__ QuadExchange S2[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
       }
 
       // Jacobi sweeps inside the warp's window
-      const int J = SLOW ? A.jslow : A.jfast;
+      const int J = REF ? (SLOW ? kSlowSweeps : kFastSweeps) : (SLOW ? A.jslow : A.jfast);
       const float2 Yrmh =
           f2(__shfl_sync(kFull, Yrm[0].x, pa), __shfl_xor_sync(kFull, Yrm[1].y, 1));
       // Velocity error and margin: the lanes' sums of four sections go to
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
         hA = f2(__shfl_sync(kFull, p[0].y, pa), __shfl_sync(kFull, p[0].x, pa));
         hB = f2(__shfl_xor_sync(kFull, p[1].y, 1), __shfl_xor_sync(kFull, p[1].x, 1));
       };
-      const bool unrolled = SLOW && !ARITH && J == 20;
+      const bool unrolled = SLOW && !ARITH && J == kSlowSweeps;
       if (!FIRST && SLOW && !unrolled) {
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) round(o);
@@ -389,15 +390,15 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
         two_step_setup();
         two_step(hA, hB);
 #pragma unroll
-        for (int r = 1; r < 10; ++r) {
+        for (int r = 1; r < kSlowSweeps / 2; ++r) {
           halo(hA, hB);
           if (!FIRST && r <= 5) round(32 >> r);
           two_step(hA, hB);
         }
-        it = 20;
-      } else if (!SLOW && J == 2) {  // and its fast count
+        it = kSlowSweeps;
+      } else if (!SLOW && J == kFastSweeps) {  // and its fast count
         sweep_pair(hA, hB, true);
-        it = 2;
+        it = kFastSweeps;
       } else if (!ARITH && J >= 4) {
         place(1);
         two_step_setup();
@@ -565,12 +566,19 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
 
 int bm_quad_launch(const BMArgs& A, int controller, int arith, cudaStream_t st) {
   const unsigned grid = (unsigned)A.n_units;
+  // The reference schedule's sweep counts compiled in: 1 unit 10.7 -> 10.0 ms
+  // (kernel 17); no gain for the reference's order.
+  const bool schedule = A.jslow == kSlowSweeps && A.jfast == kFastSweeps;
   if (arith)
-    bm_quad_kernel<1, 1><<<grid, kQThreads, 0, st>>>(A);
+    bm_quad_kernel<1, 1, false><<<grid, kQThreads, 0, st>>>(A);
+  else if (controller == 1 && schedule)
+    bm_quad_kernel<1, 0, true><<<grid, kQThreads, 0, st>>>(A);
   else if (controller == 1)
-    bm_quad_kernel<1, 0><<<grid, kQThreads, 0, st>>>(A);
+    bm_quad_kernel<1, 0, false><<<grid, kQThreads, 0, st>>>(A);
+  else if (schedule)
+    bm_quad_kernel<0, 0, true><<<grid, kQThreads, 0, st>>>(A);
   else
-    bm_quad_kernel<0, 0><<<grid, kQThreads, 0, st>>>(A);
+    bm_quad_kernel<0, 0, false><<<grid, kQThreads, 0, st>>>(A);
   CGB_TRY_CUDA(cudaGetLastError(), "bm_quad_kernel launch");
   note_launch();
   return CGB_OK;

@@ -39,14 +39,15 @@ def test_sweep_counts_against_oracle(mv, bm_solver, controller, fast, slow, max_
 @pytest.mark.parametrize("extra", [0, 1])
 def test_both_sides_of_the_unit_rule(mv, bm_solver, controller, arith, extra):
     """The same units once alone and once in a table just at (extra 0) or just
-    past (extra 1: the warp-per-unit kernel) the most units of the rule."""
+    past (extra 1: the warp-per-unit kernel) the most units of the rule: one an
+    SM for controller 0, two for controller 1."""
     import torch
     sms = torch.cuda.get_device_properties(bm_solver.device).multi_processor_count
     cfg, sc, gamma, units, x, rows = _case(mv, 0.5, 2, 20, 10, seed=5)
     sc.controller, sc.arith = controller, arith
     v, f, st = bm_solver.run(sc, gamma, units, x, rows)
     assert np.abs(v).max() > 0
-    n = 2 * sms + extra
+    n = (2 if controller else 1) * sms + extra
     copies = -(-n // len(units))
     table = np.concatenate([units] * copies)[:n].copy()
     table["out_base"] += np.repeat(np.arange(copies), len(units))[:n] * rows
