@@ -25,17 +25,16 @@
 // products as soon as a half is there.  Between the digits the same warps finish
 // the tile before: its Dot2 points, the DC sums, IHC and lambda.
 //
-// What bounds it now: the workers' chain, ~56k cycles a tile (Dot2 points 11k, DC
+// What bounds it now: the workers' chain, ~52k cycles a tile (Dot2 points 7k, DC
 // sums 11k, IHC / lambda 7k, loads 7k, digits 10k, epilogue 4k) at 41% of the
 // issue slots, not the tensor pipe.  Finishing a tile at once instead of between
 // the next one's digits takes 22.0 ms against 18.9 (JND sweep); without the products
-// (accumulators left as they are) the chain takes the same time.  The taps left over
-// by a point's batches of eight in batches of four and one, not one by one with a
-// choice of register each: 18.9 -> 18.65 ms.  DC sums whose errors run a batch
-// behind, or on two blocks at once: 19.5 and 19.6.
+// (accumulators left as they are) the chain takes the same time.  Single points by
+// a warp whose lanes share the work (sym_point): 18.65 -> 17.5 ms.  DC sums whose
+// errors run a batch behind, or on two blocks at once: 19.5 and 19.6 against 18.65.
 //
 // Measured (GB300), against the FP32 pipe: JND sweep (2.9 million rows) 53.7 ->
-// 18.3 ms, 176,000 rows in 33 intervals 4.46 -> 1.52 ms, one signal of 5,330 rows
+// 17.5 ms, 176,000 rows in 33 intervals 4.46 -> 1.43 ms, one signal of 5,330 rows
 // 0.80 -> 0.28 ms.
 
 #include <cuda_runtime.h>
@@ -65,6 +64,13 @@ constexpr int kList = 1024;                // points for Dot2 listed by tile
 constexpr int kFewPoints = 48;             // up to here a warp to a point
 constexpr int kRuns = 16;                  // runs of 24 rows of a tile's x
 
+// A warp's scratch for one point (sym_point).
+constexpr int kPairs = tfir::kMaxTaps / 2;
+struct __align__(16) PointScratch {
+  float p[kPairs];   // products; then the running sums; then the errors
+  float ep[kPairs];  // errors of the pairs' sums
+};
+
 struct TensorShared {
   uint64_t mbar[2];          // products of half h are done
   uint32_t tmem;
@@ -79,7 +85,11 @@ struct TensorShared {
   uint32_t partial[kCols];   // bits of the largest partial sum of the sampled rows
   // of the first and last row's sum over each run of 24 rows of x: the sum and
   // its largest partial sum
-  float2 sample[2][kRuns][kCols];
+  // (each warp's scratch when single points are evaluated, after their use)
+  union {
+    alignas(16) float2 sample[2][kRuns][kCols];
+    PointScratch point[kIhcWarps];
+  };
   uint16_t list[kList];
   unsigned char row[tfir::kRows];  // how the tile's row gets its AC: kRow...
 };
@@ -189,17 +199,111 @@ __device__ __forceinline__ int lane_taps(Dot2& acc, float b, float u, int q) {
   dot2_taps(acc, gb, gu);
   return N;
 }
-template <int N>
-__device__ __forceinline__ int lane_pairs(Dot2& acc, float b, float u, float w, int q) {
-  float gb[N], gu[N], gw[N];
+// Dot2 of a point with all taps of a symmetric filter (fir_row_sym's order), by a
+// warp: what is no chain by a lane per tap pair (rows and taps fetched at once, the
+// pair's sum and product with their errors, later the error of its addition), and
+// the chain of the rounded sums and then that of the errors by all lanes alike, from
+// shared memory.  A pair costs 5 instructions and 12 cycles of a chain; all lanes
+// doing all of it from shuffled values took 23 and 33.  The value of the point's own
+// row in lane 0.
+__device__ __forceinline__ float sym_point(Dot2& acc, const float* __restrict__ src,
+                                           const float* TP, int n, PointScratch& W, int lane) {
+  constexpr int kPer = kPairs / 32;
+  const int half = n / 2;
+  float p[kPer], q[kPer], own;
+  {
+    float x1[kPer], x2[kPer];
 #pragma unroll
-  for (int e = 0; e < N; ++e) {
-    gb[e] = __shfl_sync(kFull, b, q + e);
-    gu[e] = __shfl_sync(kFull, u, q + e);
-    gw[e] = __shfl_sync(kFull, w, q + e);
+    for (int i = 0; i < kPer; ++i) {
+      const int k = lane + 32 * i;
+      x1[i] = k < half ? __ldg(src - k * 256) : 0.0f;
+      x2[i] = k < half ? __ldg(src - (n - 1 - k) * 256) : 0.0f;
+    }
+    own = x1[0];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int k = lane + 32 * i;
+      const float b = k < half ? TP[k] : 0.0f;
+      const float sg = __fadd_rn(x1[i], x2[i]);
+      const float zz = __fsub_rn(sg, x1[i]);
+      p[i] = __fmul_rn(b, sg);
+      q[i] = __fmaf_rn(b, sg, -p[i]);
+      W.p[k] = p[i];
+      W.ep[k] = __fadd_rn(__fsub_rn(x1[i], __fsub_rn(sg, zz)), __fsub_rn(x2[i], zz));
+    }
   }
-  dot2_pairs(acc, gb, gu, gw);
-  return N;
+  __syncwarp();
+  float t = acc.s;
+#pragma unroll 1
+  for (int k = 0; k < half; k += 16) {
+    float4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(&W.p[k + 4 * j]);
+    if (k + 16 <= half) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[j].x = t = __fadd_rn(t, v[j].x);
+        v[j].y = t = __fadd_rn(t, v[j].y);
+        v[j].z = t = __fadd_rn(t, v[j].z);
+        v[j].w = t = __fadd_rn(t, v[j].w);
+      }
+    } else {
+      const int left = half - k;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[j].x = t = 4 * j < left ? __fadd_rn(t, v[j].x) : t;
+        v[j].y = t = 4 * j + 1 < left ? __fadd_rn(t, v[j].y) : t;
+        v[j].z = t = 4 * j + 2 < left ? __fadd_rn(t, v[j].z) : t;
+        v[j].w = t = 4 * j + 3 < left ? __fadd_rn(t, v[j].w) : t;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&W.p[k + 4 * j]) = v[j];
+    }
+  }
+  __syncwarp();
+  float g[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int k = lane + 32 * i;
+    const float to = W.p[k], a = k ? W.p[k - 1] : acc.s;
+    const float z = __fsub_rn(to, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(to, z)), __fsub_rn(p[i], z));
+    g[i] = __fadd_rn(e, q[i]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) W.p[lane + 32 * i] = g[i];
+  __syncwarp();
+  float c = acc.c;
+  int k = 0;
+#pragma unroll 1
+  for (; k + 8 <= half; k += 8) {
+    float b[8];
+    float4 g4[2], e4[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      g4[j] = *reinterpret_cast<const float4*>(&W.p[k + 4 * j]);
+      e4[j] = *reinterpret_cast<const float4*>(&W.ep[k + 4 * j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b[j] = TP[k + j];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      c = __fmaf_rn(b[4 * j], e4[j].x, __fadd_rn(c, g4[j].x));
+      c = __fmaf_rn(b[4 * j + 1], e4[j].y, __fadd_rn(c, g4[j].y));
+      c = __fmaf_rn(b[4 * j + 2], e4[j].z, __fadd_rn(c, g4[j].z));
+      c = __fmaf_rn(b[4 * j + 3], e4[j].w, __fadd_rn(c, g4[j].w));
+    }
+  }
+  for (; k < half; ++k) c = __fmaf_rn(TP[k], W.ep[k], __fadd_rn(c, W.p[k]));
+  __syncwarp();  // (the scratch is free)
+  acc.s = t;
+  acc.c = c;
+  if (n & 1) acc.add(TP[half], __ldg(src - half * 256));
+  return own;
 }
 
 // Dot2 of one output in the orders of ihc_lambda.cu (fir_row, fir_row_sym),
@@ -527,53 +631,28 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int listed = S.listed, kb = t * tfir::kRows;
       const bool all = listed > kList;
       if (listed <= kFewPoints) {
-        // Few points: a warp to each.  Its lanes fetch the point's rows and the
+        // Few points: a warp to each, whose lanes fetch the point's rows and the
         // taps at once (one trip to L2 where a lane's own sequence of batches
-        // takes sixteen) and hand them round by shuffles, which do not wait for
-        // the shared memory that the products are reading.
+        // takes sixteen).
         for (int p = warp; p < listed; p += kIhcWarps) {
           const int r = S.list[p] / kCols, c = S.list[p] % kCols;
           const float* src = vf + (int64_t)(kb + r) * 256 + c;
           const int taps = taps_used(kb + r, f, n_ac);
-          const bool sym = A.ac_sym && taps == n_ac;
-          const int half = n_ac / 2;
-          // lane + 32 i: the row of that tap, and of its mirror tap
-          float u[9], w[4], b[9];
-#pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            const int k = lane + 32 * i;
-            u[i] = k < taps ? __ldg(src - k * 256) : 0.0f;
-            b[i] = k < n_ac ? TP[k] : 0.0f;
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int k = lane + 32 * i;
-            w[i] = sym && k < half ? __ldg(src - (n_ac - 1 - k) * 256) : 0.0f;
-          }
           Dot2 acc;
           acc.init();
-          // the value of lane q of the i-th register of v (i, q uniform)
-          auto from = [&](const float (&v)[9], int k) {
-            float r = v[0];
-#pragma unroll
-            for (int i = 1; i < 9; ++i) r = k >> 5 == i ? v[i] : r;
-            return __shfl_sync(kFull, r, k & 31);
-          };
-          if (sym) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll 1
-              for (int q = 0; q < 32 && 32 * i + q < half;) {
-                const int left = half - 32 * i - q;
-                if (left >= 8)
-                  q += lane_pairs<8>(acc, b[i], u[i], w[i], q);
-                else if (left >= 4)
-                  q += lane_pairs<4>(acc, b[i], u[i], w[i], q);
-                else
-                  q += lane_pairs<1>(acc, b[i], u[i], w[i], q);
-              }
-            if (n_ac & 1) acc.add(from(b, half), from(u, half));
+          float own;  // lane 0: the point's own row
+          if (A.ac_sym && taps == n_ac) {
+            own = sym_point(acc, src, TP, n_ac, S.point[warp], lane);
           } else {
+            // lane + 32 i: the row of that tap
+            float u[9], b[9];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+              const int k = lane + 32 * i;
+              u[i] = k < taps ? __ldg(src - k * 256) : 0.0f;
+              b[i] = k < n_ac ? TP[k] : 0.0f;
+            }
+            own = u[0];
 #pragma unroll
             for (int i = 0; i < 9; ++i)
 #pragma unroll 1
@@ -588,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
           }
           const float ac = acc.result();
-          const float ms = __fmaf_rn(u[0], A.scale, -ac);  // (lane 0's is the point's own)
+          const float ms = __fmaf_rn(own, A.scale, -ac);
           int slot = at + r;
           slot -= slot >= ring ? ring : 0;
           if (lane == 0) {
