@@ -17,7 +17,11 @@
 // 40 x 2^-48 of that bound, about twice the partial sum itself; where it makes a
 // difference, and in rows whose look-back is shorter than the tile's, the point
 // is evaluated by Dot2.  On the JND sweep 39% of the tiles have no such point,
-// 48% one to eight of 8,192.
+// 48% one to eight of 8,192.  Not below a floor, what the five digits leave of x and
+// of the taps (six standard deviations, from the taps): it decides where a section's
+// sums are tiny beside its largest |x|, as at the start of a segment, whose velocity
+// grows from nothing by orders of magnitude within a tile; up to 6,000 of its points
+// go to Dot2.
 //
 // One CTA: 64 sections x a run of tiles of one frame.  Sixteen warps hold the
 // tile's 384 rows of velocity in registers (48 values a thread) and write one
@@ -32,10 +36,12 @@
 // (accumulators left as they are) the chain takes the same time.  Single points by
 // a warp whose lanes share the work (sym_point): 18.65 -> 17.5 ms.  DC sums whose
 // errors run a batch behind, or on two blocks at once: 19.5 and 19.6 against 18.65.
+// Where there are too many points for the list, a bit each says which, instead of all
+// rows of the tile: one signal 304 -> 262 us, 33 intervals 1.46 -> 1.44 ms.
 //
 // Measured (GB300), against the FP32 pipe: JND sweep (2.9 million rows) 53.7 ->
-// 17.5 ms, 176,000 rows in 33 intervals 4.46 -> 1.43 ms, one signal of 5,330 rows
-// 0.80 -> 0.28 ms.
+// 17.8 ms, 176,000 rows in 33 intervals 4.46 -> 1.44 ms, one signal of 5,330 rows
+// 0.80 -> 0.26 ms.
 
 #include <cuda_runtime.h>
 
@@ -76,7 +82,8 @@ struct TensorShared {
   uint32_t tmem;
   int abort;                 // a wait ran out
   int stop;                  // the workers have ended the run early
-  int listed;                // points for Dot2 (more than kList: all of the tile)
+  float floor;               // least slack, in units of the accumulators
+  int listed;                // points for Dot2 (more than kList: those flagged)
   int dot2_rows[2];          // rows for Dot2, by tile parity
   int kmin[2];               // first row of x of the tile, by tile parity
   uint32_t top[2][kCols];    // largest |x| bits of the tile, by tile parity
@@ -91,6 +98,7 @@ struct TensorShared {
     PointScratch point[kIhcWarps];
   };
   uint16_t list[kList];
+  alignas(4) unsigned char flag[tfir::kRows][kCols / 8];  // the points for Dot2, a bit each
   unsigned char row[tfir::kRows];  // how the tile's row gets its AC: kRow...
 };
 static_assert(offsetof(TensorShared, mbar) % 8 == 0 && offsetof(TensorShared, scale) % 16 == 0 &&
@@ -466,6 +474,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
   __syncthreads();
+  if (warp == kIhcWarps) {
+    // The remainders of x behind its last digit, at most 2^(e-45) and 2^(e-45.8) rms,
+    // times the taps: six standard deviations of their sum.
+    float sq = 0.0f;
+    for (int i = lane; i < n_ac; i += 32) sq += TP[i] * TP[i];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(kFull, sq, o);
+    if (lane == 0) S.floor = 0x1p-27f * sqrtf(sq) * __int_as_float((127 - exp_b) << 23);
+  }
   for (int e = threadIdx.x; e < tfir::kDigits * tfir::kCores * 64; e += kThreads) {
     const int j = e / (tfir::kCores * 64), q = e - j * (tfir::kCores * 64);
     const int i = 8 * (q >> 6) + ((q >> 3) & 7) + (q & 7) - (tfir::kRows - 1);
@@ -676,7 +693,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      // first the rows that the products cannot give, a warp to 32 sections;
+      // first the rows that the products cannot give, and of more points than the
+      // list holds the rows with any, a warp to 32 sections;
       // then single points, as few warps as hold them (what a warp's sequence
       // costs does not depend on its lanes), from the highest warp down
       int row = all || S.dot2_rows[t & 1] ? gw : tfir::kRows;
@@ -684,11 +702,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       while (true) {
         int r, c;
         if (row < tfir::kRows) {
-          const int kind = S.row[row];
+          // of too many points for the list: the row's, as flagged
+          uint32_t points = all ? *reinterpret_cast<const uint32_t*>(&S.flag[row][4 * sg]) : 0;
+          if (S.row[row] == kRowDot2) points = ~0u;
           r = row;
           c = sec;
           row += 8;
-          if (!(kind == kRowDot2 || (all && kind == kRowSum))) continue;
+          if (!(points >> lane & 1)) continue;
         } else {
           if (all || listed <= kFewPoints || p >= listed) break;
           r = S.list[p] / kCols;
@@ -862,7 +882,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool usable = e >= -80 && e <= 100;
       if (warp < kGroups && gw == 0) {
         S.scale[sec] =
-            make_float2(m == 0 ? 0.0f : (usable ? 0x1p-31f : __int_as_float(0x7f800000)),
+            make_float2(m == 0 ? 0.0f : (usable ? S.floor : __int_as_float(0x7f800000)),
                         usable ? __int_as_float((127 + e + exp_b - 16) << 23) : 1.0f);
         S.top[(t + 1) & 1][sec] = 0;
       }
@@ -964,7 +984,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             DS[slot * kPitch + c0 + c] = ds.x;
             DS[slot * kPitch + c0 + c + 1] = ds.y;
           }
-          if (kind == kRowSum && bad) {
+          if (kind != kRowSum) bad = 0;
+          S.flag[row][c0 >> 3] = (unsigned char)bad;
+          if (bad) {
             int p = atomicAdd(&S.listed, __popc(bad));
 #pragma unroll
             for (int c = 0; c < 8; ++c)

@@ -10,8 +10,9 @@
 // up to 256 are exact in BF16, and the products of two digits summed over the
 // taps stay below 2^24, so the FP32 accumulators hold exact integers.  The 19
 // digit pairs with i + j <= 5 go to six accumulators G_m, m = i + j:
-//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  an error of about 2^-50 of the
-// product of the two scales (2^-41 with the 15 pairs up to i + j = 4).
+//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  the digits' remainders (at most 2^(e-45)
+// of a value of x, 2^(eb-45) of a tap) and the pairs left out (about 2^-50 of the
+// product of the scales; 2^-41 with the 15 pairs up to i + j = 4).
 //
 // T has one value per diagonal.  With the rows of x stored in reverse order its
 // band is a Hankel matrix (element (r, k') depends on r + k'), and a Hankel

@@ -96,3 +96,14 @@ def test_infinities_and_nan():
     v = _velocity("tones")
     v[400, 3], v[500, 100], v[450, 200] = np.inf, np.nan, 3e38
     _check(_stage(), v, [(0, 0, 1100, 1100, 1100, 1100, 1152, 0)])
+
+
+@pytest.mark.parametrize("seg", [1100, 300])
+@pytest.mark.parametrize("decades", [6, 12])
+def test_onsets(seg, decades):
+    """Velocity that grows from nothing by many orders of magnitude within a
+    segment's first tiles, as a solved one does: more points below the digits'
+    resolution than the list holds, beside rows that the products do give."""
+    rise = np.minimum((np.arange(ROWS) % seg) / 150.0, 1.0)[:, None] - 1.0
+    v = _velocity("tones") * 10.0 ** (decades * rise * (np.arange(256)[None, :] / 255))
+    _check(_stage(), v.astype(np.float32), [(0, 0, 1100, 1100, seg, 1100, 1152, 0)])
