@@ -54,7 +54,8 @@ constexpr int kOffSecond = kOffFirst + kW1Bytes, kOffThird = kOffSecond + kWByte
 constexpr int kOffLast = kOffThird + kWBytes, kOffBiases = kOffLast + kW4Size;
 constexpr int kOffFwdShared = kOffBiases + kBiasFloats * 4;
 constexpr int kOffBwdShared = kOffLast;
-constexpr int kFwdBytes = kOffFwdShared + (int)sizeof(TensorShared);
+constexpr int kOffSquares = kOffFwdShared + (int)sizeof(TensorShared);
+constexpr int kFwdBytes = kOffSquares + kNS * 8;
 constexpr int kBwdBytes = kOffBwdShared + (int)sizeof(TensorShared);
 static_assert(kActRows * 16 <= kFeatBytes && kOffFwdShared % 16 == 0 && kOffBwdShared % 16 == 0 &&
                   kFwdBytes <= 227 * 1024,
@@ -171,9 +172,13 @@ __device__ __forceinline__ uint32_t begin(unsigned char* sm, TensorShared& S, in
   return __shfl_sync(kFull, S.tmem, 0);
 }
 
+// LOSS: the loss kernel's work too (warmstart.cu), 4 us of launch and latency less.
+template <bool LOSS>
 __global__ void __launch_bounds__(kConvThreads, 1)
     forward_kernel(const unsigned char* __restrict__ blob, const unsigned char* __restrict__ feat,
-                   int n, unsigned char* __restrict__ hid, float* __restrict__ out) {
+                   int n, unsigned char* __restrict__ hid, float* __restrict__ out,
+                   const float* __restrict__ target, float s_out,
+                   unsigned char* __restrict__ dout, double* __restrict__ loss_part) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + kOffFwdShared);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -255,8 +260,30 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         float v[8];
         tfir::tmem_load8(mine.tmem, v);
         tfir::tmem_wait_loads();
-        out[(int64_t)rec * kNS + mine.pos] =
+        const float o =
             *(volatile int*)&S.failed ? __int_as_float(0x7fffffff) : v[0] + bias[192];
+        out[(int64_t)rec * kNS + mine.pos] = o;
+        if (LOSS) {
+          double* red = reinterpret_cast<double*>(sm + kOffSquares);
+          const float e = s_out * o - target[(int64_t)rec * kNS + mine.pos];
+          const float gsc = 2.0f * s_out / ((float)n * 256.0f);
+          reinterpret_cast<uint4*>(dout)[(int64_t)rec * kNS + mine.pos] =
+              make_uint4(bf16_bits(gsc * e), 0, 0, 0);
+          red[mine.pos] = (double)e * (double)e;
+          // (warps 0 to 7; the next record's squares come after barriers of all)
+          asm volatile("bar.sync 3, %0;" ::"n"(kNS) : "memory");
+          if (warp == 0) {
+            double r[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = red[lane + 32 * i] + red[lane + 32 * i + 128];
+            r[0] += r[2];
+            r[1] += r[3];
+            r[0] += r[1];
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) r[0] += __shfl_down_sync(kFull, r[0], o);
+            if (lane == 0) loss_part[rec] = r[0];
+          }
+        }
       }
     }
     tfir::fence_before();
@@ -370,22 +397,43 @@ int conv_grid(int n, int* grid) {
 using namespace cgb;
 using namespace cgb::ws;
 
+template <bool LOSS>
+static int launch_forward(const void* d_blob, const void* d_feat, int n, void* d_hid, float* d_out,
+                          const float* d_target, float s_out, void* d_dout, double* d_loss_part,
+                          void* stream) {
+  int grid = 0;
+  if (const int rc = conv_grid(n, &grid)) return rc;
+  CGB_TRY_CUDA(cudaFuncSetAttribute(forward_kernel<LOSS>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdBytes),
+               "cudaFuncSetAttribute(forward)");
+  forward_kernel<LOSS><<<grid, kConvThreads, kFwdBytes, reinterpret_cast<cudaStream_t>(stream)>>>(
+      static_cast<const unsigned char*>(d_blob), static_cast<const unsigned char*>(d_feat), n,
+      static_cast<unsigned char*>(d_hid), d_out, d_target, s_out,
+      static_cast<unsigned char*>(d_dout), d_loss_part);
+  CGB_TRY_CUDA(cudaGetLastError(), "forward_kernel launch");
+  note_launch();
+  return CGB_OK;
+}
+
 extern "C" int cgb_ws_forward_dev(const void* d_blob, const void* d_feat, int n, void* d_hid,
                                   float* d_out, void* stream) {
   if (n == 0) return CGB_OK;
   if (n < 0 || !d_blob || !d_feat || !d_hid || !d_out)
     return fail(CGB_ERR_ARG, "cgb_ws_forward_dev: bad arguments");
-  int grid = 0;
-  if (const int rc = conv_grid(n, &grid)) return rc;
-  CGB_TRY_CUDA(cudaFuncSetAttribute(forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kFwdBytes),
-               "cudaFuncSetAttribute(forward)");
-  forward_kernel<<<grid, kConvThreads, kFwdBytes, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const unsigned char*>(d_blob), static_cast<const unsigned char*>(d_feat), n,
-      static_cast<unsigned char*>(d_hid), d_out);
-  CGB_TRY_CUDA(cudaGetLastError(), "forward_kernel launch");
-  note_launch();
-  return CGB_OK;
+  return launch_forward<false>(d_blob, d_feat, n, d_hid, d_out, nullptr, 0.0f, nullptr, nullptr,
+                               stream);
+}
+
+int cgb::ws::forward_loss(const void* d_blob, const void* d_feat, int n, void* d_hid, float* d_out,
+                          const float* d_target, float s_out, void* d_dout, double* d_loss_part,
+                          void* stream) {
+  if (n == 0) return CGB_OK;
+  if (n < 0 || !d_blob || !d_feat || !d_hid || !d_out)
+    return fail(CGB_ERR_ARG, "cgb_ws_forward_dev: bad arguments");
+  if (!d_target || !d_dout || !d_loss_part)
+    return fail(CGB_ERR_ARG, "cgb_ws_loss_dev: bad arguments");
+  return launch_forward<true>(d_blob, d_feat, n, d_hid, d_out, d_target, s_out, d_dout, d_loss_part,
+                              stream);
 }
 
 extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, const void* d_hid,

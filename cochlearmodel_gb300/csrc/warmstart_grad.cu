@@ -366,8 +366,8 @@ extern "C" int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, con
                                     float* d_partial, int n_parts, double* d_loss, float* d_grad,
                                     void* stream) {
   if (!d_loss) return fail(CGB_ERR_ARG, "cgb_ws_gradients_dev: bad arguments");
-  if (const int rc = cgb_ws_forward_dev(d_blob, d_feat, n, d_hid, d_out, stream)) return rc;
-  if (const int rc = cgb_ws_loss_dev(d_out, d_target, n, s_out, d_dout, d_loss_part, stream))
+  if (const int rc = forward_loss(d_blob, d_feat, n, d_hid, d_out, d_target, s_out, d_dout,
+                                  d_loss_part, stream))
     return rc;
   if (const int rc = cgb_ws_backward_dev(d_blobT, d_dout, d_hid, n, d_dpre, stream)) return rc;
   return launch_wgrad(d_feat, d_hid, d_dpre, d_dout, n, d_partial, n_parts, d_grad, d_loss_part,

@@ -8,6 +8,11 @@
 namespace cgb {
 namespace ws {
 
+// cgb_ws_forward_dev and cgb_ws_loss_dev in one kernel (warmstart_conv.cu).
+int forward_loss(const void* d_blob, const void* d_feat, int n, void* d_hid, float* d_out,
+                 const float* d_target, float s_out, void* d_dout, double* d_loss_part,
+                 void* stream);
+
 struct TensorShared {
   uint64_t mbar[2];  // the products of stage (or tile) h are done
   uint32_t tmem;
