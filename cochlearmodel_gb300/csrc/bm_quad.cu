@@ -24,8 +24,8 @@
 //
 // Measured (GB300, 5 ms blocks with 1 ms overlap, kernel 17 / the default
 // kernel's semantics), against a warp per unit: 1 unit 17.5 / 37.7 -> 10.0 /
-// 22.6 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 9.2 / 22.2 ms, 304 units
-// (two) 16.5 / 35.1 -> 12.5 / 25.9 ms.  Tried and slower: the next test's sums
+// 22.2 ms, 152 units (one CTA per SM) 16.7 / 37.8 -> 9.2 / 21.7 ms, 304 units
+// (two) 16.5 / 35.1 -> 11.9 / 25.4 ms.  Tried and slower: the next test's sums
 // in the same exchange as the pressure (one barrier an iteration instead of
 // two, 12.2 against 11.5 ms: its arithmetic is then ahead of the barrier),
 // two-wide fmas in the two-step update (10.8 against 10.7), rounds of the sums
@@ -204,7 +204,9 @@ __global__ void __launch_bounds__(kQThreads, 2) bm_quad_kernel(const BMArgs A) {
     }
     // known before the step, so that their latency passes under it
     const bool emit = __all_sync(kFull, tau_f > A.tout_f);
-    const bool owned_row = __all_sync(kFull, n >= un.out_first);
+    // (n is the same in all lanes; the vote that tells the compiler so pays in the own
+    // order, 10.0 against 10.2 ms, and costs in the reference's, 22.6 against 22.2)
+    const bool owned_row = ARITH ? n >= un.out_first : __all_sync(kFull, n >= un.out_first);
     const float delta = __fmul_rn(tau_f, A.fs_f);
     const float smp = __fmaf_rn(sx1, delta, __fmul_rn(sx0, __fsub_rn(1.0f, delta)));
     const float hdt = __fmul_rn(dt, 0.5f);

@@ -973,9 +973,9 @@ int g_shape = 0;
 // Tables of up to this many units per SM run on four warps per unit
 // (bm_quad.cu).  Kernel 17's controller, 5 ms blocks: up to one unit an SM 9.2 ms
 // against 11.8 with a warp per unit, which takes that long up to four units an SM;
-// two CTAs an SM take 12.5.  (Other sweep counts, 18 and 2: 11.0 against 14.6, 15.1
+// two CTAs an SM take 11.9 to 12.5.  (Other sweep counts, 18 and 2: 11.0 against 14.6, 15.1
 // at two.)  BMOHC_NEW_kernel's controller, with more iterations of two sweeps: at
-// two units an SM 25.8 ms against 30.0, in the own order 36.5 against 39.5.
+// two units an SM 25.4 ms against 30.0, in the own order 36.5 against 39.5.
 int quad_units_per_sm(int controller) { return controller == 0 ? 1 : 2; }
 
 }  // namespace cgb
