@@ -645,6 +645,10 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
         run = it->second.run;
         tensor = it->second.tensor;
         exp_b = it->second.exp_b;
+        // the tensor kernel's buffers are for the lengths that it was chosen for
+        if (tensor && (!ihc_tensor_fits(n_ac, n_dc) || ac_ext || stage != 0))
+          return fail(CGB_ERR_ARG,
+                      "cgb_ihc_lambda_launch_dev: not the filters that were uploaded");
       }
     }
   }

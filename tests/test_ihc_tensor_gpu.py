@@ -4,7 +4,7 @@ tiles, segments and filter lengths and on inputs that make its scales fail."""
 import numpy as np
 import pytest
 
-from cochlearmodel_gb300 import ihc
+from cochlearmodel_gb300 import ihc, native
 from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -107,3 +107,17 @@ def test_onsets(seg, decades):
     rise = np.minimum((np.arange(ROWS) % seg) / 150.0, 1.0)[:, None] - 1.0
     v = _velocity("tones") * 10.0 ** (decades * rise * (np.arange(256)[None, :] / 255))
     _check(_stage(), v.astype(np.float32), [(0, 0, 1100, 1100, seg, 1100, 1152, 0)])
+
+
+def test_launch_of_other_filters_than_uploaded():
+    """A launch on tables that were uploaded for another filter, longer than the
+    kernel's: an error, and no launch."""
+    import torch
+    stage = _stage()
+    fr = np.array([(0, 0, 512, 512, 512, 512, 512, 0)], ihc.FRAME_DTYPE)
+    chunk, = stage.upload_chunks([fr], 512, 512)
+    v = torch.zeros((512, 256), device="cuda:0")
+    lam = torch.zeros((3, 512, 256), device="cuda:0")
+    stage.ac = _taps(300)
+    with pytest.raises(native.CGBError, match="not the filters that were uploaded"):
+        stage.launch_chunk(v, chunk, lam, torch.cuda.current_stream())
