@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   for (int i = tid; i < 5 * 8 * 8; i += kConvThreads)  // outputs 8 .. 15
     fill_zero(sm + kOffLast + (i >> 3) * kW4Chunk + (8 + (i & 7)) * 16);
   const uint32_t tmem = begin(sm, S, tid, warp);
+  release_next();
 
   if (warp == kFinishers / 32) {
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
@@ -296,8 +297,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // dH1 = (W2^T * dH2) . [H1 > 0], with the transposed, tap-reversed weights.
 __global__ void __launch_bounds__(kConvThreads, 1)
     backward_kernel(const unsigned char* __restrict__ blobT,
-                    const unsigned char* __restrict__ dout, const unsigned char* __restrict__ hid,
-                    int n, unsigned char* __restrict__ dpre) {
+                    const unsigned char* dout, const unsigned char* hid, int n,
+                    unsigned char* dpre) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + kOffBwdShared);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -308,6 +309,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   stage_weights(sm + kOffThird, blobT + kOffT2, 64, kWChunk, kWTap, tid);
   if (tid < kActRows - kNS) fill_zero(sm + kOffIn + (tid < 2 ? tid : kNS + tid) * 16);
   const uint32_t tmem = begin(sm, S, tid, warp);
+  release_next();
+  wait_previous(dout, hid);
 
   if (warp == kFinishers / 32) {
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
@@ -324,14 +327,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     int phase = 0;
     uint4 next = make_uint4(0, 0, 0, 0), mask[4];
     auto load = [&](int rec) {
-      if (tid < kNS) next = __ldg(reinterpret_cast<const uint4*>(dout) + (int64_t)rec * kNS + tid);
+      if (tid < kNS) next = load_written(reinterpret_cast<const uint4*>(dout) + (int64_t)rec * kNS + tid);
     };
     // the activations that mask this thread's share of a layer
     auto load_mask = [&](int rec, int layer) {
       const uint4* src = reinterpret_cast<const uint4*>(hid + ((int64_t)layer * n + rec) * kHBytes);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        mask[i] = __ldg(src + mine.pos * 8 + (((mine.c0 >> 3) + i) ^ (mine.pos & 7)));
+        mask[i] = load_written(src + mine.pos * 8 + (((mine.c0 >> 3) + i) ^ (mine.pos & 7)));
     };
     auto masked = [&](unsigned char* act) {
       wait_products(S, mine.tile, phase++);
@@ -436,8 +439,8 @@ int cgb::ws::forward_loss(const void* d_blob, const void* d_feat, int n, void* d
                               stream);
 }
 
-extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, const void* d_hid,
-                                   int n, void* d_dpre, void* stream) {
+static int launch_backward(bool after, const void* d_blobT, const void* d_dout, const void* d_hid,
+                           int n, void* d_dpre, void* stream) {
   if (n == 0) return CGB_OK;
   if (n < 0 || !d_blobT || !d_dout || !d_hid || !d_dpre)
     return fail(CGB_ERR_ARG, "cgb_ws_backward_dev: bad arguments");
@@ -446,10 +449,23 @@ extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, cons
   CGB_TRY_CUDA(cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kBwdBytes),
                "cudaFuncSetAttribute(backward)");
-  backward_kernel<<<grid, kConvThreads, kBwdBytes, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const unsigned char*>(d_blobT), static_cast<const unsigned char*>(d_dout),
-      static_cast<const unsigned char*>(d_hid), n, static_cast<unsigned char*>(d_dpre));
-  CGB_TRY_CUDA(cudaGetLastError(), "backward_kernel launch");
+  CGB_TRY_CUDA(launch_after(after, backward_kernel, grid, kConvThreads, kBwdBytes,
+                            reinterpret_cast<cudaStream_t>(stream),
+                            static_cast<const unsigned char*>(d_blobT),
+                            static_cast<const unsigned char*>(d_dout),
+                            static_cast<const unsigned char*>(d_hid), n,
+                            static_cast<unsigned char*>(d_dpre)),
+               "backward_kernel launch");
   note_launch();
   return CGB_OK;
+}
+
+extern "C" int cgb_ws_backward_dev(const void* d_blobT, const void* d_dout, const void* d_hid,
+                                   int n, void* d_dpre, void* stream) {
+  return launch_backward(false, d_blobT, d_dout, d_hid, n, d_dpre, stream);
+}
+
+int cgb::ws::backward_after(const void* d_blobT, const void* d_dout, const void* d_hid, int n,
+                            void* d_dpre, void* stream) {
+  return launch_backward(true, d_blobT, d_dout, d_hid, n, d_dpre, stream);
 }

@@ -80,9 +80,9 @@ constexpr int kD0 = 0, kD1 = 96, kD2 = 160;   // layers 2, 3: shifts -1 (and one
 constexpr int kDW1 = 0, kDb1 = 64, kDW4 = 128;
 
 __global__ void __launch_bounds__(kGradThreads, 1)
-    wgrad_kernel(const unsigned char* __restrict__ feat, const unsigned char* __restrict__ hid,
-                 const unsigned char* __restrict__ dpre, const unsigned char* __restrict__ dout,
-                 int n, int parts, float* __restrict__ partial) {
+    wgrad_kernel(const unsigned char* __restrict__ feat, const unsigned char* hid,
+                 const unsigned char* dpre, const unsigned char* dout, int n, int parts,
+                 float* partial) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + 2 * kStage);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   __syncthreads();
   tfir::fence_after();
   const uint32_t tmem = __shfl_sync(kFull, S.tmem, 0);
+  wait_previous(hid, dpre, dout);
   const int64_t layer = (int64_t)n * kNS * 128;  // bytes of a layer of hid, dpre
   const int records = slot < n ? (n - slot + parts - 1) / parts : 0;
 
@@ -164,14 +165,14 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       const uint4* q = reinterpret_cast<const uint4*>(second + (int64_t)rec * kNS * 128);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        g[j] = __ldg(p + tid + kLoaders * j);
-        g[4 + j] = __ldg(q + tid + kLoaders * j);
+        g[j] = load_written(p + tid + kLoaders * j);
+        g[4 + j] = load_written(q + tid + kLoaders * j);
       }
       if (group == 2) {
         if (tid < kFeatRows)
           g[8] = __ldg(reinterpret_cast<const uint4*>(feat + (int64_t)rec * kFeat) + tid);
         if (tid < kNS)
-          g[9] = __ldg(reinterpret_cast<const uint4*>(dout + (int64_t)rec * kNS * 16) + tid);
+          g[9] = load_written(reinterpret_cast<const uint4*>(dout + (int64_t)rec * kNS * 16) + tid);
       }
     };
     auto store = [&](int st) {
@@ -282,8 +283,9 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 constexpr int kSumThreads = 128;
 
 __global__ void __launch_bounds__(kSumThreads)
-    reduce_kernel(const float* __restrict__ partial, int parts, float* __restrict__ grad,
-                  const double* __restrict__ loss_part, int n, double* __restrict__ loss) {
+    reduce_kernel(const float* partial, int parts, float* __restrict__ grad,
+                  const double* loss_part, int n, double* __restrict__ loss) {
+  wait_previous(partial, loss_part);
   if (loss && blockIdx.x == gridDim.x - 1) {
     __shared__ double red[kSumThreads];
     double d = 0.0;
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(kSumThreads)
   const float* p = partial + i;
   float s = 0.0f, c = 0.0f;
 #pragma unroll 25
-  for (int k = 0; k < parts; ++k) two_sum_add(s, c, __ldg(p + (int64_t)k * kParams));
+  for (int k = 0; k < parts; ++k) two_sum_add(s, c, p[(int64_t)k * kParams]);
   float total = __fadd_rn(s, c);
   if (!(fabsf(total) < __int_as_float(0x7f800000))) {
     double d = 0.0;
@@ -321,10 +323,11 @@ using namespace cgb::ws;
 
 namespace {
 
-// loss_part, loss: null, or the records' losses and where their mean goes.
+// loss_part, loss: null, or the records' losses and where their mean goes; after: the
+// kernel before it on the stream is the backward pass of the step.
 int launch_wgrad(const void* d_feat, const void* d_hid, const void* d_dpre, const void* d_dout,
                  int n, float* d_partial, int n_parts, float* d_grad, const double* loss_part,
-                 double* loss, cudaStream_t st) {
+                 double* loss, bool after, cudaStream_t st) {
   if (n < 0 || n_parts < 1 || !d_feat || !d_hid || !d_dpre || !d_dout || !d_partial || !d_grad)
     return fail(CGB_ERR_ARG, "cgb_ws_wgrad_dev: bad arguments");
   int dev = 0, sms = 0;
@@ -338,15 +341,17 @@ int launch_wgrad(const void* d_feat, const void* d_hid, const void* d_dpre, cons
   CGB_TRY_CUDA(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kGradSmem),
                "cudaFuncSetAttribute(wgrad)");
-  wgrad_kernel<<<kGroups * parts, kGradThreads, kGradSmem, st>>>(
-      static_cast<const unsigned char*>(d_feat), static_cast<const unsigned char*>(d_hid),
-      static_cast<const unsigned char*>(d_dpre), static_cast<const unsigned char*>(d_dout), n,
-      parts, d_partial);
-  CGB_TRY_CUDA(cudaGetLastError(), "wgrad_kernel launch");
+  CGB_TRY_CUDA(launch_after(after, wgrad_kernel, kGroups * parts, kGradThreads, kGradSmem, st,
+                            static_cast<const unsigned char*>(d_feat),
+                            static_cast<const unsigned char*>(d_hid),
+                            static_cast<const unsigned char*>(d_dpre),
+                            static_cast<const unsigned char*>(d_dout), n, parts, d_partial),
+               "wgrad_kernel launch");
   note_launch();
-  reduce_kernel<<<(kParams + kSumThreads - 1) / kSumThreads + (loss ? 1 : 0), kSumThreads, 0, st>>>(
-      d_partial, parts, d_grad, loss_part, n, loss);
-  CGB_TRY_CUDA(cudaGetLastError(), "reduce_kernel launch");
+  CGB_TRY_CUDA(launch_after(true, reduce_kernel,
+                            (kParams + kSumThreads - 1) / kSumThreads + (loss ? 1 : 0),
+                            kSumThreads, 0, st, d_partial, parts, d_grad, loss_part, n, loss),
+               "reduce_kernel launch");
   note_launch();
   return CGB_OK;
 }
@@ -357,7 +362,7 @@ extern "C" int cgb_ws_wgrad_dev(const void* d_feat, const void* d_hid, const voi
                                 const void* d_dout, int n, float* d_partial, int n_parts,
                                 float* d_grad, void* stream) {
   return launch_wgrad(d_feat, d_hid, d_dpre, d_dout, n, d_partial, n_parts, d_grad, nullptr,
-                      nullptr, reinterpret_cast<cudaStream_t>(stream));
+                      nullptr, false, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, const void* d_feat,
@@ -369,7 +374,7 @@ extern "C" int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, con
   if (const int rc = forward_loss(d_blob, d_feat, n, d_hid, d_out, d_target, s_out, d_dout,
                                   d_loss_part, stream))
     return rc;
-  if (const int rc = cgb_ws_backward_dev(d_blobT, d_dout, d_hid, n, d_dpre, stream)) return rc;
+  if (const int rc = backward_after(d_blobT, d_dout, d_hid, n, d_dpre, stream)) return rc;
   return launch_wgrad(d_feat, d_hid, d_dpre, d_dout, n, d_partial, n_parts, d_grad, d_loss_part,
-                      d_loss, reinterpret_cast<cudaStream_t>(stream));
+                      d_loss, n > 0, reinterpret_cast<cudaStream_t>(stream));
 }

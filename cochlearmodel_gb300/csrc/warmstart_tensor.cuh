@@ -49,5 +49,54 @@ __device__ __forceinline__ void wait_products(TensorShared& S, int h, int phase)
   }
 }
 
+// A training step's kernels are launched so that one's CTAs start where the one
+// before it leaves an SM (launch_after): weights, zero rows and tensor memory are
+// prepared beside its last records, and the launch takes no time of its own.
+// release_next() comes after the CTA's own tensor memory is allocated, so that a CTA
+// which holds tensor memory only ever waits for CTAs that have theirs.
+// wait_previous() comes before the first access to what the earlier kernels write,
+// whose addresses it passes on: the compiler may move load_written, but not over the
+// wait (with plain loads 2 us more at 256 records).  wgrad releases its sum's CTAs only
+// by ending: started early they cost it 2 to 3 us.  Measured (GB300), step of 32 / 256 /
+// 1,024 records: 41.0 / 61.5 / 183 -> 32.8 / 55.3 / 174 us.
+__device__ __forceinline__ void release_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... T>
+__device__ __forceinline__ void wait_previous(const T*&... written) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ((void)[](const T*& p) { asm volatile("" : "+l"(p)::"memory"); }(written), ...);
+}
+
+__device__ __forceinline__ uint4 load_written(const uint4* p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p));
+  return v;
+}
+
+// after: the kernel before it on the stream is the step's previous one.
+template <typename... Params, typename... Args>
+cudaError_t launch_after(bool after, void (*kernel)(Params...), int grid, int threads, int smem,
+                         cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)grid);
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = (size_t)smem;
+  config.stream = st;
+  config.attrs = &attr;
+  config.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// cgb_ws_backward_dev, after the forward pass of the same step (warmstart_conv.cu).
+int backward_after(const void* d_blobT, const void* d_dout, const void* d_hid, int n, void* d_dpre,
+                   void* stream);
+
 }  // namespace ws
 }  // namespace cgb

@@ -122,3 +122,36 @@ def test_mean_loss(n):
     # an FP32 product and difference (two roundings) per term, or one if contracted
     assert abs(float(loss) - want) <= 2.0 ** -21 * want
     assert abs(float(loss) - float(buf["loss"].sum()) / (n * 256)) <= (n + 16) * 2.0 ** -52 * want
+
+
+@pytest.mark.parametrize("n", [1, 151, 153, 400])
+def test_overlapped_step_is_the_separate_calls(n):
+    """The one-call step, whose kernels overlap, on changing inputs and from a
+    graph, against its kernels called one by one: the same bits."""
+    g = torch.Generator(device=D).manual_seed(n)
+    net = warmstart.WarmStartNet(D, seed=n)
+    feat = torch.zeros(n, 280, 8, dtype=torch.bfloat16, device=D)
+    target = torch.zeros(n, 256, device=D)
+    buf, ref = net.buffers(n), net.buffers(n)
+    net.gradients(feat, target, buf)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        net.gradients(feat, target, buf)
+    ref["partial"] = torch.zeros_like(buf["partial"])
+    parts = buf["partial"].shape[0]
+    p = native.ptr
+    for i in range(8):
+        feat[:, 8:264] = torch.randn(n, 256, 8, generator=g, device=D).to(torch.bfloat16)
+        target.normal_(generator=g)
+        graph.replay() if i % 2 else net.gradients(feat, target, buf)
+        st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        net.forward(feat, ref)
+        native.check(net.lib.cgb_ws_loss_dev(p(ref["out"]), p(target), n, net.s_out,
+                                             p(ref["dout"]), p(ref["loss"]), st), "loss")
+        native.check(net.lib.cgb_ws_backward_dev(p(net.blobT), p(ref["dout"]), p(ref["hid"]), n,
+                                                 p(ref["dpre"]), st), "backward")
+        native.check(net.lib.cgb_ws_wgrad_dev(p(feat), p(ref["hid"]), p(ref["dpre"]),
+                                              p(ref["dout"]), n, p(ref["partial"]), parts,
+                                              p(ref["grad"]), st), "wgrad")
+        for k in ("hid", "out", "dout", "dpre", "loss", "grad"):
+            assert torch.equal(buf[k], ref[k]), (i, k)
