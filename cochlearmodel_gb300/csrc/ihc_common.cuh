@@ -98,18 +98,32 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+__device__ __forceinline__ void mbar_init(uint64_t* mbar, int arrivals) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(arrivals));
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
+}
+// Whether completion `phase` (from 0) of mbar has come; the instruction waits a short
+// time for it.
+__device__ __forceinline__ bool mbar_done(uint64_t* mbar, int phase) {
+  uint32_t done;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+      : "=r"(done)
+      : "r"(smem_u32(mbar)), "r"((uint32_t)(phase & 1))
+      : "memory");
+  return done != 0;
+}
+
 // Wait on phase `parity` of mbar by every thread, for at most kWaitNs of the
 // global timer (each try_wait returns within a short system-defined time),
 // then a block-wide vote so that all threads take the same branch.
 __device__ __forceinline__ bool wait_stage(uint64_t* mbar, uint32_t parity) {
-  uint32_t done = 0;
+  bool done = false;
   const unsigned long long t_start = global_ns();
   while (!done) {
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(smem_u32(mbar)), "r"(parity)
-        : "memory");
+    done = mbar_done(mbar, (int)parity);
     if (!done && global_ns() - t_start > kWaitNs) break;
   }
   return __syncthreads_and(done) != 0;

@@ -58,7 +58,6 @@ namespace {
 
 constexpr int kWorkers = kIhcWarps * 32;   // threads that do everything but issue
 constexpr int kThreads = kWorkers + 128;   // the issuing warp's group of four
-constexpr int kBarrier = kWorkers + 32;
 // registers a thread: 96 at launch (640 threads), then 112 for the workers and
 // 32 for the issuing warp's group, together the same
 constexpr int kWorkerRegs = 112, kIssueRegs = 32;
@@ -79,9 +78,10 @@ struct __align__(16) PointScratch {
 
 struct TensorShared {
   uint64_t mbar[2];          // products of half h are done
+  uint64_t ready[2];         // a digit of half h is in shared memory (a warp, an arrival)
+  uint64_t drained;          // all products that were issued are done
   uint32_t tmem;
   int abort;                 // a wait ran out
-  int stop;                  // the workers have ended the run early
   float floor;               // least slack, in units of the accumulators
   int listed;                // points for Dot2 (more than kList: those flagged)
   int dot2_rows[2];          // rows for Dot2, by tile parity
@@ -109,11 +109,21 @@ constexpr int kRowZero = 0, kRowSum = 1, kRowDot2 = 2;
 __device__ __forceinline__ void sync_workers() {
   asm volatile("bar.sync 3, %0;" ::"n"(kWorkers) : "memory");
 }
-__device__ __forceinline__ void half_ready(int h) {  // workers
-  asm volatile("bar.arrive %0, %1;" ::"r"(1 + h), "n"(kBarrier) : "memory");
+// Workers: this warp's share of half h of a digit is in shared memory.
+__device__ __forceinline__ void half_ready(TensorShared& S, int h, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&S.ready[h]);
 }
-__device__ __forceinline__ void half_wait(int h) {  // the issuing warp
-  asm volatile("bar.sync %0, %1;" ::"r"(1 + h), "n"(kBarrier) : "memory");
+// The issuing warp, converged: phase `n` of ready[h]; false where a wait of the
+// workers, or this one, ran out.
+__device__ __forceinline__ bool half_wait(TensorShared& S, int h, int n) {
+  const unsigned long long start = global_ns();
+  while (!__all_sync(kFull, mbar_done(&S.ready[h], n))) {
+    // (the workers' steps between two digits are far shorter, their waits a fourth)
+    const bool late = global_ns() - start > 4 * kWaitNs;
+    if (__any_sync(kFull, late || *(volatile int*)&S.abort)) return false;
+  }
+  return true;
 }
 
 // TwoSum, two at once
@@ -450,10 +460,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int first = t0 - back;
 
   if (threadIdx.x == 0) {
-    for (int h = 0; h < 2; ++h)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.mbar[h])));
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&S.mbar[h], 1);
+      mbar_init(&S.ready[h], kIhcWarps);
+    }
+    mbar_init(&S.drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    S.abort = S.stop = 0;
+    S.abort = 0;
     S.listed = 0;
     S.dot2_rows[0] = S.dot2_rows[1] = 0;
   }
@@ -500,11 +513,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kIhcWarps) {
     // the issuing warp
     const uint32_t issue = tfir::elected();
+    int n = 0;  // digits so far
     for (int t = first; t < t1; ++t) {
-      for (int i = 0; i < tfir::kDigits; ++i) {
+      for (int i = 0; i < tfir::kDigits; ++i, ++n) {
         for (int h = 0; h < 2; ++h) {
-          half_wait(h);
-          if (i == 0 && h == 0 && *(volatile int*)&S.stop) goto done;
+          if (!half_wait(S, h, n)) goto done;
           tfir::fence_after();
           // (test-only: the first half's products are left out, so that the
           // wait for them runs out)
@@ -515,7 +528,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
-  done:;
+  done:
+    // The shared memory that the products read and the tensor memory that they write
+    // are given up only after the last of them, also where nobody waited for it.
+    if (issue) tfir::commit(&S.drained);
+    const unsigned long long start = global_ns();
+    while (!mbar_done(&S.drained, 0) && global_ns() - start < kWaitNs) {
+    }
+    __syncwarp();
   } else if (warp < kIhcWarps) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
     const int sg = warp & 1, gw = warp >> 1;  // section half; rows of x 24 gw .. of each half
@@ -613,20 +633,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                        tfir::pack2(d[6], d[7]));
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      half_ready(h);
+      half_ready(S, h, lane);
     };
     // Phase `n` of mbar[h].  Bounded; after a wait that ran out none waits, the
     // tile goes on with what is there and the run ends with it.
     auto wait_half = [&](int h, int n) {
-      uint32_t done = 0;
       unsigned long long start = 0;
-      while (!done) {
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(done)
-            : "r"(smem_u32(&S.mbar[h])), "r"((uint32_t)(n & 1))
-            : "memory");
-        if (done) break;
+      while (!mbar_done(&S.mbar[h], n)) {
         if (*(volatile int*)&S.abort) break;
         if (start == 0) start = global_ns();
         if (global_ns() - start > kWaitNs) {
@@ -1004,12 +1017,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       at += tfir::kRows;
       at -= at >= ring ? ring : 0;
       if (*(volatile int*)&S.abort) {
-        if (threadIdx.x == 0) {
-          S.stop = 1;
-          atomicOr(A.status, 1);
-        }
-        sync_workers();
-        if (t + 1 < t1) half_ready(0);
+        if (threadIdx.x == 0) atomicOr(A.status, 1);
         break;
       }
     }
