@@ -113,16 +113,6 @@ __device__ __forceinline__ void issue_conv8(TensorShared& S, uint32_t in, int ro
   }
 }
 
-__device__ __forceinline__ void hand_over() {  // finishers: the operand is complete
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  tfir::fence_before();
-  asm volatile("bar.arrive 1, %0;" ::"n"(kConvThreads) : "memory");
-}
-__device__ __forceinline__ void take_over() {  // the issuing warp
-  asm volatile("bar.sync 1, %0;" ::"n"(kConvThreads) : "memory");
-  tfir::fence_after();
-}
-
 // A finished layer to global memory (64-channel rows).
 __device__ __forceinline__ void write_layer(unsigned char* __restrict__ dst,
                                             const unsigned char* act, int tid) {
@@ -158,7 +148,7 @@ struct Share {
 
 // What both kernels begin with; the address of tensor memory.
 __device__ __forceinline__ uint32_t begin(unsigned char* sm, TensorShared& S, int tid, int warp) {
-  if (tid == 0) init_barriers(S);
+  if (tid == 0) init_barriers(S, kFinishers / 32);
   if (warp == kFinishers / 32) tfir::tmem_alloc(&S.tmem);
   // rows beside the positions
   if (tid < 2 * 8 * 4) {
@@ -178,7 +168,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     forward_kernel(const unsigned char* __restrict__ blob, const unsigned char* __restrict__ feat,
                    int n, unsigned char* __restrict__ hid, float* __restrict__ out,
                    const float* __restrict__ target, float s_out,
-                   unsigned char* __restrict__ dout, double* __restrict__ loss_part) {
+                   unsigned char* __restrict__ dout, double* __restrict__ loss_part, int skip) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + kOffFwdShared);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -199,16 +189,19 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 
   if (warp == kFinishers / 32) {
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
+    int phase = 0;
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-      take_over();
-      issue_conv8(S, base + kOffIn, 6, base + kOffFirst, tmem, issue);
-      take_over();
+      if (!take_over(S, 0, phase++)) break;
+      if (!skip || phase > 1)
+        issue_conv8(S, base + kOffIn, 6, base + kOffFirst, tmem, issue);
+      if (!take_over(S, 0, phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffSecond, kWChunk, kWTap, instr(64, false), tmem, issue);
-      take_over();
+      if (!take_over(S, 0, phase++)) break;
       issue_conv64(S, base + kOffB, base + kOffThird, kWChunk, kWTap, instr(64, false), tmem, issue);
-      take_over();
+      if (!take_over(S, 0, phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffLast, kW4Chunk, kW4Tap, instr(16, false), tmem, issue);
     }
+    drain(S, issue);
   } else {
     const Share mine(tmem, warp, lane);
     int phase = 0;
@@ -239,7 +232,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]),
                        pack_bf16(r[6], r[7]));
       }
-      hand_over();
+      hand_over(S, 0, lane);
       // what is copied next was written by all
       asm volatile("bar.sync 2, %0;" ::"n"(kFinishers) : "memory");
     };
@@ -247,7 +240,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
       unsigned char* h = hid + (int64_t)rec * kHBytes;
       if (tid < kFeatRows) reinterpret_cast<uint4*>(sm + kOffIn)[tid] = next;
-      hand_over();
+      hand_over(S, 0, lane);
       if (rec + gridDim.x < n) load(rec + gridDim.x);
       hidden(sm + kOffA, bias);
       write_layer(h, sm + kOffA, tid);
@@ -261,15 +254,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         float v[8];
         tfir::tmem_load8(mine.tmem, v);
         tfir::tmem_wait_loads();
-        const float o =
-            *(volatile int*)&S.failed ? __int_as_float(0x7fffffff) : v[0] + bias[192];
+        const bool failed = *(volatile int*)&S.failed;
+        const float o = failed ? __int_as_float(0x7fffffff) : v[0] + bias[192];
         out[(int64_t)rec * kNS + mine.pos] = o;
         if (LOSS) {
           double* red = reinterpret_cast<double*>(sm + kOffSquares);
           const float e = s_out * o - target[(int64_t)rec * kNS + mine.pos];
           const float gsc = 2.0f * s_out / ((float)n * 256.0f);
           reinterpret_cast<uint4*>(dout)[(int64_t)rec * kNS + mine.pos] =
-              make_uint4(bf16_bits(gsc * e), 0, 0, 0);
+              make_uint4(failed ? 0x7fffu : bf16_bits(gsc * e), 0, 0, 0);
           red[mine.pos] = (double)e * (double)e;
           // (warps 0 to 7; the next record's squares come after barriers of all)
           asm volatile("bar.sync 3, %0;" ::"n"(kNS) : "memory");
@@ -298,7 +291,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 __global__ void __launch_bounds__(kConvThreads, 1)
     backward_kernel(const unsigned char* __restrict__ blobT,
                     const unsigned char* dout, const unsigned char* hid, int n,
-                    unsigned char* dpre) {
+                    unsigned char* dpre, int skip) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + kOffBwdShared);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -314,14 +307,17 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 
   if (warp == kFinishers / 32) {
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
+    int phase = 0;
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-      take_over();
-      issue_conv8(S, base + kOffIn, 0, base + kOffFirst, tmem, issue);
-      take_over();
+      if (!take_over(S, 0, phase++)) break;
+      if (!skip || phase > 1)
+        issue_conv8(S, base + kOffIn, 0, base + kOffFirst, tmem, issue);
+      if (!take_over(S, 0, phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffSecond, kWChunk, kWTap, instr(64, false), tmem, issue);
-      take_over();
+      if (!take_over(S, 0, phase++)) break;
       issue_conv64(S, base + kOffB, base + kOffThird, kWChunk, kWTap, instr(64, false), tmem, issue);
     }
+    drain(S, issue);
   } else {
     const Share mine(tmem, warp, lane);
     int phase = 0;
@@ -360,16 +356,16 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
       unsigned char* d = dpre + (int64_t)rec * kHBytes;
       if (tid < kNS) reinterpret_cast<uint4*>(sm + kOffIn)[tid + 2] = next;
-      hand_over();
+      hand_over(S, 0, lane);
       load_mask(rec, 2);
       if (rec + gridDim.x < n) load(rec + gridDim.x);
       masked(sm + kOffA);
-      hand_over();
+      hand_over(S, 0, lane);
       load_mask(rec, 1);
       asm volatile("bar.sync 2, %0;" ::"n"(kFinishers) : "memory");
       write_layer(d + 2 * (int64_t)n * kHBytes, sm + kOffA, tid);
       masked(sm + kOffB);
-      hand_over();
+      hand_over(S, 0, lane);
       load_mask(rec, 0);
       asm volatile("bar.sync 2, %0;" ::"n"(kFinishers) : "memory");
       write_layer(d + (int64_t)n * kHBytes, sm + kOffB, tid);
@@ -400,6 +396,13 @@ int conv_grid(int n, int* grid) {
 using namespace cgb;
 using namespace cgb::ws;
 
+int cgb::ws::g_fault_skip_products = 0;
+
+extern "C" int cgb_ws_set_fault_injection(int skip_products) {
+  g_fault_skip_products = skip_products ? 1 : 0;
+  return CGB_OK;
+}
+
 template <bool LOSS>
 static int launch_forward(const void* d_blob, const void* d_feat, int n, void* d_hid, float* d_out,
                           const float* d_target, float s_out, void* d_dout, double* d_loss_part,
@@ -412,7 +415,7 @@ static int launch_forward(const void* d_blob, const void* d_feat, int n, void* d
   forward_kernel<LOSS><<<grid, kConvThreads, kFwdBytes, reinterpret_cast<cudaStream_t>(stream)>>>(
       static_cast<const unsigned char*>(d_blob), static_cast<const unsigned char*>(d_feat), n,
       static_cast<unsigned char*>(d_hid), d_out, d_target, s_out,
-      static_cast<unsigned char*>(d_dout), d_loss_part);
+      static_cast<unsigned char*>(d_dout), d_loss_part, g_fault_skip_products);
   CGB_TRY_CUDA(cudaGetLastError(), "forward_kernel launch");
   note_launch();
   return CGB_OK;
@@ -454,7 +457,7 @@ static int launch_backward(bool after, const void* d_blobT, const void* d_dout, 
                             static_cast<const unsigned char*>(d_blobT),
                             static_cast<const unsigned char*>(d_dout),
                             static_cast<const unsigned char*>(d_hid), n,
-                            static_cast<unsigned char*>(d_dpre)),
+                            static_cast<unsigned char*>(d_dpre), g_fault_skip_products),
                "backward_kernel launch");
   note_launch();
   return CGB_OK;

@@ -82,12 +82,12 @@ constexpr int kDW1 = 0, kDb1 = 64, kDW4 = 128;
 __global__ void __launch_bounds__(kGradThreads, 1)
     wgrad_kernel(const unsigned char* __restrict__ feat, const unsigned char* hid,
                  const unsigned char* dpre, const unsigned char* dout, int n, int parts,
-                 float* partial) {
+                 float* partial, int skip) {
   extern __shared__ __align__(128) unsigned char sm[];
   TensorShared& S = *reinterpret_cast<TensorShared*>(sm + 2 * kStage);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = blockIdx.x % kGroups, slot = blockIdx.x / kGroups;
-  if (tid == 0) init_barriers(S);
+  if (tid == 0) init_barriers(S, kLoaders / 32);
   if (warp == kLoaders / 32) tfir::tmem_alloc(&S.tmem);
   // zero rows around the positions, and the rows of ones
   for (int st = 0; st < 2; ++st) {
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     for (int it = 0; it < records; ++it) {
       const int st = it & 1;
       const uint32_t base = tfir::saddr(sm) + st * kStage;
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + st), "n"(kGradThreads) : "memory");
-      tfir::fence_after();
+      if (!take_over(S, st, it >> 1)) break;
+      if (skip) continue;
       if (group < 2) {
         const uint64_t a = operand(base, kAChunk), b = operand(base + kOffB, kBChunk);
 #pragma unroll 1
@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       if (issue) tfir::commit(&S.mbar[st]);
       __syncwarp();
     }
+    drain(S, issue);
   } else {
     // 16 bytes u of a record: row u / 8, and its chunk by the rows' swizzle.  The
     // first factor (dPre) in g[0..3], the second (In) in g[4..7]; layers 1 and 4
@@ -193,8 +194,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         if (tid < kFeatRows) *reinterpret_cast<uint4*>(s + tid * 16) = g[8];
         if (tid < kNS) *reinterpret_cast<uint4*>(s + kOffO + (tid + 2) * 16) = g[9];
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("bar.arrive %0, %1;" ::"r"(1 + st), "n"(kGradThreads) : "memory");
+      hand_over(S, st, lane);
     };
     if (records) load(slot);
     for (int it = 0; it < records; ++it) {
@@ -345,7 +345,8 @@ int launch_wgrad(const void* d_feat, const void* d_hid, const void* d_dpre, cons
                             static_cast<const unsigned char*>(d_feat),
                             static_cast<const unsigned char*>(d_hid),
                             static_cast<const unsigned char*>(d_dpre),
-                            static_cast<const unsigned char*>(d_dout), n, parts, d_partial),
+                            static_cast<const unsigned char*>(d_dout), n, parts, d_partial,
+                            g_fault_skip_products),
                "wgrad_kernel launch");
   note_launch();
   CGB_TRY_CUDA(launch_after(true, reduce_kernel,

@@ -14,9 +14,11 @@ int forward_loss(const void* d_blob, const void* d_feat, int n, void* d_hid, flo
                  void* stream);
 
 struct TensorShared {
-  uint64_t mbar[2];  // the products of stage (or tile) h are done
+  uint64_t mbar[2];   // the products of stage (or tile) h are done
+  uint64_t ready[2];  // the operands (of stage h) are in shared memory: an arrival a warp
+  uint64_t drained;   // all products that were issued are done
   uint32_t tmem;
-  int failed;        // a wait ran out
+  int failed;         // a wait ran out
 };
 
 // FP32 accumulators, BF16 operands (both K-major, or both MN-major), M = 128.
@@ -25,9 +27,13 @@ __host__ __device__ constexpr uint32_t instr(int n, bool mn_major) {
          ((uint32_t)(n / 8) << 17) | (8u << 24);
 }
 
-__device__ __forceinline__ void init_barriers(TensorShared& S) {  // one thread
-  for (int h = 0; h < 2; ++h)
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tfir::saddr(&S.mbar[h])));
+// warps: that prepare the operands
+__device__ __forceinline__ void init_barriers(TensorShared& S, int warps) {  // one thread
+  for (int h = 0; h < 2; ++h) {
+    mbar_init(&S.mbar[h], 1);
+    mbar_init(&S.ready[h], warps);
+  }
+  mbar_init(&S.drained, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   S.failed = 0;
 }
@@ -35,19 +41,47 @@ __device__ __forceinline__ void init_barriers(TensorShared& S) {  // one thread
 // Completion `phase` (from 0) of mbar[h].  Bounded; after a wait that ran out none
 // waits, and the kernel's results become NaN.
 __device__ __forceinline__ void wait_products(TensorShared& S, int h, int phase) {
-  uint32_t done = 0;
   unsigned long long start = 0;
-  while (!done) {
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-        : "=r"(done)
-        : "r"(tfir::saddr(&S.mbar[h])), "r"((uint32_t)(phase & 1))
-        : "memory");
-    if (done || *(volatile int*)&S.failed) break;
+  while (!mbar_done(&S.mbar[h], phase)) {
+    if (*(volatile int*)&S.failed) break;
     if (start == 0) start = global_ns();
     if (global_ns() - start > kWaitNs) *(volatile int*)&S.failed = 1;
   }
 }
+
+// This warp's share of an operand (of stage h) is in shared memory.
+__device__ __forceinline__ void hand_over(TensorShared& S, int h, int lane) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tfir::fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&S.ready[h]);
+}
+// The issuing warp, converged: completion `phase` of ready[h]; false after a wait
+// that ran out.
+__device__ __forceinline__ bool take_over(TensorShared& S, int h, int phase) {
+  const unsigned long long start = global_ns();
+  while (!__all_sync(kFull, mbar_done(&S.ready[h], phase))) {
+    // (the other warps' work between two operands is far shorter, their waits a fourth)
+    const bool late = global_ns() - start > 4 * kWaitNs;
+    if (__any_sync(kFull, late || *(volatile int*)&S.failed)) return false;
+  }
+  tfir::fence_after();
+  return true;
+}
+// The issuing warp's last step: the shared memory that its products read and the
+// tensor memory that they write are given up only after the last of them, also where
+// nobody waited for it.
+__device__ __forceinline__ void drain(TensorShared& S, uint32_t issue) {
+  if (issue) tfir::commit(&S.drained);
+  const unsigned long long start = global_ns();
+  while (!mbar_done(&S.drained, 0) && global_ns() - start < kWaitNs) {
+  }
+  __syncwarp();
+}
+
+// Test-only (cgb_ws_set_fault_injection): the next launches leave out products that
+// are waited for.
+extern int g_fault_skip_products;
 
 // A training step's kernels are launched so that one's CTAs start where the one
 // before it leaves an SM (launch_after): weights, zero rows and tensor memory are

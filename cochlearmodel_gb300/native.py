@@ -107,6 +107,7 @@ _SIGS = {
                                   _p, _p]),
     "cgb_ws_adam_dev": (_i, [_p, _p, _p, _p, _i, C.c_float, C.c_float, C.c_float, C.c_float,
                              _p]),
+    "cgb_ws_set_fault_injection": (_i, [_i]),
     "cgb_ws_infer_dev": (_i, [_p, _p, _i, _p, _p]),
 }
 

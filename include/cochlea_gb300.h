@@ -248,6 +248,11 @@ int cgb_ws_gradients_dev(const void* d_blob, const void* d_blobT, const void* d_
 int cgb_ws_adam_dev(float* d_params, const float* d_grad, float* d_m, float* d_v, int step,
                     float lr, float beta1, float beta2, float eps, void* stream);
 int cgb_ws_infer_dev(const void* d_blob, const void* d_feat, int n, float* d_out, void* stream);
+/* Test-only fault injection for the training kernels' bounded waits: with 1, later
+ * launches of the forward and backward kernels leave out each CTA's first products, and
+ * of the weight-gradient kernel all, so that the wait for them runs out after about one
+ * second and the results are NaN; 0 restores normal launches. */
+int cgb_ws_set_fault_injection(int skip_products);
 
 /* IHC + lambda over n_frames frames (host frame table, device buffers).
  *   d_v      float[v_rows][256]  BM velocity (16-byte aligned)
