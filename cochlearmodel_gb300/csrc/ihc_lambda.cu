@@ -491,14 +491,19 @@ int g_forced_run = 0;
 
 // How each scratch buffer's tables were uploaded: the tile prefix on the device
 // depends on the kernel and the run length, so a launch of uploaded tables must
-// use the same ones whatever the settings are by then.
+// use the same ones whatever the settings are by then, and what the kernels take
+// from the taps is of the uploaded ones.  A launch with other lengths would read
+// the tables at the wrong places: it is an error.
 struct Uploaded {
+  int n_frames, n_ac, n_dc;
+  int n_tiles;  // runs of tiles of all frames
   int run;
   bool tensor;
-  int exp_b;  // of the uploaded taps, for the tensor kernel
+  int exp_b;  // for the tensor kernel
+  int ac_sym, dc_uniform;
 };
-std::mutex g_upload_run_mu;
-std::unordered_map<const void*, Uploaded> g_upload_run;
+std::mutex g_uploaded_mu;
+std::unordered_map<const void*, Uploaded> g_uploaded;
 
 int sm_count() {
   int dev = 0, n_sm = 0;
@@ -631,28 +636,24 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   // The AC filter goes to the tensor cores where the kernel is built for it: a
   // uniform DC filter, no debug stage, no AC given, lengths that fit.
   int exp_b = 0;
-  bool tensor = !ac_ext && stage == 0 && dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
-                tensor_taps(ac_taps, n_ac, prm->scale, &exp_b);
-  int run = tensor ? pick_tensor_run(frames, n_frames, n_dc)
-                   : pick_run(frames, n_frames, TR, n_dc);
-  {
-    std::lock_guard<std::mutex> lock(g_upload_run_mu);
-    if (mode & kUpload) {
-      g_upload_run[d_scratch] = {run, tensor, exp_b};
-    } else {
-      const auto it = g_upload_run.find(d_scratch);
-      if (it != g_upload_run.end()) {
-        run = it->second.run;
-        tensor = it->second.tensor;
-        exp_b = it->second.exp_b;
-        // the tensor kernel's buffers are for the lengths that it was chosen for
-        if (tensor && (!ihc_tensor_fits(n_ac, n_dc) || ac_ext || stage != 0))
-          return fail(CGB_ERR_ARG,
-                      "cgb_ihc_lambda_launch_dev: not the filters that were uploaded");
-      }
-    }
+  const bool tensor = !ac_ext && stage == 0 && dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
+                      tensor_taps(ac_taps, n_ac, prm->scale, &exp_b);
+  Uploaded up{n_frames, n_ac, n_dc, 0,
+              tensor ? pick_tensor_run(frames, n_frames, n_dc)
+                     : pick_run(frames, n_frames, TR, n_dc),
+              tensor, exp_b, ac_symmetric(ac_taps, n_ac, prm->scale), dc_uniform};
+  bool known = false;
+  if (!(mode & kUpload)) {
+    std::lock_guard<std::mutex> lock(g_uploaded_mu);
+    const auto it = g_uploaded.find(d_scratch);
+    known = it != g_uploaded.end();
+    if (known) up = it->second;
   }
-  if (tensor) TR = kTensorTileRows;
+  if (up.n_ac != n_ac || up.n_dc != n_dc)
+    return fail(CGB_ERR_ARG, "cgb_ihc_lambda_launch_dev: not the filters that were uploaded");
+  if (up.n_frames != n_frames)
+    return fail(CGB_ERR_ARG, "cgb_ihc_lambda_launch_dev: not the frames that were uploaded");
+  if (up.tensor) TR = kTensorTileRows;
   for (int i = 0; i < n_frames; ++i) {
     const cgb_ihc_frame& fr = frames[i];
     const bool ok = fr.v_row0 >= 0 && fr.lam_rows >= 0 && fr.lam_rows <= fr.rows &&
@@ -663,9 +664,16 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
       return fail(CGB_ERR_RANGE,
                   "cgb_ihc_lambda_dev: frame " + std::to_string(i) + " out of range");
     const int tiles = (fr.lam_rows + TR - 1) / TR;
-    prefix[i + 1] = prefix[i] + (tiles + run - 1) / run;
+    prefix[i + 1] = prefix[i] + (tiles + up.run - 1) / up.run;
   }
   const int n_tiles = prefix[n_frames];
+  if (known && n_tiles != up.n_tiles)
+    return fail(CGB_ERR_ARG, "cgb_ihc_lambda_launch_dev: not the frames that were uploaded");
+  up.n_tiles = n_tiles;
+  if (mode & kUpload) {
+    std::lock_guard<std::mutex> lock(g_uploaded_mu);
+    g_uploaded[d_scratch] = up;
+  }
   if (n_tiles == 0) return CGB_OK;
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -720,10 +728,10 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   A.skip_first_copy = g_fault_skip_copy;
   A.stage = stage == 12 ? 11 : stage;  // the reference's 12 ("Shigh") is dS too
   A.stage_out = d_stage;
-  A.run = run;
-  A.dc_uniform = dc_uniform;
-  A.ac_sym = ac_symmetric(ac_taps, n_ac, prm->scale);
-  if (tensor) return ihc_tensor_launch(A, d_v, n_tiles, exp_b, st);
+  A.run = up.run;
+  A.dc_uniform = up.dc_uniform;
+  A.ac_sym = up.ac_sym;
+  if (up.tensor) return ihc_tensor_launch(A, d_v, n_tiles, up.exp_b, st);
 
   CUtensorMap map;
   auto encode = get_encode();
