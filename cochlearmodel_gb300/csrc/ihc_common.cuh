@@ -80,6 +80,30 @@ struct Dot2 {
   __device__ __forceinline__ float result() const { return __fadd_rn(s, c); }
 };
 
+// Dot2 on two independent sums at once (two-wide FP32); each element
+// performs exactly the scalar Dot2 sequence.
+struct Dot2x2 {
+  float2 s, c;
+  __device__ __forceinline__ void init() { s = c = f2b(0.0f); }
+  __device__ __forceinline__ void add(float2 b, float2 x) {
+    const float2 p = mul2(b, x);
+    const float2 q = fma2(b, x, neg2(p));
+    const float2 t = add2(s, p);
+    const float2 z = sub2(t, s);
+    const float2 e = add2(sub2(s, sub2(t, z)), sub2(p, z));
+    s = t;
+    c = add2(c, add2(e, q));
+  }
+  __device__ __forceinline__ void add_pair(float2 b, float2 x1, float2 x2) {
+    const float2 sg = add2(x1, x2);
+    const float2 zz = sub2(sg, x1);
+    const float2 ep = add2(sub2(x1, sub2(sg, zz)), sub2(x2, zz));
+    add(b, sg);
+    c = fma2(b, ep, c);
+  }
+  __device__ __forceinline__ float2 result() const { return add2(s, c); }
+};
+
 // s + c += x exactly (Knuth's TwoSum; the rounding error goes to c).
 __device__ __forceinline__ void two_sum_add(float& s, float& c, float x) {
   const float t = __fadd_rn(s, x);

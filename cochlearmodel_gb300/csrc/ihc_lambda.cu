@@ -53,30 +53,6 @@ constexpr int kTilesPerRun = 8;  // consecutive tiles per CTA (short runs)
 // wait runs out with nothing in flight and the kernel reports status bit 1.
 int g_fault_skip_copy = 0;
 
-// Dot2 on two independent sums at once (two-wide FP32); each element
-// performs exactly the scalar Dot2 sequence.
-struct Dot2x2 {
-  float2 s, c;
-  __device__ __forceinline__ void init() { s = c = f2b(0.0f); }
-  __device__ __forceinline__ void add(float2 b, float2 x) {
-    const float2 p = mul2(b, x);
-    const float2 q = fma2(b, x, neg2(p));
-    const float2 t = add2(s, p);
-    const float2 z = sub2(t, s);
-    const float2 e = add2(sub2(s, sub2(t, z)), sub2(p, z));
-    s = t;
-    c = add2(c, add2(e, q));
-  }
-  __device__ __forceinline__ void add_pair(float2 b, float2 x1, float2 x2) {
-    const float2 sg = add2(x1, x2);
-    const float2 zz = sub2(sg, x1);
-    const float2 ep = add2(sub2(x1, sub2(sg, zz)), sub2(x2, zz));
-    add(b, sg);
-    c = fma2(b, ep, c);
-  }
-  __device__ __forceinline__ float2 result() const { return add2(s, c); }
-};
-
 // FIR of one 8-row block, rows kb..kb+7 all using `taps` taps.  src points at
 // the staged row of output kb (lane's column); rows above it are older.  One
 // shared-memory load feeds the eight rows' accumulators.  Rows r and r+4 form

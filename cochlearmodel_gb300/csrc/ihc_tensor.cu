@@ -23,6 +23,17 @@
 // grows from nothing by orders of magnitude within a tile; up to 6,000 of its points
 // go to Dot2.
 //
+// Some inputs leave nearly all points in doubt for long: tones in a null of the filter (a
+// sum 2^-20 of its partial sums), a stop band of 100 dB, values below the digits' range.
+// A tile of 128 rows then costs what it costs on the FP32 pipe, and the products' part in
+// vain: such tiles are told from the start of a segment by their last rows, and after two
+// of them the next are taken without products, eight rows to a warp (ac_blocks), while
+// half of the warps finish the tile before.  100,000 rows of a 2 kHz tone, which the 255
+// taps have a null at: row by row 4.25 ms, so 2.63 (FP32 kernel 2.41); a Blackman window,
+// 4 kHz 4.18 -> 2.61 (2.39); 60,000 rows below 2^-80 2.90 -> 1.73 (1.60).  At once after
+// the first such tile: 2.60 and 0.90 instead of 0.86 for 125 Hz; none finished before the
+// next is begun: 2.73 and 0.84.
+//
 // One CTA: 64 sections x a run of tiles of one frame.  Sixteen warps hold the
 // tile's 384 rows of velocity in registers (48 values a thread) and write one
 // digit after another into two shared-memory halves; a seventeenth issues the
@@ -67,6 +78,8 @@ constexpr int kPitch = kCols + 1;          // a row of dS / AC: lanes along rows
 constexpr int kGroups = kCols / 32;        // section halves
 constexpr int kList = 1024;                // points for Dot2 listed by tile
 constexpr int kFewPoints = 48;             // up to here a warp to a point
+constexpr int kLate = 256;                 // of the last 32 rows, from which more will follow
+constexpr int kDirectTiles = 15;           // tiles without products before they are tried again
 constexpr int kRuns = 16;                  // runs of 24 rows of a tile's x
 
 // A warp's scratch for one point (sym_point).
@@ -82,8 +95,10 @@ struct TensorShared {
   uint64_t drained;          // all products that were issued are done
   uint32_t tmem;
   int abort;                 // a wait ran out
+  int stop;                  // the workers have issued their last digit
   float floor;               // least slack, in units of the accumulators
   int listed;                // points for Dot2 (more than kList: those flagged)
+  int late;                  // those in the tile's last 32 rows
   int dot2_rows[2];          // rows for Dot2, by tile parity
   int kmin[2];               // first row of x of the tile, by tile parity
   uint32_t top[2][kCols];    // largest |x| bits of the tile, by tile parity
@@ -114,14 +129,15 @@ __device__ __forceinline__ void half_ready(TensorShared& S, int h, int lane) {
   __syncwarp();
   if (lane == 0) mbar_arrive(&S.ready[h]);
 }
-// The issuing warp, converged: phase `n` of ready[h]; false where a wait of the
-// workers, or this one, ran out.
+// The issuing warp, converged: phase `n` of ready[h]; false where there is none, or a
+// wait of the workers, or this one, ran out.
 __device__ __forceinline__ bool half_wait(TensorShared& S, int h, int n) {
   const unsigned long long start = global_ns();
   while (!__all_sync(kFull, mbar_done(&S.ready[h], n))) {
     // (the workers' steps between two digits are far shorter, their waits a fourth)
     const bool late = global_ns() - start > 4 * kWaitNs;
-    if (__any_sync(kFull, late || *(volatile int*)&S.abort)) return false;
+    if (__any_sync(kFull, late || *(volatile int*)&S.abort || *(volatile int*)&S.stop))
+      return false;
   }
   return true;
 }
@@ -364,6 +380,111 @@ __device__ __forceinline__ float dot2_row(const float* __restrict__ src,
   return acc.result();
 }
 
+// Dot2 of eight rows with all n taps each, in the orders of dot2_row, a section to a
+// lane; src points at the first row.  Rows r and r + 4 form pair r (fir_block8 and
+// fir_block8_sym of ihc_lambda.cu); the rows of the next four taps are fetched while
+// four are added, since they come from L2.  The rows read lie in [0, 7] and, of the
+// older ones, not past the last tap's.
+__device__ __forceinline__ void dot2_block8(const float* __restrict__ src, const float* TP, int n,
+                                         bool sym, float (&out)[8]) {
+  constexpr int kAhead = 4;
+  Dot2x2 acc[4];
+  float2 W[4];
+  const float* older = src - 256;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    acc[j].init();
+    W[j] = f2(__ldg(src + j * 256), __ldg(src + (j + 4) * 256));
+  }
+  auto shift = [&](float u) {
+    const float last = W[3].x;
+    W[3] = W[2];
+    W[2] = W[1];
+    W[1] = W[0];
+    W[0] = f2(u, last);
+  };
+  if (sym) {
+    const float* far = src - (n - 1) * 256;
+    float2 V[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) V[j] = f2(__ldg(far + j * 256), __ldg(far + (j + 4) * 256));
+    far += 8 * 256;
+    const int half = n / 2;
+    float u[kAhead], w[kAhead];
+    auto fetch = [&](int k) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        u[i] = __ldg(older - (k + i) * 256);
+        w[i] = __ldg(far + (k + i) * 256);
+      }
+    };
+    auto step = [&](int k, float un, float wn) {
+      const float2 bk = f2b(TP[k]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j].add_pair(bk, W[j], V[j]);
+      shift(un);
+      const float next = V[0].y;
+      V[0] = V[1];
+      V[1] = V[2];
+      V[2] = V[3];
+      V[3] = f2(next, wn);
+    };
+    // (the last fetch reaches rows -half - 4 and half + 12 - n)
+    static_assert(kTensorMinTaps / 2 >= 5, "rows fetched ahead stay inside the window");
+    fetch(0);
+    int k = 0;
+#pragma unroll 1
+    for (; k + kAhead <= half; k += kAhead) {
+      float un[kAhead], wn[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        un[i] = u[i];
+        wn[i] = w[i];
+      }
+      fetch(k + kAhead);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) step(k + i, un[i], wn[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead - 1; ++i)
+      if (k + i < half) step(k + i, u[i], w[i]);
+    if (n & 1) {
+      const float2 bc = f2b(TP[half]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j].add(bc, W[j]);
+    }
+  } else {
+    float u[kAhead];
+    auto fetch = [&](int k) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) u[i] = __ldg(older - min(k + i, n - 2) * 256);
+    };
+    fetch(0);
+#pragma unroll 1
+    for (int k = 0; k < n; k += kAhead) {
+      float un[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) un[i] = u[i];
+      fetch(k + kAhead);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        if (k + i < n) {
+          const float2 b = f2b(TP[k + i]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[j].add(b, W[j]);
+        }
+        shift(un[i]);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 r = acc[j].result();
+    out[j] = r.x;
+    out[j + 4] = r.y;
+  }
+}
+
 // Adds N values to s + c by TwoSum, in order: the chain of rounded sums first,
 // then their errors, which do not depend on each other, then the chain of those.
 template <int N>
@@ -426,6 +547,48 @@ __device__ __forceinline__ void window_sum(const float* col, int i, int taps, in
   wc = c;
 }
 
+// Dot2 of a tile's rows (first frame row kb, before k_hi), a warp to eight rows and 32
+// sections: of all, whose AC goes to ac[row][kPitch], or of those with a point in doubt and
+// those that the products cannot give.  Eight rows with all taps together take 18k cycles
+// of the FP32 pipe; a row for itself fetches its window from L2, which takes longer than
+// its sums.  v: the frame's row 0 at the lane's section, col: that section's column.
+// (Not inline: the loop over the tiles has no registers to spare.)
+__device__ __noinline__ void ac_blocks(const TensorShared& S, const float* __restrict__ v,
+                                       const cgb_ihc_frame& f, const float* TP, int n_ac,
+                                       bool sym, int kb, int k_lo, int k_hi, bool all, int warp,
+                                       float* ac, int col) {
+  const int sg = warp & 1, gw = warp >> 1;
+#pragma unroll 1
+  for (int r0 = 8 * gw; r0 < tfir::kRows; r0 += 64) {
+    const int k0 = kb + r0;
+    uint32_t rows = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = r0 + i;
+      if (k0 + i >= k_lo && k0 + i < k_hi &&
+          (all || S.row[r] == kRowDot2 ||
+           *reinterpret_cast<const uint32_t*>(&S.flag[r][4 * sg]) != 0))
+        rows |= 1u << i;
+    }
+    const float* src = v + (int64_t)k0 * 256;
+    const int sgm = k0 < f.frdp - 1 ? f.seg : f.total, lim = (k0 + 1) % sgm;
+    const bool full = k0 + 8 <= k_hi && lim >= n_ac && lim + 7 < sgm &&
+                      (k0 + 8 <= f.frdp - 1 || k0 >= f.frdp - 1);
+    if (full && __popc(rows) >= 5) {
+      float y[8];
+      dot2_block8(src, TP, n_ac, sym, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ac[(r0 + i) * kPitch + col] = y[i];
+    } else {
+      for (; rows; rows &= rows - 1) {
+        const int i = __ffs(rows) - 1;
+        ac[(r0 + i) * kPitch + col] =
+            dot2_row(src + i * 256, TP, taps_used(k0 + i, f, n_ac), n_ac, sym);
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
     ihc_tensor_kernel(const IHCArgs A, const float* __restrict__ v, int exp_b) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -466,8 +629,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     mbar_init(&S.drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    S.abort = 0;
-    S.listed = 0;
+    S.abort = S.stop = 0;
+    S.listed = S.late = 0;
     S.dot2_rows[0] = S.dot2_rows[1] = 0;
   }
   if (threadIdx.x < 2 * kCols) (&S.top[0][0])[threadIdx.x] = 0;
@@ -513,15 +676,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kIhcWarps) {
     // the issuing warp
     const uint32_t issue = tfir::elected();
-    int n = 0;  // digits so far
-    for (int t = first; t < t1; ++t) {
+    for (int n = 0;;) {  // digits so far
       for (int i = 0; i < tfir::kDigits; ++i, ++n) {
         for (int h = 0; h < 2; ++h) {
           if (!half_wait(S, h, n)) goto done;
           tfir::fence_after();
           // (test-only: the first half's products are left out, so that the
           // wait for them runs out)
-          if (A.skip_first_copy && t == first && i == 0 && h == 0) continue;
+          if (A.skip_first_copy && n == 0 && h == 0) continue;
           tfir::products(smem_u32(AD), smem_u32(XD) + h * tfir::kHalfBytes, tmem, i, h, issue);
           if (issue) tfir::commit(&S.mbar[h]);
           __syncwarp();
@@ -553,9 +715,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (tu == 0) tu = taps_used(++k, f, n_ac);
       return k - tu + 1;
     };
+    // (rows that the DC filter does not look back on count as rows without taps)
+    const int needed = t0 * tfir::kRows - (n_dc - 1);
     auto classify = [&](int t, int r) {
       const int k = t * tfir::kRows + r;
-      const int tu = k < f.lam_rows ? taps_used(k, f, n_ac) : 0;
+      const int tu = k >= needed && k < f.lam_rows ? taps_used(k, f, n_ac) : 0;
       const int kmin = window_start(t * tfir::kRows);
       const bool fits = (tu == n_ac && k - n_ac + 1 >= kmin) || k - tu + 1 == kmin;
       S.row[r] = tu == 0 ? kRowZero : (fits ? kRowSum : kRowDot2);
@@ -585,6 +749,15 @@ __global__ void __launch_bounds__(kThreads, 1)
               x[h][g][c] = top - c >= kmin && top - c < kmax ? __ldg(row - c * 256) : 0.0f;
           }
         }
+    };
+    // (its registers are free)
+    auto clear_tile = [&]() {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int g = 0; g < 3; ++g)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) x[h][g][c] = 0.0f;
     };
     // The sums of the tile's last and first row over this thread's two runs of
     // 24 rows, in tap order, with their largest partial sums.
@@ -655,11 +828,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       put_digit(1, 512.0f);
     };
 
+    // AC and dS of row r and section c of the tile.  at: ring row of its first dS row.
+    auto store_point = [&](int at, int r, int c, float ac, float own) {
+      const float ms = __fmaf_rn(own, A.scale, -ac);
+      int slot = at + r;
+      slot -= slot >= ring ? ring : 0;
+      AC[r * kPitch + c] = ac;
+      DS[slot * kPitch + c] = __fmul_rn(ms, ms);
+    };
+    auto blocks = [&](int t, bool all, float* ac) {
+      ac_blocks(S, vf + sec, f, TP, n_ac, A.ac_sym != 0, t * tfir::kRows, needed,
+                min((t + 1) * tfir::kRows, f.lam_rows), all, warp, ac, sec);
+    };
+    // AC and dS of a tile from its AC.
+    auto take_blocks = [&](int t, int at, const float* ac) {
+      const int kb = t * tfir::kRows, rows = min(tfir::kRows, f.lam_rows - kb);
+      for (int r = gw; r < rows; r += 8)
+        store_point(at, r, sec, ac[r * kPitch + sec], __ldg(vf + (int64_t)(kb + r) * 256 + sec));
+    };
     // The steps that finish a tile, each between two barriers of the workers.
-    // at: ring row of the tile's first dS row.
     auto dot2_points = [&](int t, int at) {
       const int listed = S.listed, kb = t * tfir::kRows;
-      const bool all = listed > kList;
       if (listed <= kFewPoints) {
         // Few points: a warp to each, whose lanes fetch the point's rows and the
         // taps at once (one trip to L2 where a lane's own sequence of batches
@@ -697,19 +886,14 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
           }
           const float ac = acc.result();
-          const float ms = __fmaf_rn(own, A.scale, -ac);
-          int slot = at + r;
-          slot -= slot >= ring ? ring : 0;
-          if (lane == 0) {
-            AC[r * kPitch + c] = ac;
-            DS[slot * kPitch + c] = __fmul_rn(ms, ms);
-          }
+          if (lane == 0) store_point(at, r, c, ac, own);
         }
       }
       // first the rows that the products cannot give, and of more points than the
       // list holds the rows with any, a warp to 32 sections;
       // then single points, as few warps as hold them (what a warp's sequence
       // costs does not depend on its lanes), from the highest warp down
+      const bool all = listed > kList;
       int row = all || S.dot2_rows[t & 1] ? gw : tfir::kRows;
       int p = (kIhcWarps - 1 - warp) * 32 + lane;
       while (true) {
@@ -729,13 +913,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           p += kWorkers;
         }
         const float* src = vf + (int64_t)(kb + r) * 256 + c;
-        const float ac =
-            dot2_row(src, TP, taps_used(kb + r, f, n_ac), n_ac, A.ac_sym != 0);
-        const float ms = __fmaf_rn(__ldg(src), A.scale, -ac);
-        int slot = at + r;
-        slot -= slot >= ring ? ring : 0;
-        AC[r * kPitch + c] = ac;
-        DS[slot * kPitch + c] = __fmul_rn(ms, ms);
+        store_point(at, r, c,
+                    dot2_row(src, TP, taps_used(kb + r, f, n_ac), n_ac, A.ac_sym != 0),
+                    __ldg(src));
       }
     };
     // DC sums of ihc_lambda.cu's kernel: a warp per 32 rows and section half
@@ -820,13 +1000,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         now = now + 1 == ring ? 0 : now + 1;
       }
     };
-    auto emit = [&](int t, int from, int to) {
+    // kEmitRows rows each from `from` on, `step` apart, before `to`
+    auto emit = [&](int t, int from, int to, int step) {
       const int row0 = t * tfir::kRows, k_hi = min(row0 + to, f.lam_rows);
       const float dmg = __ldg(A.dmg + (size_t)f.ihc_profile * 256 + s0 + sec);
       const float a0 = __ldg(A.aihc + s0 + sec), a1 = __ldg(A.aihc + 256 + s0 + sec),
                   a2 = __ldg(A.aihc + 512 + s0 + sec);
       const bool sec0 = s0 + sec == 0;
-      for (int kb = row0 + from + gw * kEmitRows; kb < k_hi; kb += 8 * kEmitRows) {
+      for (int kb = row0 + from; kb < k_hi; kb += step) {
         float lg[kEmitRows], l0[kEmitRows], l1[kEmitRows], l2[kEmitRows];
 #pragma unroll
         for (int r = 0; r < kEmitRows; r += 2) {
@@ -871,7 +1052,62 @@ __global__ void __launch_bounds__(kThreads, 1)
     int n = 0;       // completed phases of each half's barrier
     int at = 0;      // ring row of the tile's first dS row
     int at_prev = 0; // and of the tile before
-    for (int t = first; t < t1; ++t, n += tfir::kDigits) {
+    bool pending = false;  // the tile before is to be finished
+    // A tile with more points in doubt than the list holds, also among its last rows (at
+    // the start of a segment only the first rows have them) is finished before the next
+    // is begun; after two the next tiles take Dot2 for all points: three, then more each
+    // time.
+    auto crowded = [&]() { return S.listed > kList && S.late > kLate; };
+    bool before = false;  // the last tile with products was such a one
+    int direct = 0, next_direct = 0;
+    for (int t = first;; ++t) {
+      if (direct > 0 || t == t1 || (pending && crowded())) {
+        clear_tile();
+        if (pending) {
+          if (S.listed > kList) {
+            blocks(t - 1, false, AC);
+            sync_workers();
+            take_blocks(t - 1, at_prev, AC);
+          } else {
+            dot2_points(t - 1, at_prev);
+          }
+          sync_workers();
+        }
+        // A tile without products: the FP32 pipe is busy with its sums while half of the
+        // warps first finish the tile before, 32 rows each.
+        const bool own = direct > 0 && t < t1;
+        float* const all = reinterpret_cast<float*>(XD);
+        static_assert(tfir::kRows * kPitch * 4 <= 2 * tfir::kHalfBytes, "AC in the digits' place");
+        if (pending && t > t0) {
+          dc_sums(t - 1, at_prev);
+          if (!own) sync_workers();
+          if (!own || warp < 4 * kGroups)
+            emit(t - 1, own ? kDcAnchor * gw : kEmitRows * gw,
+                 own ? kDcAnchor * (gw + 1) : tfir::kRows, own ? kEmitRows : 8 * kEmitRows);
+        }
+        if (own) blocks(t, true, all);
+        if (threadIdx.x == 0) {
+          S.listed = S.late = 0;
+          S.dot2_rows[t & 1] = S.dot2_rows[(t + 1) & 1] = 0;
+          S.kmin[(t + 1) & 1] = window_start((t + 1) * tfir::kRows);
+        }
+        if (t == t1) break;
+        if (own) {
+          if (warp < kGroups && gw == 0) S.top[(t + 1) & 1][sec] = 0;
+          sync_workers();
+          take_blocks(t, at, all);
+          if (--direct == 0 && t + 1 < t1) load_tile(t + 1);
+          sync_workers();
+          pending = true;
+          at_prev = at;
+          at += tfir::kRows;
+          at -= at >= ring ? ring : 0;
+          continue;
+        }
+        pending = false;
+        load_tile(t);
+        sync_workers();
+      }
       const int kb = t * tfir::kRows, k_hi = min(kb + tfir::kRows, f.lam_rows);
       // scales: the exponent of the section's largest |x| (a NaN is not seen
       // here: it makes every sum of its section a NaN, which Dot2 then replaces)
@@ -900,25 +1136,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         S.top[(t + 1) & 1][sec] = 0;
       }
       const float up = usable ? __int_as_float((127 + 8 - e) << 23) : 0.0f;
-      if (!usable) {  // (0 times an infinity is no digit)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int g = 0; g < 3; ++g)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) x[h][g][c] = 0.0f;
-      }
+      if (!usable) clear_tile();  // (0 times an infinity is no digit)
       put_digit(0, up);
       put_digit(1, up);
       if (warp >= 8 && warp < 12) sampled_partial((warp >> 1) & 1, 32 * (warp & 1) + lane);
       sync_workers();
       // the tile before, between the digits of this one
-      const bool prev = t > first, prev_out = t > t0;
-      if (prev) dot2_points(t - 1, at_prev);
+      const bool prev_out = pending && t > t0;
+      if (pending) dot2_points(t - 1, at_prev);
       next_digit(n);
       sync_workers();
       if (threadIdx.x == 0) {
-        S.listed = 0;
+        S.listed = S.late = 0;
         S.dot2_rows[(t + 1) & 1] = 0;
         S.kmin[(t + 1) & 1] = window_start((t + 1) * tfir::kRows);
       }
@@ -931,9 +1160,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         S.scale[sec].x += __fdiv_rn(__uint_as_float(S.partial[sec]) * 0x1.4p-43f, S.scale[sec].y);
         S.partial[sec] = 0;
       }
-      if (prev_out) emit(t - 1, 0, tfir::kRows / 2);
+      if (prev_out) emit(t - 1, gw * kEmitRows, tfir::kRows / 2, 8 * kEmitRows);
       next_digit(n + 2);
-      if (prev_out) emit(t - 1, tfir::kRows / 2, tfir::kRows);
+      if (prev_out)
+        emit(t - 1, tfir::kRows / 2 + gw * kEmitRows, tfir::kRows, 8 * kEmitRows);
       next_digit(n + 3);
       // the row's velocity, for dS
       const int row = (warp & 3) * 32 + lane, cols = (warp >> 2) * 16;
@@ -1001,6 +1231,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           S.flag[row][c0 >> 3] = (unsigned char)bad;
           if (bad) {
             int p = atomicAdd(&S.listed, __popc(bad));
+            if ((warp & 3) == 3) atomicAdd(&S.late, __popc(bad));
 #pragma unroll
             for (int c = 0; c < 8; ++c)
               if (bad >> c & 1) {
@@ -1020,14 +1251,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (threadIdx.x == 0) atomicOr(A.status, 1);
         break;
       }
+      pending = true;
+      n += tfir::kDigits;
+      const bool now = crowded();
+      next_direct = now && before ? min(2 * next_direct + 3, kDirectTiles) : 0;
+      direct = next_direct;
+      before = now;
     }
-    if (!*(volatile int*)&S.abort) {
-      dot2_points(t1 - 1, at_prev);
-      sync_workers();
-      dc_sums(t1 - 1, at_prev);
-      sync_workers();
-      emit(t1 - 1, 0, tfir::kRows);
-    }
+    if (threadIdx.x == 0) *(volatile int*)&S.stop = 1;
   }
   __syncthreads();
   if (warp == kIhcWarps) tfir::tmem_free(tmem);
