@@ -545,6 +545,47 @@ int pick_run(const cgb_ihc_frame* frames, int n_frames, int TR, int n_dc) {
   return kTilesPerRun;
 }
 
+// Whether the tensor kernel is the faster one for these frames.  It takes whole tiles of
+// 128 rows, rows or not, at the same time for all of its filters, and evaluates the rows
+// behind a segment's end inside a tile one by one; the FP32 kernel's time goes with the
+// rows and their taps, and its CTAs have half as many sections, which counts while the
+// chip is not full.  Times in us of an SM for 64 sections, fitted to (FP32 / tensor, us)
+//   600 frames of 100 rows, 64 taps: 614 / 650, 255 taps: 740 / 650; 2,400 of 25: 1,381 /
+//   2,260; 200 of 300: 450 / 557, 1,204 / 601; 60 of 1,000: 523 / 455, 1,412 / 481; 3 of
+//   100: 35 / 54; one of 30: 25 / 49; one of 60,000 in segments of 50 (255 taps): 435 / 755,
+//   100: 696 / 846, 200: 1,122 / 792; 2.9 million rows, 64 taps: 19,200 / 17,100.
+bool tensor_faster(const cgb_ihc_frame* frames, int n_frames, int n_ac, int n_dc, int TR,
+                   int run, int tensor_run) {
+  const double back = (n_dc - 1 + kTensorTileRows - 1) / kTensorTileRows;
+  double all = 0.0, all_t = 0.0, one = 0.0, one_t = 0.0;  // of all CTAs, of the longest
+  double ctas = 0.0, ctas_t = 0.0;
+  for (int i = 0; i < n_frames; ++i) {
+    const cgb_ihc_frame& f = frames[i];
+    if (f.lam_rows <= 0 || f.seg <= 0) continue;
+    const double rows = f.lam_rows, len = std::min(f.seg, f.lam_rows), segs = rows / len;
+    const double part = std::min(len, (double)n_ac);  // rows of a segment with fewer taps
+    const double row = 0.075 + (4.5e-3 * part * part / 2 + 2.75e-3 * n_ac * (len - part)) / len;
+    const double runs = std::ceil(rows / ((double)run * TR));
+    ctas += runs * (256 / kSecTile);
+    all += 21.0 * runs + row * rows;
+    one = std::max(one, 21.0 + row * std::min(rows, (double)run * TR + (runs > 1 ? n_dc : 0)));
+    const double tiles = std::ceil(rows / kTensorTileRows);
+    const double runs_t = std::ceil(tiles / tensor_run);
+    const double cut = f.seg % kTensorTileRows ? std::min(len, kTensorTileRows / 2.0) : 0.0;
+    const double tile = 27.0 + 5e-3 * (segs - 1) / tiles * cut * cut;
+    ctas_t += runs_t * (256 / kTensorSections);
+    all_t += 14.0 * runs_t + tile * (tiles + (runs_t - 1) * back);
+    one_t = std::max(one_t, 14.0 + tile * (std::min(tiles, (double)tensor_run) +
+                                           (runs_t > 1 ? back : 0)));
+  }
+  const double sms = std::max(1, sm_count());
+  // few CTAs go in whole waves
+  auto time = [&](double total, double longest, double n) {
+    return n <= 4 * sms ? std::ceil(n / sms) * longest : std::max(4 * total / sms, longest);
+  };
+  return 1.05 * time(all_t, one_t, ctas_t) < time(all, one / 2, ctas);
+}
+
 }  // namespace
 }  // namespace cgb
 
@@ -607,23 +648,26 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   int TR = 0, xrows = 0;
   pick_tile(n_ac, n_dc, &TR, &xrows);
   if (TR < 32) return fail(CGB_ERR_RANGE, "cgb_ihc_lambda_dev: filters too long for one tile");
-  int dc_uniform = 1;
-  for (int i = 1; i < n_dc; ++i) dc_uniform &= dc_taps[i] == dc_taps[0];
-  // The AC filter goes to the tensor cores where the kernel is built for it: a
-  // uniform DC filter, no debug stage, no AC given, lengths that fit.
-  int exp_b = 0;
-  const bool tensor = !ac_ext && stage == 0 && dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
-                      tensor_taps(ac_taps, n_ac, prm->scale, &exp_b);
-  Uploaded up{n_frames, n_ac, n_dc, 0,
-              tensor ? pick_tensor_run(frames, n_frames, n_dc)
-                     : pick_run(frames, n_frames, TR, n_dc),
-              tensor, exp_b, ac_symmetric(ac_taps, n_ac, prm->scale), dc_uniform};
+  Uploaded up{};
   bool known = false;
   if (!(mode & kUpload)) {
     std::lock_guard<std::mutex> lock(g_uploaded_mu);
     const auto it = g_uploaded.find(d_scratch);
     known = it != g_uploaded.end();
     if (known) up = it->second;
+  }
+  if (!known) {
+    up = {n_frames, n_ac, n_dc, 0, pick_run(frames, n_frames, TR, n_dc), false, 0,
+          ac_symmetric(ac_taps, n_ac, prm->scale), 1};
+    for (int i = 1; i < n_dc; ++i) up.dc_uniform &= dc_taps[i] == dc_taps[0];
+    // The AC filter goes to the tensor cores where the kernel is built for it (a uniform DC
+    // filter, no debug stage, no AC given, lengths that fit) and the faster one.
+    if (!ac_ext && stage == 0 && up.dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
+        tensor_taps(ac_taps, n_ac, prm->scale, &up.exp_b)) {
+      const int run = pick_tensor_run(frames, n_frames, n_dc);
+      up.tensor = tensor_faster(frames, n_frames, n_ac, n_dc, TR, up.run, run);
+      if (up.tensor) up.run = run;
+    }
   }
   if (up.n_ac != n_ac || up.n_dc != n_dc)
     return fail(CGB_ERR_ARG, "cgb_ihc_lambda_launch_dev: not the filters that were uploaded");

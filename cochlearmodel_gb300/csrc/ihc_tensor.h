@@ -7,7 +7,8 @@
 
 namespace cgb {
 
-// Shorter filters stay on the FP32 pipe: a tile costs about the same for any length.
+// Shorter filters stay on the FP32 pipe: a tile costs about the same for any length (and
+// frames of few rows, tensor_faster of ihc_lambda.cu).
 // JND sweep, FP32 against tensor cores: 32 taps 13.3 / 17.0 ms, 48 16.2 / 17.0, 64
 // 19.2 / 17.1, 128 31.2 / 18.1; 286,000 rows: 48 taps 1.93 / 1.94, 64 2.28 / 1.98.
 constexpr int kTensorMinTaps = 64;
