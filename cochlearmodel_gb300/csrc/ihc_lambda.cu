@@ -475,7 +475,7 @@ struct Uploaded {
   int n_tiles;  // runs of tiles of all frames
   int run;
   bool tensor;
-  int exp_b;  // for the tensor kernel
+  TensorTaps taps;
   int ac_sym, dc_uniform;
 };
 std::mutex g_uploaded_mu;
@@ -513,20 +513,6 @@ int pick_tensor_run(const cgb_ihc_frame* frames, int n_frames, int n_dc) {
     }
   }
   return best;
-}
-
-// The exponent of the largest AC tap (scaled, as the kernels use them), for the
-// tensor kernel.  False: none that it can use.
-bool tensor_taps(const float* ac_taps, int n_ac, float scale, int* exp_b) {
-  float top = 0.0f;
-  for (int i = 0; i < n_ac; ++i) {
-    const float b = ac_taps[i] * scale;
-    if (!std::isfinite(b)) return false;
-    top = std::max(top, std::fabs(b));
-  }
-  if (!(top > 0.0f)) return false;
-  std::frexp(top, exp_b);
-  return *exp_b >= -16 && *exp_b <= 16;
 }
 
 int pick_run(const cgb_ihc_frame* frames, int n_frames, int TR, int n_dc) {
@@ -657,13 +643,13 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
     if (known) up = it->second;
   }
   if (!known) {
-    up = {n_frames, n_ac, n_dc, 0, pick_run(frames, n_frames, TR, n_dc), false, 0,
+    up = {n_frames, n_ac, n_dc, 0, pick_run(frames, n_frames, TR, n_dc), false, {},
           ac_symmetric(ac_taps, n_ac, prm->scale), 1};
     for (int i = 1; i < n_dc; ++i) up.dc_uniform &= dc_taps[i] == dc_taps[0];
     // The AC filter goes to the tensor cores where the kernel is built for it (a uniform DC
     // filter, no debug stage, no AC given, lengths that fit) and the faster one.
     if (!ac_ext && stage == 0 && up.dc_uniform && ihc_tensor_fits(n_ac, n_dc) &&
-        tensor_taps(ac_taps, n_ac, prm->scale, &up.exp_b)) {
+        ihc_tensor_taps(ac_taps, n_ac, prm->scale, &up.taps)) {
       const int run = pick_tensor_run(frames, n_frames, n_dc);
       up.tensor = tensor_faster(frames, n_frames, n_ac, n_dc, TR, up.run, run);
       if (up.tensor) up.run = run;
@@ -751,7 +737,7 @@ int ihc_lambda_impl(const float* d_v, int64_t v_rows, const cgb_ihc_frame* frame
   A.run = up.run;
   A.dc_uniform = up.dc_uniform;
   A.ac_sym = up.ac_sym;
-  if (up.tensor) return ihc_tensor_launch(A, d_v, n_tiles, up.exp_b, st);
+  if (up.tensor) return ihc_tensor_launch(A, d_v, n_tiles, up.taps, st);
 
   CUtensorMap map;
   auto encode = get_encode();

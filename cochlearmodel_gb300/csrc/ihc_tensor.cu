@@ -17,11 +17,16 @@
 // 40 x 2^-48 of that bound, about twice the partial sum itself; where it makes a
 // difference, and in rows whose look-back is shorter than the tile's, the point
 // is evaluated by Dot2.  On the JND sweep 39% of the tiles have no such point,
-// 48% one to eight of 8,192.  Not below a floor, what the five digits leave of x and
-// of the taps (six standard deviations, from the taps): it decides where a section's
-// sums are tiny beside its largest |x|, as at the start of a segment, whose velocity
-// grows from nothing by orders of magnitude within a tile; up to 6,000 of its points
-// go to Dot2.
+// 48% one to eight of 8,192.  (The 59 is measured, not proven: a point past it would be
+// the exact sum's rounding where Dot2's is the other neighbour of a tie.)
+//
+// Not below a floor, which bounds the error of the digits' sum (ihc_tensor_taps): what the
+// digits leave of x and of the taps, and the pairs left out.  It decides where a section's
+// sums are tiny beside its largest |x|, as at the start of a segment, whose velocity grows
+// from nothing by orders of magnitude within a tile.  (Five digits of x, and six standard
+// deviations of what they leave: steady values of 2^-22 of the tile's largest came out as
+// the other neighbour.  Five digits and the bound of what they leave: 33 intervals
+// 1.41 -> 1.54 ms, with the remainders' own maximum 1.50; six digits 1.43.)
 //
 // Some inputs leave nearly all points in doubt for long: tones in a null of the filter (a
 // sum 2^-20 of its partial sums), a stop band of 100 dB, values below the digits' range.
@@ -51,12 +56,14 @@
 // rows of the tile: one signal 304 -> 262 us, 33 intervals 1.46 -> 1.44 ms.
 //
 // Measured (GB300), against the FP32 pipe: JND sweep (2.9 million rows) 53.7 ->
-// 17.8 ms, 176,000 rows in 33 intervals 4.46 -> 1.44 ms, one signal of 5,330 rows
+// 18.0 ms, 176,000 rows in 33 intervals 4.46 -> 1.43 ms, one signal of 5,330 rows
 // 0.80 -> 0.26 ms.
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstddef>
+#include <limits>
 
 #include "cgb_device.cuh"
 #include "cgb_internal.h"
@@ -96,7 +103,6 @@ struct TensorShared {
   uint32_t tmem;
   int abort;                 // a wait ran out
   int stop;                  // the workers have issued their last digit
-  float floor;               // least slack, in units of the accumulators
   int listed;                // points for Dot2 (more than kList: those flagged)
   int late;                  // those in the tile's last 32 rows
   int dot2_rows[2];          // rows for Dot2, by tile parity
@@ -590,7 +596,8 @@ __device__ __noinline__ void ac_blocks(const TensorShared& S, const float* __res
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-    ihc_tensor_kernel(const IHCArgs A, const float* __restrict__ v, int exp_b) {
+    ihc_tensor_kernel(const IHCArgs A, const float* __restrict__ v,
+                      const TensorTaps taps) {
   extern __shared__ __align__(128) unsigned char smem[];
   // layout: digits of x, two halves | band of the taps | dS, a ring of n_dc + 128
   // rows | AC [128] | taps with 128 zeros before and zeros up to 384 | TensorShared
@@ -643,22 +650,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     TP[i] = b;
     if (i < 0 || i >= n_ac) continue;
     float r = b;
-    float up = __int_as_float((127 + 8 - exp_b) << 23);
+    float up = __int_as_float((127 + 8 - taps.exp_b) << 23);
     for (int j = 0; j < tfir::kDigits; ++j) {
       td[j * n_ac + i] = (uint16_t)(__float_as_uint(tfir::digit(r, up)) >> 16);
       up = 512.0f;
     }
   }
   __syncthreads();
-  if (warp == kIhcWarps) {
-    // The remainders of x behind its last digit, at most 2^(e-45) and 2^(e-45.8) rms,
-    // times the taps: six standard deviations of their sum.
-    float sq = 0.0f;
-    for (int i = lane; i < n_ac; i += 32) sq += TP[i] * TP[i];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) sq += __shfl_xor_sync(kFull, sq, o);
-    if (lane == 0) S.floor = 0x1p-27f * sqrtf(sq) * __int_as_float((127 - exp_b) << 23);
-  }
   for (int e = threadIdx.x; e < tfir::kDigits * tfir::kCores * 64; e += kThreads) {
     const int j = e / (tfir::kCores * 64), q = e - j * (tfir::kCores * 64);
     const int i = 8 * (q >> 6) + ((q >> 3) & 7) + (q & 7) - (tfir::kRows - 1);
@@ -677,7 +675,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // the issuing warp
     const uint32_t issue = tfir::elected();
     for (int n = 0;;) {  // digits so far
-      for (int i = 0; i < tfir::kDigits; ++i, ++n) {
+      for (int i = 0; i < tfir::kRowDigits; ++i, ++n) {
         for (int h = 0; h < 2; ++h) {
           if (!half_wait(S, h, n)) goto done;
           tfir::fence_after();
@@ -1131,8 +1129,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool usable = e >= -80 && e <= 100;
       if (warp < kGroups && gw == 0) {
         S.scale[sec] =
-            make_float2(m == 0 ? 0.0f : (usable ? S.floor : __int_as_float(0x7f800000)),
-                        usable ? __int_as_float((127 + e + exp_b - 16) << 23) : 1.0f);
+            make_float2(m == 0 ? 0.0f : (usable ? taps.floor : __int_as_float(0x7f800000)),
+                        usable ? __int_as_float((127 + e + taps.exp_b - 16) << 23) : 1.0f);
         S.top[(t + 1) & 1][sec] = 0;
       }
       const float up = usable ? __int_as_float((127 + 8 - e) << 23) : 0.0f;
@@ -1175,8 +1173,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < 4; ++i)
           own[i] = kb + row < k_hi ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
-      wait_half(0, n + 4);
-      wait_half(1, n + 4);
+      next_digit(n + 4);
+      wait_half(0, n + 5);
+      wait_half(1, n + 5);
       sync_workers();
       tfir::fence_after();
 
@@ -1214,9 +1213,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             float2 ac = mul2(res, f2(sc.y, sc.w));
             const float2 up = add2(res, add2(rest, slack)), down = add2(res, sub2(rest, slack));
             const float least = 1e-30f;  // (far from where the unit's product would round)
-            if (!(up.x == res.x && down.x == res.x && (sc.x == 0.0f || fabsf(ac.x) > least)))
+            if (!(up.x == res.x && down.x == res.x && (sc.x == 0.0f || fabsf(ac.x) > least)) ||
+                fmaxf(fmaxf(fabsf(g[2].x), fabsf(g[3].x)), fabsf(g[4].x)) >= taps.limit)
               bad |= 1u << c;
-            if (!(up.y == res.y && down.y == res.y && (sc.z == 0.0f || fabsf(ac.y) > least)))
+            if (!(up.y == res.y && down.y == res.y && (sc.z == 0.0f || fabsf(ac.y) > least)) ||
+                fmaxf(fmaxf(fabsf(g[2].y), fabsf(g[3].y)), fabsf(g[4].y)) >= taps.limit)
               bad |= 2u << c;
             if (kind == kRowZero) ac = f2b(0.0f);
             const float4 o = own[2 * part + c / 4];
@@ -1252,7 +1253,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         break;
       }
       pending = true;
-      n += tfir::kDigits;
+      n += tfir::kRowDigits;
       const bool now = crowded();
       next_direct = now && before ? min(2 * next_direct + 3, kDirectTiles) : 0;
       direct = next_direct;
@@ -1277,13 +1278,61 @@ bool ihc_tensor_fits(int n_ac, int n_dc) {
          tensor_smem(n_dc) <= 227 * 1024;
 }
 
-int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b,
+bool ihc_tensor_taps(const float* taps, int n_ac, float scale, TensorTaps* out) {
+  float top = 0.0f;
+  for (int i = 0; i < n_ac; ++i) {
+    const float b = taps[i] * scale;
+    if (!std::isfinite(b)) return false;
+    top = std::fmax(top, std::fabs(b));
+  }
+  if (!(top > 0.0f)) return false;
+  std::frexp(top, &out->exp_b);
+  if (out->exp_b < -16 || out->exp_b > 16) return false;
+  // the digits as the kernel forms them (exactly), their sums and what they leave; in
+  // units of 2^exp_b
+  double S[tfir::kDigits] = {}, sum = 0.0, left = 0.0;
+  for (int i = 0; i < n_ac; ++i) {
+    double y = std::ldexp((double)(taps[i] * scale), 8 - out->exp_b);
+    sum += std::fabs(y) / 256;
+    for (int j = 0; j < tfir::kDigits; ++j) {
+      const double d = std::nearbyint(y);
+      S[j] += std::fabs(d);
+      y = (y - d) * 512;
+    }
+    left += std::ldexp(std::fabs(y), -8 - 9 * tfir::kDigits);
+  }
+  // M_m of tensor_fir.cuh: digit i of x is at most 256
+  double M[tfir::kSums];
+  for (int m = 0; m < tfir::kSums; ++m) {
+    M[m] = 0.0;
+    for (int j = 0; j < tfir::kDigits && j <= m; ++j) M[m] += 256 * S[j];
+  }
+  const double exact = 0x1p24;
+  const double most = std::fmax(M[2], std::fmax(M[3], M[4]));
+  // (with random digits the accumulators have a standard deviation of 2^19.5)
+  if (M[1] >= exact || most > 2 * exact - 0x1p22) return false;
+  // What an accumulator of partial sums up to M may lose: at most 17 addends in each of
+  // 18 steps of a digit pair, each cut to a multiple of 2^q.
+  auto lost = [&](int pairs, double m) {
+    const int q = m < exact ? 0 : (int)std::floor(std::log2(m / exact)) + 1;
+    return 17.0 * 18.0 * pairs * (std::ldexp(1.0, q) - 1.0);
+  };
+  out->limit = most < exact ? std::numeric_limits<float>::infinity()
+                            : (float)(2 * exact - most - lost(5, most));
+  out->floor = (float)(1.01 * (std::ldexp(sum, 16 - 54) + std::ldexp(left, 16) +
+                               std::ldexp(256 * (S[1] + S[2] + S[3] + S[4]), -54) +
+                               std::ldexp(lost(5, M[5]), -45) +
+                               0x1p-28));  // (and the rounding of g3 in the epilogue)
+  return true;
+}
+
+int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, const TensorTaps& taps,
                       cudaStream_t st) {
   const size_t smem = tensor_smem(A.n_dc);
   CGB_TRY_CUDA(cudaFuncSetAttribute(ihc_tensor_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "cudaFuncSetAttribute(ihc tensor smem)");
-  ihc_tensor_kernel<<<dim3((unsigned)n_runs, 256 / kCols), kThreads, smem, st>>>(A, d_v, exp_b);
+  ihc_tensor_kernel<<<dim3((unsigned)n_runs, 256 / kCols), kThreads, smem, st>>>(A, d_v, taps);
   CGB_TRY_CUDA(cudaGetLastError(), "ihc_tensor_kernel launch");
   note_launch();
   return CGB_OK;

@@ -17,8 +17,15 @@ constexpr int kTensorSections = 64;
 
 // Whether the filters' lengths fit the kernel (taps of one tile, shared memory).
 bool ihc_tensor_fits(int n_ac, int n_dc);
-// exp_b: the exponent of the largest |tap| (2^(exp_b-1) <= it < 2^exp_b).
-int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, int exp_b,
+// What the kernel takes from the AC taps (scaled, as they are uploaded).
+struct TensorTaps {
+  int exp_b;    // 2^(exp_b-1) <= largest |tap| < 2^exp_b
+  float floor;  // largest error of a sum, in units of the accumulators (head of ihc_tensor.cu)
+  float limit;  // of the third to fifth accumulator: exact below
+};
+// False: taps whose digit products the accumulators do not hold.
+bool ihc_tensor_taps(const float* taps, int n_ac, float scale, TensorTaps* out);
+int ihc_tensor_launch(const IHCArgs& A, const float* d_v, int n_runs, const TensorTaps& taps,
                       cudaStream_t st);
 
 }  // namespace cgb

@@ -3,16 +3,22 @@
 //
 // A tile is 128 output rows x 64 sections.  Its filter outputs are T x, T the
 // 128 x 384 band of the taps and x the 384 rows that end with the tile.  Both
-// factors are written as fixed-point numbers of five digits in base 2^9,
+// factors are written as fixed-point numbers in base 2^9, of six and five digits,
 //   x = 2^(e-8)  sum_i X_i 2^(-9 i),   b = 2^(eb-8) sum_j B_j 2^(-9 j),
 // |X_i|, |B_j| <= 256 (rounded to nearest, so signed), e and eb the exponents
 // of the largest magnitude of a section's 384 rows and of the taps.  Integers
-// up to 256 are exact in BF16, and the products of two digits summed over the
-// taps stay below 2^24, so the FP32 accumulators hold exact integers.  The 19
-// digit pairs with i + j <= 5 go to six accumulators G_m, m = i + j:
-//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  the digits' remainders (at most 2^(e-45)
+// up to 256 are exact in BF16.  The 20 digit pairs with i + j <= 5 go to six
+// accumulators G_m, m = i + j:
+//   T x = 2^(e+eb-16) sum_m G_m 2^(-9 m)  +  the digits' remainders (at most 2^(e-54)
 // of a value of x, 2^(eb-45) of a tap) and the pairs left out (about 2^-50 of the
 // product of the scales; 2^-41 with the 15 pairs up to i + j = 4).
+// An FP32 accumulator holds exact integers while no partial sum reaches 2^24.  A
+// partial sum of G_m is at most M_m = 256 (S_0 + .. + S_m), S_j the sum of |B_j| over
+// the taps.  The filter is taken only if that holds G_0 and G_1 (0.61 x 2^24 for the
+// default one); G_2 to G_4 (1.11, 1.46, 1.46) are told to be exact from their final values:
+// if a partial sum had reached 2^24, what is left of M_m could not bring the sum back
+// below 2^25 - M_m.  What G_5 may have lost counts as an error of the sum (bounds:
+// ihc_tensor_taps).
 //
 // T has one value per diagonal.  With the rows of x stored in reverse order its
 // band is a Hankel matrix (element (r, k') depends on r + k'), and a Hankel
@@ -40,7 +46,8 @@ constexpr int kRows = 128;           // output rows of a tile (M)
 constexpr int kCols = 64;            // sections of a tile (N)
 constexpr int kDepth = 384;          // rows of x of a tile (K)
 constexpr int kHalf = kDepth / 2;    // rows in one of the two buffers of a digit
-constexpr int kDigits = 5;
+constexpr int kDigits = 5;           // of a tap
+constexpr int kRowDigits = 6;        // of a value of x
 constexpr int kSums = 6;             // accumulators
 constexpr int kMaxTaps = kDepth - kRows + 1;
 constexpr int kCores = (kRows + kDepth) / 8 - 1;  // block diagonals of the band
