@@ -191,14 +191,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
     int phase = 0;
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       if (!skip || phase > 1)
         issue_conv8(S, base + kOffIn, 6, base + kOffFirst, tmem, issue);
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffSecond, kWChunk, kWTap, instr(64, false), tmem, issue);
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       issue_conv64(S, base + kOffB, base + kOffThird, kWChunk, kWTap, instr(64, false), tmem, issue);
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffLast, kW4Chunk, kW4Tap, instr(16, false), tmem, issue);
     }
     drain(S, issue);
@@ -309,12 +309,12 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     const uint32_t issue = tfir::elected(), base = tfir::saddr(sm);
     int phase = 0;
     for (int rec = blockIdx.x; rec < n; rec += gridDim.x) {
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       if (!skip || phase > 1)
         issue_conv8(S, base + kOffIn, 0, base + kOffFirst, tmem, issue);
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       issue_conv64(S, base + kOffA, base + kOffSecond, kWChunk, kWTap, instr(64, false), tmem, issue);
-      if (!take_over(S, 0, phase++)) break;
+      if (!take_over(S, &S.ready[0], phase++)) break;
       issue_conv64(S, base + kOffB, base + kOffThird, kWChunk, kWTap, instr(64, false), tmem, issue);
     }
     drain(S, issue);

@@ -14,7 +14,7 @@ int forward_loss(const void* d_blob, const void* d_feat, int n, void* d_hid, flo
                  void* stream);
 
 struct TensorShared {
-  uint64_t mbar[2];   // the products of stage (or tile) h are done
+  uint64_t mbar[3];   // the products of tile (or accumulator) h are done
   uint64_t ready[2];  // the operands (of stage h) are in shared memory: an arrival a warp
   uint64_t drained;   // all products that were issued are done
   uint32_t tmem;
@@ -29,10 +29,8 @@ __host__ __device__ constexpr uint32_t instr(int n, bool mn_major) {
 
 // warps: that prepare the operands
 __device__ __forceinline__ void init_barriers(TensorShared& S, int warps) {  // one thread
-  for (int h = 0; h < 2; ++h) {
-    mbar_init(&S.mbar[h], 1);
-    mbar_init(&S.ready[h], warps);
-  }
+  for (int h = 0; h < 3; ++h) mbar_init(&S.mbar[h], 1);
+  for (int h = 0; h < 2; ++h) mbar_init(&S.ready[h], warps);
   mbar_init(&S.drained, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   S.failed = 0;
@@ -56,11 +54,11 @@ __device__ __forceinline__ void hand_over(TensorShared& S, int h, int lane) {
   __syncwarp();
   if (lane == 0) mbar_arrive(&S.ready[h]);
 }
-// The issuing warp, converged: completion `phase` of ready[h]; false after a wait
-// that ran out.
-__device__ __forceinline__ bool take_over(TensorShared& S, int h, int phase) {
+// The issuing warp, converged: completion `phase` of a barrier that the other warps
+// arrive at; false after a wait that ran out.
+__device__ __forceinline__ bool take_over(TensorShared& S, uint64_t* bar, int phase) {
   const unsigned long long start = global_ns();
-  while (!__all_sync(kFull, mbar_done(&S.ready[h], phase))) {
+  while (!__all_sync(kFull, mbar_done(bar, phase))) {
     // (the other warps' work between two operands is far shorter, their waits a fourth)
     const bool late = global_ns() - start > 4 * kWaitNs;
     if (__any_sync(kFull, late || *(volatile int*)&S.failed)) return false;

@@ -183,7 +183,8 @@ class WarmStartNet:
         """Forward, loss and backward; returns (mean loss tensor, grad tensor)."""
         n = int(feat.shape[0])
         buf = buf or self.buffers(n)
-        parts = n_parts or max(1, min(n, 2 * _sm_count(self.device)))
+        # (what the weight gradients use: a slot for three SMs, and its rounding errors')
+        parts = n_parts or max(1, min(n, 2 * (_sm_count(self.device) // 3)))
         if "partial" not in buf or buf["partial"].shape[0] < parts:
             buf["partial"] = torch.zeros((parts, self.n_params), dtype=torch.float32,
                                          device=self.device)

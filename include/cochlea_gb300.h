@@ -222,7 +222,9 @@ int cgb_bm_run_ex_dev(const float* d_secp, const float* d_gamma, int n_profiles,
  *   target   float[n][256] (p* - pe) / max|rt|; nr float[n] = max|rt|
  *   hid      BF16 [3][n][256][64] hidden activations (64-channel rows)
  *   dout     BF16 [n][256][8] dL/d(output); dpre BF16 [3][n][256][64]
- *   partial  float[n_parts][cgb_ws_param_count()]; grad float[param_count] */
+ *   partial  float[n_parts][cgb_ws_param_count()] of scratch, of which at most
+ *            min(n, 2 (SMs / 3)) rows are used: sums of records, and what their
+ *            rounding left; grad float[param_count] */
 int cgb_ws_blob_bytes(void);
 int cgb_ws_blobT_bytes(void);
 int cgb_ws_param_count(void);
