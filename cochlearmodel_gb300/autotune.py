@@ -9,10 +9,13 @@ this library on the workload and GPU at hand, and caches the winner:
   previous-step state in registers or shared memory);
 - the IHC/lambda run length (cgb_ihc_set_run_length: consecutive tiles per CTA).
 
-Every candidate gives the same results bit for bit (the search checks it); the
-tile rows of the IHC kernel are fixed by the filters (the largest tile that fits
-shared memory and holds the DC look-back), and the JND kernel's row groups set
-its summation order, so neither is searched.
+Every candidate gives the same results bit for bit (the search checks it).  Which
+kernels the candidates are of depends on the workload: launch shape 0 of few units
+is the kernel of four warps per unit, or one with the sweep counts compiled in; a
+tile of the IHC stage has 128 rows where the AC filter runs on the tensor cores
+(by the filters and the frame table), else the most that fit shared memory.  The
+workload's key holds what decides it.  The tile rows themselves and the JND
+kernel's row groups, which set its summation order, are not searched.
 
 The cache is a JSON file (CGB_TUNE_CACHE, default cochlearmodel_gb300/_tune/
 tuning.json) keyed by the device name, a hash of the library and a description
@@ -163,15 +166,30 @@ def search(stage_bm: Callable[[], None], stage_ihc: Callable[[], None],
     return choice, {k: {str(c): t for c, t in v.items()} for k, v in timings.items()}
 
 
+def workload(run) -> str:
+    """What decides, besides the device and the library, which kernels run and how long
+    they take: the tables' sizes, the solver's method and the IHC stage's filters and
+    frames (hashed)."""
+    sc = run.sc
+    method = (sc.controller, sc.arith, sc.jacobi_mode, sc.jacobi_slow, sc.jacobi_fast,
+              sc.max_outer)
+    h = hashlib.sha256()
+    for a in (run.ihc.ac, run.ihc.dc, run.frames):
+        h.update(a.tobytes())
+        h.update(b"|")
+    return (f"{type(run).__name__}:units={len(run.units)}:"
+            f"frames={len(run.frames)}:lam_rows={int(run.d_lam.shape[1])}:"
+            f"bm={'.'.join(map(str, method))}:ac={len(run.ihc.ac)}:dc={len(run.ihc.dc)}:"
+            f"ihc={h.hexdigest()[:12]}")
+
+
 def tune_sweep(run, device, rounds: int = 3, use_cache: bool = True):
     """Tunes a BatchSweep or ProfileRun on `device` (or takes the cached
     choice) and applies it; returns (Choice, source) with source 'cache' or
     'search'."""
     import torch
     name = torch.cuda.get_device_name(device)
-    workload = (f"{type(run).__name__}:units={len(run.units)}:"
-                f"frames={len(run.frames)}:lam_rows={int(run.d_lam.shape[1])}")
-    key = cache_key(name, workload)
+    key = cache_key(name, workload(run))
     if use_cache:
         hit = lookup(key)
         if hit is not None:
@@ -216,7 +234,9 @@ def occupancy_profile(run, shapes: Sequence[int], prefixes: Sequence[int], reps:
     table (longest first) for each launch shape and n in `prefixes`.  With
     n below one wave the time is that of the longest units at n / (SMs x 4)
     warps per scheduler, so the table separates per-warp speed, throughput
-    per scheduler and the last wave's fill."""
+    per scheduler and the last wave's fill.  Shape 0 gives up to one unit per
+    SM (two with controller 1) to the kernel of four warps per unit: such a
+    prefix says nothing of the warp-per-unit kernel's speed."""
     import torch
     lib = native.load()
     dev = run.d_v.device
@@ -260,7 +280,7 @@ def _main(argv=None) -> None:
     import json as _json
     ap = argparse.ArgumentParser(description="BM launch-shape occupancy profile on the JND sweep")
     ap.add_argument("--shapes", default="0,3")
-    ap.add_argument("--prefixes", default="152,608,912,1216,1824,2432,100000")
+    ap.add_argument("--prefixes", default="608,912,1216,1824,2432,100000")
     ap.add_argument("--n-seeds", type=int, default=4)
     a = ap.parse_args(argv)
     from . import batch
