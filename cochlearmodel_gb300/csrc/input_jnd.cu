@@ -363,7 +363,9 @@ extern "C" int cgb_jnd_dev(const float* d_lam, int64_t plane_rows, int n_int, in
     return fail(CGB_ERR_ARG, "cgb_jnd_dev: bad arguments");
   if ((int64_t)n_int * interval_nodes > plane_rows || head + len > interval_nodes)
     return fail(CGB_ERR_RANGE, "cgb_jnd_dev: intervals reach outside the lambda planes");
-  if (n_int > 2147483647 / kJndCluster) return fail(CGB_ERR_RANGE, "cgb_jnd_dev: too many intervals");
+  // (their rates would not fit a GPU's memory)
+  if (n_int > 2147483647 / kJndCluster)
+    return fail(CGB_ERR_RANGE, "cgb_jnd_dev: too many intervals");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const double T = delta_alpha_len_factor / Fs;
   dim3 grid((unsigned)n_int * kJndCluster, 3);
@@ -415,19 +417,25 @@ extern "C" int cgb_jnd_batch_dev(const float* d_lam, int64_t plane_rows,
   if (!d_lam || !d_iv || !d_nihc || !W || !d_F_RA || !d_F_AI || n_iv < 0 || n_out <= 0 ||
       plane_rows <= 0)
     return fail(CGB_ERR_ARG, "cgb_jnd_batch_dev: bad arguments");
-  if (n_iv > 2147483647 / (3 * kJndCluster)) return fail(CGB_ERR_RANGE, "cgb_jnd_batch_dev: too many intervals");
+  if (n_iv > 2147483647 / 3) return fail(CGB_ERR_RANGE, "cgb_jnd_batch_dev: too many intervals");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const double T = delta_alpha_len_factor / Fs;
-  dim3 grid((unsigned)(3 * n_iv) * kJndCluster);
   const int copies = jnd_copies(d_lam, 3LL * n_iv * kJndCluster);
   auto kernel = copies == 0   ? jnd_batch_kernel<false, false>
                 : copies == 1 ? jnd_batch_kernel<true, false>
                               : jnd_batch_kernel<true, true>;
-  kernel<<<grid, kJndThreads, 0, st>>>(d_lam, plane_rows, d_iv, n_out, d_nihc,
-                                                 (double)W[0], (double)W[1], (double)W[2], Fs, T,
-                                                 d_F_RA, d_F_AI, d_MR);
-  CGB_TRY_CUDA(cudaGetLastError(), "jnd_batch_kernel launch");
-  note_launch();
+  // a grid has room for the clusters of an eighth of the intervals that the call takes
+  constexpr int kPerGrid = 2147483647 / (3 * kJndCluster);
+  for (int at = 0, left = n_iv; left > 0;) {
+    const int part = left < kPerGrid ? left : kPerGrid;
+    kernel<<<(unsigned)part * (3 * kJndCluster), kJndThreads, 0, st>>>(
+        d_lam, plane_rows, d_iv + at, n_out, d_nihc, (double)W[0], (double)W[1], (double)W[2], Fs,
+        T, d_F_RA, d_F_AI, d_MR);
+    CGB_TRY_CUDA(cudaGetLastError(), "jnd_batch_kernel launch");
+    note_launch();
+    left -= part;
+    if (left > 0) at += part;
+  }
   return CGB_OK;
 }
 
