@@ -16,7 +16,13 @@
 //   lambda_j = s ? min(SAT, max(A_js IHC, spont_j)) : spont_j,  j = 0..2
 // in FP32, each FIR accumulated with a compensated dot product (Dot2).
 //
-// GB300 layout: one CTA = 32 sections x a run of consecutive TR-row tiles.
+// This file holds the FP32 kernel, the host side of the stage and the IIR form of the
+// AC filter.  The same stage with the AC filter on the tensor cores is ihc_tensor.cu;
+// ihc_lambda_impl gives it the calls that it is built for (64 to 257 taps whose digit
+// sums it holds, a uniform DC filter, no debug stage, no AC given) where the frame
+// table makes it the faster one (tensor_faster).
+//
+// The FP32 kernel: one CTA = 32 sections x a run of consecutive TR-row tiles.
 // Each tile's velocity window (TR rows plus the look-back) is staged into
 // shared memory by TMA (cp.async.bulk.tensor.2d, 64-row boxes, completion on
 // an mbarrier with a bounded wait), the next tile's while the current one
@@ -49,8 +55,9 @@ constexpr int kRB = 8;         // output rows per register block
 constexpr int kTilesPerRun = 8;  // consecutive tiles per CTA (short runs)
 
 // Test-only fault injection (cgb_ihc_set_fault_injection): the next launches
-// arm the first staging mbarrier without issuing its copies, so the bounded
-// wait runs out with nothing in flight and the kernel reports status bit 1.
+// arm the first staging mbarrier without issuing its copies (the tensor kernel
+// leaves out its first products), so the bounded wait runs out and the kernel
+// reports status bit 1.
 int g_fault_skip_copy = 0;
 
 // FIR of one 8-row block, rows kb..kb+7 all using `taps` taps.  src points at
@@ -456,7 +463,7 @@ int ac_symmetric(const float* ac_taps, int n_ac, float scale) {
   return 1;
 }
 
-// Tiles per CTA run.  A run's first tile recomputes the DC filter's n_dc - 1
+// Tiles per CTA run of the FP32 kernel.  A run's first tile recomputes the DC filter's n_dc - 1
 // look-back rows, so longer runs cost less; the longest of 32 and 16 tiles
 // that still leaves at least two CTAs per SM (eight section blocks per run),
 // else 8.  Runs need TR >= n_dc (the look-back is inherited in place).  The

@@ -4,7 +4,7 @@
 // What bounded the stage: 127 tap pairs of compensated FP32 arithmetic per
 // point, ~2,170 lane operations (43 ms of the FP32 pipe on 2.9 million rows).
 // Here the filter is a product of digit matrices (tensor_fir.cuh) that is exact
-// to about 2^-50 of the scales, 22k cycles of the tensor pipe for a tile of
+// to about 2^-50 of the scales, 23k cycles of the tensor pipe for a tile of
 // 128 rows x 64 sections; six exact integers per point leave TMEM.
 //
 // The same bits as the compensated FIR (Dot2).  Both are the sum rounded once,
@@ -45,8 +45,8 @@
 // products as soon as a half is there.  Between the digits the same warps finish
 // the tile before: its Dot2 points, the DC sums, IHC and lambda.
 //
-// What bounds it now: the workers' chain, ~52k cycles a tile (Dot2 points 7k, DC
-// sums 11k, IHC / lambda 7k, loads 7k, digits 10k, epilogue 4k) at 41% of the
+// What bounds it now: the workers' chain, ~54k cycles a tile (Dot2 points 7k, DC
+// sums 11k, IHC / lambda 7k, loads 7k, digits 12k, epilogue 4k) at 41% of the
 // issue slots, not the tensor pipe.  Finishing a tile at once instead of between
 // the next one's digits takes 22.0 ms against 18.9 (JND sweep); without the products
 // (accumulators left as they are) the chain takes the same time.  Single points by

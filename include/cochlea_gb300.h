@@ -354,19 +354,21 @@ int cgb_ihc_lambda_iir_stage_dev(const float* d_v, int64_t v_rows, const cgb_ihc
                                  int32_t* d_status, void* stream);
 
 /* Tiles each IHC/lambda CTA walks in a run (the DC look-back is recomputed
- * once per run): 0 restores the automatic choice (32 or 16 tiles while at
- * least two CTAs per SM remain, else 8); 1-64 forces that run length.  It
- * takes effect at the next upload of the per-call tables (cgb_ihc_lambda_dev,
+ * once per run): 0 restores the automatic choice (FP32 kernel: 32 or 16 tiles
+ * while at least two CTAs per SM remain, else 8; tensor kernel, whose tiles have
+ * 128 rows: the length with the least waves x tiles over the SMs); 1-64 forces
+ * that run length.  It takes effect at the next upload of the per-call tables (cgb_ihc_lambda_dev,
  * _upload_dev, _noalloc_dev): a launch of tables uploaded earlier keeps the
  * run length they were uploaded with.  Every choice gives the same results
  * bit for bit; the autotuner times them. */
 int cgb_ihc_set_run_length(int tiles);
 
-/* Test-only fault injection for the IHC/lambda kernel's bounded staging
- * wait -- no counterpart in the reference.  With skip_first_copy = 1, later
- * launches arm each CTA's first staging mbarrier but issue none of its copies,
- * so the wait runs out after about one second with no copy in flight and the
- * kernel sets bit 1 of *d_status; 0 restores normal launches. */
+/* Test-only fault injection for the IHC/lambda kernels' bounded waits -- no
+ * counterpart in the reference.  With skip_first_copy = 1, later launches of
+ * the FP32 kernel arm each CTA's first staging mbarrier but issue none of its
+ * copies, and those of the tensor kernel leave out each CTA's first products,
+ * so that the wait runs out after about one second and the kernel sets bit 1 of
+ * *d_status; 0 restores normal launches. */
 int cgb_ihc_set_fault_injection(int skip_first_copy);
 
 /* IHC + lambda without any device allocation -- no counterpart in the
