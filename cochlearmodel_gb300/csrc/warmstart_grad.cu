@@ -294,7 +294,9 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     for (int low = 0; low < (split ? 2 : 1); ++low) {
       asm volatile("bar.sync 3, %0;" ::"n"(kLoaders) : "memory");
       // columns c0 + c .. + 7 of accumulator j, and the column of ones
+      // (a sum out of FP32's range has no low part)
       auto value = [&](float h, float l) {
+        l = fabsf(h) < __int_as_float(0x7f800000) ? l : 0.0f;
         return failed ? __int_as_float(0x7fffffff) : low ? l : split ? h : __fadd_rn(h, l);
       };
       auto read = [&](int j, int c, float (&v)[8]) {

@@ -56,6 +56,29 @@ def test_same_sign(n, parts):
     assert err <= tol, (err, tol)
 
 
+@pytest.mark.parametrize("n, parts", [(120, 100), (120, 40), (10, 10)])
+def test_out_of_range(n, parts):
+    """A product past the FP32 range is an infinity in its gradients and nothing elsewhere."""
+    feat = torch.zeros(n, 280, 8, dtype=torch.bfloat16, device=D)
+    hid = torch.ones(3, n, 256, 64, dtype=torch.bfloat16, device=D)
+    dpre = torch.ones(3, n, 256, 64, dtype=torch.bfloat16, device=D)
+    dout = torch.zeros(n, 256, 8, dtype=torch.bfloat16, device=D)
+    hid[0, n // 2, 100, 5], dpre[1, n // 2, 100, 7] = 4.0, 3e38  # layer 2, the middle tap
+    lib = native.load()
+    count = lib.cgb_ws_param_count()
+    partial = torch.zeros(parts, count, device=D)
+    grad = torch.zeros(count, device=D)
+    p = native.ptr
+    k_hid, k_dpre = _rows64(hid), _rows64(dpre)
+    native.check(lib.cgb_ws_wgrad_dev(p(feat), p(k_hid), p(k_dpre), p(dout), n, p(partial), parts,
+                                      p(grad), C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                 "cgb_ws_wgrad_dev")
+    w2 = grad[5 * 64 * 8 + 64:][:5 * 64 * 64].reshape(5, 64, 64)
+    assert w2[2, 7, 5].item() == float("inf")
+    w2[2, 7, 5] = 0.0
+    assert torch.isfinite(grad).all()
+
+
 @pytest.mark.parametrize("n", [64, 256, 1000])
 def test_slots_of_the_network(n):
     """gradients() gives the slots room for both parts, and no more."""
